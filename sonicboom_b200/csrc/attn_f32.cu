@@ -1,0 +1,321 @@
+// Float32 attention over the paged cache for the 32-bit path: FFMA only, a block per tile of query rows of one
+// key/value head of one sequence.
+//
+// A query row is a (token, head in group) pair, so that all query heads of a key/value head share its tiles.  Two
+// forms: 16 rows (a decode step: one token's heads), 64 rows (prompts).  Keys come in tiles of 64 at absolute
+// positions, which a cluster of blocks takes in turn (8 blocks for 16 rows, where a step has few blocks and the
+// sequence is long; 2 for 64 rows); the blocks' running softmaxes are merged in rank order through distributed shared
+// memory, so no workspace is needed and a row's sums depend on its own keys and the form alone.
+//
+// What attn_plain.cu says about masks, caps, biases and sinks holds here; that kernel (a block per row and head, a
+// warp per key) stays for head sizes this one does not take.  12/2 heads of 128: three single tokens at 100 to 400 keys
+// took 324 us there, bound by a block's dependent steps over its keys, and 19 here; a prompt of 201 tokens 183 and 67.
+#include <cooperative_groups.h>
+#include <math.h>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int THREADS = 256, KEYS = 64;
+
+struct F32Attn {
+  const float* q;
+  float* out;
+  const int32_t* seq_row0;
+  const int32_t* seq_pos0;
+  const int32_t* page_off;
+  const int32_t* page_ids;
+  const float* cache;
+  int page_size, n_pages, n_q_heads, n_kv_heads, hd, window, chunk, bias_len;
+  float scale, softcap;
+  const float* sink;
+  const float* bias;
+};
+
+// TQ query rows a thread in the scores and the output (16 threads of neighbouring lanes share a row's keys or
+// dimensions); head sizes up to 64 ND.
+template <int TQ, int ND>
+struct Form {
+  static constexpr int QB = 16 * TQ;
+  static constexpr int SPLITS = TQ == 1 ? 8 : 2;
+  static int floats(int hd) {      // queries, keys (later probabilities), values, maximum and sum, their merge
+    const int kp = KEYS * (hd + 4), pp = QB * (KEYS + 4), op = QB * hd;
+    const int first = kp > pp ? kp : pp;
+    return QB * hd + (first > op ? first : op) + KEYS * hd + 2 * QB;
+  }
+};
+
+template <int TQ, int ND>
+__global__ void __launch_bounds__(THREADS)
+attn_f32_kernel(F32Attn p, int tiles_per_seq) {
+  using F = Form<TQ, ND>;
+  constexpr int QB = F::QB;
+  extern __shared__ __align__(16) float smem[];
+  const int hd = p.hd, kpitch = hd + 4, ppitch = KEYS + 4;
+  float* qs = smem;
+  float* ks = qs + QB * hd;
+  float* ps = ks;                                       // over the keys, once the scores are made
+  const int first = max(max(KEYS * kpitch, QB * ppitch), QB * hd);
+  float* vs = ks + first;
+  float* stat = vs + KEYS * hd;                         // maximum and sum per row, for the merge
+  __shared__ int bad_values;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = blockIdx.z, tid = threadIdx.x;
+  const int seq = blockIdx.x / tiles_per_seq, tile = blockIdx.x % tiles_per_seq, g = blockIdx.y;
+  const int group = p.n_q_heads / p.n_kv_heads;
+  sb_pdl_wait();
+  const int row0 = p.seq_row0[seq], n_new = p.seq_row0[seq + 1] - row0, pos0 = p.seq_pos0[seq];
+  const int pairs = n_new * group, pair0 = tile * QB;
+  if (pair0 >= pairs) return;                           // the same for the whole cluster
+  const int32_t* pages = p.page_ids + p.page_off[seq];
+  const int held = (p.page_off[seq + 1] - p.page_off[seq]) * p.page_size;      // positions with a page
+
+  const int tx = tid & 15, ty = tid >> 4;               // rows ty * TQ + i
+  // what each of the thread's rows sees: keys lo ... pos (none where the position has no page: the row is zeros)
+  int pos[TQ], lo[TQ];
+  bool live[TQ];
+#pragma unroll
+  for (int i = 0; i < TQ; ++i) {
+    const int pair = pair0 + ty * TQ + i;
+    pos[i] = pos0 + pair / group;
+    live[i] = pair < pairs && pos[i] >= 0 && pos[i] / p.page_size < held / p.page_size;
+    lo[i] = max(p.window > 0 ? max(0, pos[i] - p.window + 1) : 0, p.chunk > 0 ? max(pos[i], 0) / p.chunk * p.chunk : 0);
+  }
+  // the tile's keys: from the first row's first to the last row's last
+  const int first_pos = pos0 + pair0 / group, last_pos = pos0 + (min(pair0 + QB, pairs) - 1) / group;
+  const int k_lo = max(p.window > 0 ? max(0, first_pos - p.window + 1) : 0,
+                       p.chunk > 0 ? max(first_pos, 0) / p.chunk * p.chunk : 0);
+  const int k_hi = min(last_pos, held - 1);
+
+  const int quads = hd / 4;
+  for (int i = tid; i < QB * quads; i += THREADS) {
+    const int r = i / quads, c = i % quads, pair = pair0 + r;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (pair < pairs)
+      v = *reinterpret_cast<const float4*>(p.q + ((size_t)(row0 + pair / group) * p.n_q_heads + g * group + pair % group) * hd + 4 * c);
+    *reinterpret_cast<float4*>(qs + r * hd + 4 * c) = v;
+  }
+
+  float m[TQ], l[TQ];
+  float4 acc[TQ][ND];
+#pragma unroll
+  for (int i = 0; i < TQ; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.0f;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) acc[i][d] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+
+  for (int t = k_lo / KEYS + rank; t <= k_hi / KEYS && k_hi >= k_lo; t += F::SPLITS) {
+    const int base = t * KEYS;
+    __syncthreads();                                    // the tile before this one has been read
+    if (tid == 0) bad_values = 0;
+    __syncthreads();
+    bool bad = false;
+    for (int i = tid; i < KEYS * quads; i += THREADS) {
+      const int r = i / quads, c = i % quads, j = base + r;
+      float4 kv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv = kv;
+      const int page = j >= k_lo && j <= k_hi ? pages[j / p.page_size] : -1;
+      if (page >= 0 && page < p.n_pages) {
+        const float* at = p.cache + (((size_t)page * 2 * p.n_kv_heads + g) * p.page_size + j % p.page_size) * hd + 4 * c;
+        kv = *reinterpret_cast<const float4*>(at);
+        vv = *reinterpret_cast<const float4*>(at + (size_t)p.n_kv_heads * p.page_size * hd);
+      }
+      *reinterpret_cast<float4*>(ks + r * kpitch + 4 * c) = kv;
+      *reinterpret_cast<float4*>(vs + r * hd + 4 * c) = vv;
+      const float s = fabsf(vv.x) + fabsf(vv.y) + fabsf(vv.z) + fabsf(vv.w);
+      bad |= !(s < INFINITY);
+    }
+    if (bad) bad_values = 1;
+    __syncthreads();
+
+    // scores: rows ty * TQ + i, keys tx + 16 j
+    float s[TQ][4] = {};
+    for (int c = 0; c < quads; ++c) {
+      float4 kq[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kq[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * kpitch + 4 * c);
+#pragma unroll
+      for (int i = 0; i < TQ; ++i) {
+        const float4 qv = *reinterpret_cast<const float4*>(qs + (ty * TQ + i) * hd + 4 * c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(qv.x, kq[j].x, s[i][j]);
+          s[i][j] = fmaf(qv.y, kq[j].y, s[i][j]);
+          s[i][j] = fmaf(qv.z, kq[j].z, s[i][j]);
+          s[i][j] = fmaf(qv.w, kq[j].w, s[i][j]);
+        }
+      }
+    }
+    __syncthreads();                                    // the keys have been read: the probabilities take their place
+#pragma unroll
+    for (int i = 0; i < TQ; ++i) {
+      float tile_max = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = base + tx + 16 * j;
+        float v = s[i][j] * p.scale;
+        if (p.softcap > 0.0f) v = p.softcap * tanhf(v / p.softcap);
+        const bool sees = live[i] && key >= lo[i] && key <= pos[i];
+        if (p.bias && sees) {
+          const int h = g * group + (pair0 + ty * TQ + i) % group;
+          v += p.bias[(size_t)h * p.bias_len + min(pos[i] - key, p.bias_len - 1)];
+        }
+        s[i][j] = sees ? v : -INFINITY;
+        tile_max = fmaxf(tile_max, s[i][j]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, o));
+      const float m_new = fmaxf(m[i], tile_max);
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = s[i][j] == -INFINITY ? 0.0f : expf(s[i][j] - m_new);
+        ps[(ty * TQ + i) * ppitch + tx + 16 * j] = e;
+        sum += e;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      const float alpha = m[i] == -INFINITY ? 0.0f : expf(m[i] - m_new);
+      l[i] = l[i] * alpha + sum;
+      m[i] = m_new;
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        acc[i][d].x *= alpha; acc[i][d].y *= alpha; acc[i][d].z *= alpha; acc[i][d].w *= alpha;
+      }
+    }
+    __syncwarp();                                       // a row's probabilities are read by the lanes that wrote them
+    // output: rows ty * TQ + i, dimensions tx * 4 + 64 d.  A value that is not finite must not reach rows that do not
+    // see its key, so a tile that holds one takes the keys one by one.
+    const bool check = bad_values != 0;
+    for (int k4 = 0; k4 < KEYS; k4 += 4) {
+      float4 pr[TQ];
+#pragma unroll
+      for (int i = 0; i < TQ; ++i) pr[i] = *reinterpret_cast<const float4*>(ps + (ty * TQ + i) * ppitch + k4);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          if (tx * 4 + 64 * d >= hd) continue;
+          const float4 v = *reinterpret_cast<const float4*>(vs + (k4 + c) * hd + tx * 4 + 64 * d);
+#pragma unroll
+          for (int i = 0; i < TQ; ++i) {
+            const float w = c == 0 ? pr[i].x : c == 1 ? pr[i].y : c == 2 ? pr[i].z : pr[i].w;
+            if (check) {
+              const int key = base + k4 + c;
+              if (!(live[i] && key >= lo[i] && key <= pos[i])) continue;
+            }
+            acc[i][d].x = fmaf(w, v.x, acc[i][d].x);
+            acc[i][d].y = fmaf(w, v.y, acc[i][d].y);
+            acc[i][d].z = fmaf(w, v.z, acc[i][d].z);
+            acc[i][d].w = fmaf(w, v.w, acc[i][d].w);
+          }
+        }
+      }
+    }
+  }
+
+  // merge: every block leaves its sums over its keys' space, then takes a share of the rows
+  sb_pdl_launch();
+  __syncthreads();
+  float* os = ks;
+#pragma unroll
+  for (int i = 0; i < TQ; ++i) {
+    const int r = ty * TQ + i;
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if (tx * 4 + 64 * d < hd) *reinterpret_cast<float4*>(os + r * hd + tx * 4 + 64 * d) = acc[i][d];
+    if (tx == 0) { stat[2 * r] = m[i]; stat[2 * r + 1] = l[i]; }
+  }
+  cluster.sync();
+  for (int r = rank * (QB / F::SPLITS) + ty; r < (rank + 1) * (QB / F::SPLITS); r += 16) {
+    const int pair = pair0 + r;
+    if (pair >= pairs) continue;
+    const int h = g * group + pair % group, at = pos0 + pair / group;
+    const bool row_live = at >= 0 && at / p.page_size < held / p.page_size;
+    float m_all = -INFINITY, total = 0.0f;
+    for (int s = 0; s < F::SPLITS; ++s) m_all = fmaxf(m_all, cluster.map_shared_rank(stat, s)[2 * r]);
+    if (p.sink) m_all = fmaxf(m_all, p.sink[h]);
+    float f[F::SPLITS];
+#pragma unroll
+    for (int s = 0; s < F::SPLITS; ++s) {
+      const float* st = cluster.map_shared_rank(stat, s);
+      f[s] = st[2 * r] == -INFINITY ? 0.0f : expf(st[2 * r] - m_all);
+      total += st[2 * r + 1] * f[s];
+    }
+    if (p.sink) total += expf(p.sink[h] - m_all);
+    const float inv = 1.0f / total;
+    float* to = p.out + ((size_t)(row0 + pair / group) * p.n_q_heads + h) * hd;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      const int at_d = tx * 4 + 64 * d;
+      if (at_d >= hd) continue;
+      float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (row_live) {
+#pragma unroll
+        for (int s = 0; s < F::SPLITS; ++s) {
+          const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(os, s) + r * hd + at_d);
+          o.x = fmaf(v.x, f[s], o.x); o.y = fmaf(v.y, f[s], o.y); o.z = fmaf(v.z, f[s], o.z); o.w = fmaf(v.w, f[s], o.w);
+        }
+        o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+      }
+      *reinterpret_cast<float4*>(to + at_d) = o;
+    }
+  }
+  cluster.sync();                                       // nobody's sums go while another block reads them
+}
+
+template <int TQ, int ND>
+int launch(const F32Attn& p, int n_seqs, int max_new, cudaStream_t stream) {
+  using F = Form<TQ, ND>;
+  const int group = p.n_q_heads / p.n_kv_heads;
+  const int tiles = (int)(((long)max_new * group + F::QB - 1) / F::QB);
+  const size_t smem = (size_t)F::floats(p.hd) * sizeof(float);
+  if (cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<TQ, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           F::floats(64 * ND) * (int)sizeof(float)))
+    SB_FAIL(SB_ERR_CUDA, "sb_attention_f32: %s", cudaGetErrorString(e));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)n_seqs * (unsigned)tiles, p.n_kv_heads, F::SPLITS);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = F::SPLITS;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (sb_pdl_enabled() & SB_K_OTHER) ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, attn_f32_kernel<TQ, ND>, p, tiles);
+  SB_CHECK_LAUNCH("sb_attention_f32");
+  return SB_OK;
+}
+
+}  // namespace
+
+int sb_check_attention_args(const char* who, int n_rows, int n_q_heads, int n_kv_heads, int hd, int window, int page_size);
+
+extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, const int32_t* seq_row0,
+                                const int32_t* seq_pos0, const int32_t* page_off, const int32_t* page_ids, int page_size,
+                                const float* cache, int n_pages, int n_q_heads, int n_kv_heads, int hd, int window,
+                                float scale, const float* sink, float softcap, int chunk, const float* bias, int bias_len,
+                                cudaStream_t stream) {
+  if (chunk < 0 || (bias && bias_len < 1))
+    SB_FAIL(SB_ERR_ARG, "sb_attention_f32: chunk %d, a distance bias of %d entries", chunk, bias_len);
+  if (softcap < 0.0f) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: score cap %g (0: none)", softcap);
+  if (int rc = sb_check_attention_args("sb_attention_f32", n_rows, n_q_heads, n_kv_heads, hd, window, page_size)) return rc;
+  if (n_seqs <= 0 || max_new <= 0) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: %d sequences, at most %d new rows", n_seqs, max_new);
+  if (hd % 4 || hd > 256 || n_kv_heads > 65535)
+    SB_FAIL(SB_ERR_UNSUPPORTED, "sb_attention_f32: head size %d (a multiple of 4 up to 256), %d key/value heads", hd, n_kv_heads);
+  const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
+                  chunk, bias_len, scale, softcap, sink, bias};
+  // one token's heads fit the 16-row form; a row of a longer stretch sees up to 64 rows' keys loaded once
+  const bool few = (long)max_new * (n_q_heads / n_kv_heads) <= 16;
+  if (hd <= 64) return few ? launch<1, 1>(p, n_seqs, max_new, stream) : launch<4, 1>(p, n_seqs, max_new, stream);
+  if (hd <= 128) return few ? launch<1, 2>(p, n_seqs, max_new, stream) : launch<4, 2>(p, n_seqs, max_new, stream);
+  return few ? launch<1, 4>(p, n_seqs, max_new, stream) : launch<4, 4>(p, n_seqs, max_new, stream);
+}

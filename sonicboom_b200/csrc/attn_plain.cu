@@ -1,6 +1,6 @@
 // Plain attention over the paged cache: one block per (row, query head), float32 arithmetic.
-// It is the true 32-bit path's attention and, with bfloat16 storage, the kernel the
-// tensor-core attention is checked against.
+// It takes every head size up to 1,024 and, with bfloat16 storage, is the kernel the tensor-core
+// attention is checked against; float32 at head sizes up to 256 runs attn_f32.cu.
 //
 // For the query at absolute position i: key j is visible when j <= i and (window == 0 or
 // i < j + window); s_j = (q . k_j) * scale with the scale applied after the whole dot;

@@ -559,8 +559,9 @@ def attention(q: torch.Tensor, out: torch.Tensor, plan, group_index: int, cache:
     start, are visible.  `bias`: the capped score of a key d positions back gets the head's bias for
     distance d added (`DistanceBias`).
 
-    bfloat16 runs the tensor-core kernels (built for the head size at first use); float32, a
-    head size those kernels do not take, or `kernel="plain"` run the plain kernel.  `"mma"` keeps
+    bfloat16 runs the tensor-core kernels (built for the head size at first use); float32 at head
+    sizes that are multiples of 4 up to 256 runs the tiled FFMA kernel; other head sizes, or
+    `kernel="plain"`, run the plain kernel.  `"mma"` keeps
     to the mma.sync kernels where the tensor-memory prefill kernel or the persistent TMA decode
     kernel would run (head sizes 64, 128); `"tma"` runs that decode kernel whatever the number of
     key splits (by itself it runs from about a wave of splits on).
@@ -596,6 +597,14 @@ def attention(q: torch.Tensor, out: torch.Tensor, plan, group_index: int, cache:
             raise KernelError(f"attention: {al.sb_last_error().decode()}")
         global LAUNCHES
         LAUNCHES += int(al.sb_attention_last_launches())
+    elif (q.dtype == out.dtype == cache.dtype == torch.float32 and kernel != "plain" and head_dim % 4 == 0 and head_dim <= 256
+          and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0):
+        _check(lib().sb_attention_f32(
+            _ptr(q), _ptr(out), n, plan.n_seqs, plan.max_new, _i32(plan.seq_row0, "seq_row0"),
+            _i32(plan.seq_pos0, "seq_pos0"), _i32(g.page_off, "page_off"), _i32(g.page_ids, "page_ids"), g.page_size,
+            _ptr(cache), cache.shape[0], n_q_heads, n_kv_heads, head_dim, window, ctypes.c_float(scale), _ptr(sink),
+            ctypes.c_float(softcap), int(chunk), _ptr(bias.values) if bias is not None else None, bias_len, _stream()),
+            "attention (float32 kernel)")
     else:
         _check(lib().sb_attention_plain(
             _ptr(q), _ptr(out), _code(q.dtype), n, _i32(plan.row_seq, "row_seq"),

@@ -1,0 +1,106 @@
+"""The float32 path's own kernels at the edges of their forms, against float64 and against the plain kernels."""
+import pytest
+import torch
+
+import plain_model as pm
+from sonicboom_b200 import ops
+from sonicboom_b200.cache.kv import Cache, KVNeed
+from sonicboom_b200.engine.step import StepEntry, StepPlan
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(*shape, seed=0, scale=1.0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).mul_(scale).to(DEV)
+
+
+def off_by_one(t):
+    """The same values at an address that is no multiple of 16: the plain kernel takes them."""
+    flat = torch.empty(t.numel() + 1, device=DEV)
+    flat[1:] = t.reshape(-1)
+    return flat[1:].view(t.shape)
+
+
+# rows: one to 32 stream the weights (1, 2, 4 and groups of 8), 33 on are tiled (2 to 8 rows a thread); K: one lane's
+# 16 bytes, less and more than a warp's 128 values, odd numbers of K tiles; N: less than a block's rows or columns
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 32, 33, 48, 81, 112, 129, 201])
+@pytest.mark.parametrize("N,K", [(16, 4), (48, 132), (1536, 1540), (272, 8960), (130, 100)])
+def test_products(M, N, K):
+    a, w, bias, res = rnd(M, K), rnd(N, K, seed=1, scale=K ** -0.5), rnd(N, seed=2), rnd(M, N, seed=3)
+    y = a.double() @ w.double().T
+    for epi, dtype in [(ops.EPI_NONE, torch.float32), (ops.EPI_BIAS, torch.float32), (ops.EPI_RESIDUAL, torch.float32),
+                       (ops.EPI_RELU2, torch.float32), (ops.EPI_SWIGLU, torch.float32), (ops.EPI_NONE, torch.bfloat16)]:
+        if epi == ops.EPI_SWIGLU and N % 16:
+            continue
+        want = {ops.EPI_BIAS: y + bias.double(), ops.EPI_RESIDUAL: y + res.double(), ops.EPI_RELU2: y.clamp(min=0) ** 2}.get(epi, y)
+        if epi == ops.EPI_SWIGLU:
+            z = y.view(M, -1, 2, 8)
+            want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2)
+        errs = []
+        for x in (a, off_by_one(a)):
+            out = res.clone() if epi == ops.EPI_RESIDUAL else torch.full(want.shape, float("nan"), device=DEV, dtype=dtype)
+            ops.linear(x, w, out, epi, bias=bias if epi == ops.EPI_BIAS else None,
+                       residual=out if epi == ops.EPI_RESIDUAL else None)
+            errs.append(float((out.double() - want).norm() / want.norm()))
+        # sums of K terms that are rounded one after the other are off by about sqrt(K) / 2 * 2^-24 of their terms'
+        # root mean square sum, squared or multiplied by about twice that
+        assert errs[0] < (2 ** -8 if dtype == torch.bfloat16 else (K ** 0.5 + 8) * 2 ** -24 * 2), (epi, errs)
+        assert errs[0] <= 1.3 * errs[1] + 2 ** -24, (epi, errs)     # and no more than the plain kernel's
+
+
+def test_products_let_infinities_through():
+    a, w = rnd(40, 256), rnd(64, 256, seed=1).abs()
+    a[3, 7], a[35, 200], a[39, 0] = float("inf"), float("-inf"), float("nan")
+    for rows in (40, 4):                               # tiled, streamed
+        out = torch.empty(rows, 64, device=DEV)
+        ops.linear(a[:rows].contiguous(), w, out)
+        assert bool((out[3] == float("inf")).all()) and bool(out[:3].isfinite().all())
+        if rows == 40:
+            assert bool((out[35] == float("-inf")).all()) and bool(out[39].isnan().all()) and bool(out[36:39].isfinite().all())
+
+
+def attention_both(hq, hkv, hd, held, new, window=0, chunk=0, sink=None, softcap=0.0, bias=None, edit=None, seed=0):
+    cache = Cache([KVNeed(hkv, hd, window, 0, chunk)], [None], 64 * sum((h + n + 63) // 64 for h, n in zip(held, new)),
+                  torch.float32, DEV)
+    storage = cache.groups[0].entry_storage(0)
+    storage.copy_(rnd(*storage.shape, seed=seed))
+    slots = [cache.open() for _ in held]
+    for s, h, n in zip(slots, held, new):
+        cache.reserve(s, h + n)
+        cache.advance(s, h)
+    if edit is not None:
+        edit(cache, storage, slots)
+    plan = StepPlan(cache, [StepEntry(s, [0] * n, []) for s, n in zip(slots, new)], DEV)
+    q = rnd(sum(new), hq, hd, seed=seed + 1)
+    outs = []
+    for kernel in ("auto", "plain"):
+        out = torch.full((sum(new), hq * hd), float("nan"), device=DEV)
+        ops.attention(q, out, plan, 0, storage, hq, hkv, hd, window, hd ** -0.5, kernel=kernel, sink=sink, softcap=softcap,
+                      chunk=chunk, bias=bias)
+        outs.append(out)
+    return outs
+
+
+# one token's heads in the 16-row form (and one head more than fits), stretches in the 64-row form; head sizes below,
+# at and over each width; lengths around a tile of 64 keys and around all of a cluster's tiles
+@pytest.mark.parametrize("hq,hkv,hd", [(4, 2, 16), (12, 2, 128), (17, 1, 36), (16, 1, 64), (3, 3, 100), (2, 1, 256)])
+@pytest.mark.parametrize("held,new", [([0, 63, 64, 511, 513, 1100], [1] * 6), ([0, 5, 200], [63, 130, 17]), ([0], [201])])
+def test_attention(hq, hkv, hd, held, new):
+    sink = rnd(hq, seed=5)
+    bias = ops.DistanceBias(rnd(hq, 33, seed=6))
+    for kw in (dict(), dict(window=70), dict(chunk=96, sink=sink), dict(softcap=3.0, bias=bias), dict(window=1, sink=sink, bias=bias)):
+        got, want = attention_both(hq, hkv, hd, held, new, **kw)
+        # two orders of a softmax's sums in float32: 2^-24 of the largest value for each of about 16 roundings
+        assert pm.rel_err(got.cpu(), want.cpu()) < 16 * 2 ** -24 * 2, kw
+
+
+def test_attention_of_values_that_are_not_finite():
+    """A later token's infinite value stays out of the rows that do not see it; the rows that do get what they get."""
+    def edit(cache, storage, slots):
+        page = cache.page_list(slots[0], 0)[1]
+        storage[page, 1, :, 20] = float("inf")         # position 84
+        storage[page, 0, :, 25] = float("nan")         # the key at 89
+    got, want = attention_both(4, 2, 32, [10], [120], edit=edit)
+    assert torch.equal(got.isfinite(), want.isfinite()) and bool(got[:74].isfinite().all())
+    assert pm.rel_err(got[:74].cpu(), want[:74].cpu()) < 16 * 2 ** -24 * 2
