@@ -58,11 +58,11 @@ __host__ __device__ constexpr uint32_t instr_desc(int bn) {
 }
 
 // SiLU of a value that is rounded to TO afterwards: for bfloat16 outputs with the hardware's
-// exponential (relative error about 1e-6 against bfloat16's 4e-3; a gate so negative that the
-// exponential overflows gives 1 / inf = 0, as it should); for float32 outputs the accurate one.
+// exponential and division (relative error about 1e-6 against bfloat16's 4e-3; a gate so negative that the
+// exponential overflows gives 0, as it should); for float32 outputs the accurate one.
 template <typename TO>
 __device__ __forceinline__ float sb_silu_out(float x) {
-  if (sizeof(TO) == 2) return x * __frcp_rn(1.0f + __expf(-x));
+  if (sizeof(TO) == 2) return __fdividef(x, 1.0f + __expf(-x));
   return sb_silu(x);
 }
 
@@ -89,6 +89,25 @@ __device__ __forceinline__ float sb_gated(const P& p, float gate, float up) {
   return sb_silu_out<TO>(gate) * up;
 }
 
+// The same for N outputs (gates v[0..7], their up values v[8..15], and so on): one branch for all of them, so that
+// their exponentials and divisions overlap.  (With a branch an output the gate/up epilogue of a prompt took 35
+// instructions an output one after the other: at K = 1,536 longer than the next tile's MMAs, 110 us for 2,048
+// rows of 17,920 x 1,536 where it is now 100.)
+template <typename TO, int N, typename P>
+__device__ __forceinline__ void sb_gated_row(const P& p, const float* v, float* o) {
+  if (p.gate_kind == SB_GATE_GELU_TANH) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) o[j] = sb_gelu_out<TO>(v[j / 8 * 16 + j % 8]) * v[j / 8 * 16 + 8 + j % 8];
+  } else if (p.gate_limit > 0.0f) {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      o[j] = sb_glu_clamped(v[j / 8 * 16 + j % 8], v[j / 8 * 16 + 8 + j % 8], p.gate_limit, p.gate_slope);
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) o[j] = sb_silu_out<TO>(v[j / 8 * 16 + j % 8]) * v[j / 8 * 16 + 8 + j % 8];
+  }
+}
+
 template <typename TB>
 __device__ __forceinline__ float bias_at(const void* bias, int n) {
   return sb_to_f32<TB>(((const TB*)bias)[n]);
@@ -101,6 +120,7 @@ struct Tc5Params {
   const float* residual;
   void* out;
   int tiles_a, tiles_b;        // tiles along the A rows and along the B rows
+  int group_a;                 // pair form: A tiles of a group (pair_tile)
   int k_splits;                // swapped form: blocks that share one output tile
   float* scratch;              // swapped form with k_splits > 1: partial tiles [tile][split][BN][128]
   const char* warm;            // asked into L2 by every block as it ends (or null)
@@ -143,9 +163,33 @@ __device__ __forceinline__ void store_row(bf16* dst, const float* v, int n) {
 // and written with 16-byte accesses: an eighth of the instructions of the transposed form and
 // no shared memory, which measured 53.5 against 66.1 us for the 2,048 x 3,584 x 3,584 product
 // with the residual (the last tile's epilogue is not hidden behind anything).  Needs the whole
-// chunk inside the matrix and rows that start on 16-byte boundaries (p.rowwise).
+// chunk inside the matrix and rows that start on 16-byte boundaries (chunk_rowwise).
+//
+// What is added to a chunk (residual, bias) does not depend on the accumulator, so it is asked for ahead of it
+// (chunk_ahead): by the pair kernel for a tile's first chunk before it waits for the MMAs and for the others a chunk
+// ahead, since a load's latency a chunk was longer than the MMAs of a tile with a short inner dimension (16,000 rows of
+// 1,536 x 1,536: 129 to 120 us).
+__device__ __forceinline__ bool chunk_rowwise(const Tc5Params& p, int n0) { return p.rowwise && n0 + 32 <= p.N; }
+
+__device__ __forceinline__ void chunk_ahead(const Tc5Params& p, uint4 (&add)[8], int m, int n0) {
+  if (p.epilogue == SB_EPI_RESIDUAL) {
+    if (m >= p.M) return;
+    const uint4* res = reinterpret_cast<const uint4*>(p.residual + (size_t)m * p.N + n0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) add[j] = res[j];
+  } else if (p.epilogue == SB_EPI_BIAS) {
+    const bool f32 = p.bias_dtype == SB_F32;
+    const uint4* b = reinterpret_cast<const uint4*>((const char*)p.bias + (size_t)n0 * (f32 ? 4 : 2));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < 4 || f32) add[j] = b[j];
+  }
+}
+
+// `next`: the column of the chunk to ask for once `add` has been used (-1: none).
 template <typename TO>
-__device__ __forceinline__ void store_chunk_rowwise(const Tc5Params& p, const uint32_t (&r)[32], int m, int n0) {
+__device__ __forceinline__ void store_chunk_rowwise(const Tc5Params& p, const uint32_t (&r)[32], uint4 (&add)[8], int m,
+                                                    int n0, int next) {
   if (m >= p.M) return;
   float v[32];
 #pragma unroll
@@ -153,46 +197,29 @@ __device__ __forceinline__ void store_chunk_rowwise(const Tc5Params& p, const ui
   if (p.epilogue == SB_EPI_SWIGLU) {
     // columns come as 8 gates, then their 8 up values
     float o[16];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      o[j] = sb_gated<TO>(p, v[j], v[j + 8]);
-      o[j + 8] = sb_gated<TO>(p, v[j + 16], v[j + 24]);
-    }
+    sb_gated_row<TO, 16>(p, v, o);
     store_row((TO*)p.out + (size_t)m * (p.N / 2) + n0 / 2, o, 16);
     return;
   }
-  if (p.epilogue == SB_EPI_BIAS) {
-    if (p.bias_dtype == SB_F32) {
-      const float4* b = reinterpret_cast<const float4*>((const float*)p.bias + n0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 x = b[j];
-        v[4 * j] += x.x; v[4 * j + 1] += x.y; v[4 * j + 2] += x.z; v[4 * j + 3] += x.w;
-      }
-    } else {
-      const uint4* b = reinterpret_cast<const uint4*>((const bf16*)p.bias + n0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint4 x = b[j];
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-          v[8 * j + 2 * k] += f.x;
-          v[8 * j + 2 * k + 1] += f.y;
-        }
-      }
-    }
-  } else if (p.epilogue == SB_EPI_RESIDUAL) {
-    // every residual value is loaded before any store: the output may be the residual itself
-    const float4* res = reinterpret_cast<const float4*>(p.residual + (size_t)m * p.N + n0);
-    float4 x[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = res[j];
+  if (p.epilogue == SB_EPI_RESIDUAL || (p.epilogue == SB_EPI_BIAS && p.bias_dtype == SB_F32)) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      v[4 * j] += x[j].x; v[4 * j + 1] += x[j].y; v[4 * j + 2] += x[j].z; v[4 * j + 3] += x[j].w;
+      v[4 * j] += __uint_as_float(add[j].x); v[4 * j + 1] += __uint_as_float(add[j].y);
+      v[4 * j + 2] += __uint_as_float(add[j].z); v[4 * j + 3] += __uint_as_float(add[j].w);
     }
+    if (next >= 0) chunk_ahead(p, add, m, next);
+  } else if (p.epilogue == SB_EPI_BIAS) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w[4] = {add[j].x, add[j].y, add[j].z, add[j].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
+        v[8 * j + 2 * k] += f.x;
+        v[8 * j + 2 * k + 1] += f.y;
+      }
+    }
+    if (next >= 0) chunk_ahead(p, add, m, next);
   } else if (p.epilogue == SB_EPI_RELU2) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = sb_relu2(v[j]);
@@ -203,8 +230,10 @@ __device__ __forceinline__ void store_chunk_rowwise(const Tc5Params& p, const ui
 template <typename TO, int NC = 32>
 __device__ __forceinline__ void store_chunk(const Tc5Params& p, float* stage, const uint32_t (&r)[32],
                                             int m_base, int n0, int lane) {
-  if (NC == 32 && p.rowwise && n0 + 32 <= p.N) {
-    store_chunk_rowwise<TO>(p, r, m_base + lane, n0);
+  if (NC == 32 && chunk_rowwise(p, n0)) {
+    uint4 add[8];
+    chunk_ahead(p, add, m_base + lane, n0);
+    store_chunk_rowwise<TO>(p, r, add, m_base + lane, n0, -1);
     return;
   }
   __syncwarp();
@@ -963,6 +992,17 @@ bool pair_enabled() {
   return on;
 }
 
+// Row tiles of a group of the pair kernel's tile order (pair_tile).  While all of A stays in L2 beside what else
+// passes through, one group: a column tile's weights leave memory once.  A larger A would be read from memory again for
+// every column tile; groups of about eight row tiles read it once and the weights once a group.  Measured (one group / groups
+// of eight): 16,000 rows, 1,536 x 8,960 460 / 392 us, 33,000 rows 958 / 795; 8,000 rows, 3,584 x 18,944 1,017 / 930,
+// 37,888 x 3,584 (A of 57 MB) 1,765 / 1,700; A of 25 MB (8,000 x 1,536) no difference.
+int pair_group(int tiles_a, int K) {
+  if ((size_t)tiles_a * PAIR_M * K * 2 <= (size_t)40 << 20 || tiles_a < 12) return tiles_a;
+  const int groups = (tiles_a + 4) / 8;
+  return (tiles_a + groups - 1) / groups;
+}
+
 // Tile width of the pair kernel.  The prefill products run at the GPU's power limit, where a
 // partly filled last wave of tiles costs next to nothing (the idle SMs' share of the power lets
 // the busy ones clock higher) and what counts is the work per flop: the columns computed beyond
@@ -1179,6 +1219,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
     p.scratch = splits > 1 ? (float*)scratch : nullptr;
     p.tiles_a = (M + PAIR_M - 1) / PAIR_M;
     p.tiles_b = (N + bn - 1) / bn;
+    p.group_a = pair_group(p.tiles_a, K);
     const long n_tiles = (long)p.tiles_a * p.tiles_b * splits;
     if (n_tiles > 2147483647L) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: too many tiles");
     int clusters = 0;

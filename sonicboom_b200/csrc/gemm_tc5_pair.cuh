@@ -46,6 +46,15 @@ __host__ __device__ constexpr uint32_t pair_instr_desc(int bn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(PAIR_M >> 4) << 24);
 }
 
+// The row tile and the column tile of a tile number.  Row tiles come in groups, and a group's tiles walk its row tiles
+// first: a wave of tiles then shares what it reads through L2 (p.group_a, see pair_group).
+__device__ __forceinline__ void pair_tile(const Tc5Params& p, int tile, int& tile_a, int& tile_b) {
+  const int first = tile / (p.group_a * p.tiles_b) * p.group_a, in_group = tile - first * p.tiles_b;
+  const int rows = min(p.group_a, p.tiles_a - first);
+  tile_a = first + in_group % rows;
+  tile_b = in_group / rows;
+}
+
 template <int BN, int STAGES, typename TO>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS)
 gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -92,17 +101,31 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0 && lane == 0) {
-    // ---- producer (both blocks): this block's half of every stage
-    sb_pdl_wait();
+    // ---- producer (both blocks): this block's half of every stage.  B (the weights) does not depend on the
+    // kernel before this one: the first ring's B tiles are requested before the wait on that kernel.
     const uint32_t full_of_0 = map_to_block(full0, 0);
     uint32_t it = 0;
     bool ok = true;
     for (int unit = first; unit < n_tiles && ok; unit += step) {
-      const int tile = unit / S, split = unit % S;
-      const int tile_a = tile % p.tiles_a, tile_b = tile / p.tiles_a;
+      const int split = unit % S;
+      int tile_a, tile_b;
+      pair_tile(p, unit / S, tile_a, tile_b);
       const int a_row = tile_a * PAIR_M + (int)rank * BM, b_row = tile_b * BN + (int)rank * (BN / 2);
-      const int k_end = min(n_k_all, (split + 1) * k_per);
-      for (int kt = split * k_per; kt < k_end; ++kt, ++it) {
+      int kt = split * k_per;
+      const int k_end = min(n_k_all, kt + k_per);
+      if (unit == first) {
+        const int head = max(0, min(STAGES, k_end - kt));
+        for (int s = 0; s < head; ++s) {
+          if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * pair_stage_bytes(BN));
+          tma_load_2d_pair(tiles + s * pair_stage_bytes(BN) + BM * BK * 2, &map_b, (kt + s) * BK, b_row, full_of_0 + 8 * s);
+        }
+        sb_pdl_wait();
+        for (int s = 0; s < head; ++s)
+          tma_load_2d_pair(tiles + s * pair_stage_bytes(BN), &map_a, (kt + s) * BK, a_row, full_of_0 + 8 * s);
+        kt += head;
+        it = head;
+      }
+      for (; kt < k_end; ++kt, ++it) {
         const uint32_t s = it % STAGES;
         ok = mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, 1);
         if (!ok) break;
@@ -153,13 +176,16 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     const uint32_t acc_empty_of_0 = map_to_block(acc_empty0, 0);
     uint32_t lt = 0;
     for (int unit = first; unit < n_tiles; unit += step, ++lt) {
-      const int tile = unit / S, split = unit % S;
-      const int tile_a = tile % p.tiles_a, tile_b = tile / p.tiles_a;
+      const int split = unit % S;
+      int tile_a, tile_b;
+      pair_tile(p, unit / S, tile_a, tile_b);
       const uint32_t acc = lt & 1;
+      const int m_base = tile_a * PAIR_M + (int)rank * BM + q * 32;
+      uint4 add[8];
+      if (S == 1 && chunk_rowwise(p, tile_b * BN + group * 32)) chunk_ahead(p, add, m_base + lane, tile_b * BN + group * 32);
       if (!mbar_wait(acc_full0 + 8 * acc, (lt >> 1) & 1, 4)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * ACC_COLS;
-      const int m_base = tile_a * PAIR_M + (int)rank * BM + q * 32;
       if (S > 1) {
         // the split's part of the sum as it is: the thread's row, 16 bytes at a time
         const int m = m_base + lane;
@@ -181,8 +207,11 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       for (int c = group; c < BN / 32; c += PAIR_EPI_GROUPS) {
         uint32_t r[32];
         tmem_ld32(t_row + c * 32, r);
-        const int n0 = tile_b * BN + c * 32;
-        if (n0 < p.N) store_chunk<TO>(p, stage, r, m_base, n0, lane);
+        const int n0 = tile_b * BN + c * 32, next = n0 + PAIR_EPI_GROUPS * 32;
+        if (chunk_rowwise(p, n0))
+          store_chunk_rowwise<TO>(p, r, add, m_base + lane, n0, c + PAIR_EPI_GROUPS < BN / 32 && chunk_rowwise(p, next) ? next : -1);
+        else if (n0 < p.N)
+          store_chunk<TO>(p, stage, r, m_base, n0, lane);
       }
       if (BN % 32 && group == (BN / 32) % PAIR_EPI_GROUPS) {   // a last chunk of 16 columns
         uint32_t r[32];
@@ -229,8 +258,7 @@ __global__ void __launch_bounds__(256) tc5_splitk_reduce_kernel(const Tc5Params 
   }
   if (p.epilogue == SB_EPI_SWIGLU) {
     float o[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = sb_gated<TO>(p, v[j], v[j + 8]);
+    sb_gated_row<TO, 8>(p, v, o);
     store_row((TO*)p.out + (size_t)m * (p.N / 2) + n0 / 2, o, 8);
     return;
   }

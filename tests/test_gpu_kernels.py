@@ -220,6 +220,22 @@ def test_product_with_few_rows_splits_k_over_the_pairs(M, N, K):
         assert pm.rel_err(a.float().cpu(), b.float().cpu()) < (1e-5 if a.dtype == torch.float32 else 5e-3)
 
 
+@pytest.mark.parametrize("M", [3072, 3100, 4353])
+def test_product_whose_rows_come_in_groups_of_tiles(M):
+    """Activations of more than 40 MB: the pair kernel's tiles walk groups of row tiles (12, 13 and 18 tiles of 256
+    rows: two groups, of 6 and 6, 7 and 6, 9 and 9), with the residual asked for ahead, in place.  Every value
+    against cuBLAS in float32 on the same bfloat16 operands: the sums differ in their order only, a few
+    float32 roundings of sqrt(K) terms of size one."""
+    N, K = 1072, 7168
+    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, scale=K ** -0.5, seed=1)
+    res = rnd(M, N, seed=3)
+    want = a.float() @ w.float().T + res
+    out = res.clone()
+    ops.linear(a, w, out, ops.EPI_RESIDUAL, residual=out)
+    assert float((out - want).abs().max()) < 1e-4
+    assert ops.tc5_status() == 0
+
+
 @pytest.mark.parametrize("kernel", ["plain", "skinny", "tiled", "tc5"])
 def test_linear_rows_do_not_depend_on_the_batch(kernel):
     a, w = rnd(40, 256, dtype=torch.bfloat16), rnd(88, 256, dtype=torch.bfloat16, seed=1)
