@@ -14,8 +14,8 @@
 //            rows it is a persistent kernel (further down), from 129 rows on one on pairs of SMs
 //            (gemm_tc5_pair.cuh); their epilogue keeps a thread's row and writes 16 bytes at a
 //            time along it (store_chunk_rowwise);
-//   swapped  A = weights (128 weight rows per tile), B = activations (up to 64 rows): the
-//            decode product, which is bound by reading the weights once.  K may be split over
+//   swapped  A = weights (128 weight rows per tile), B = activations (up to 128 rows): the
+//            decode and short-prompt product, which is bound by reading the weights once.  K may be split over
 //            several blocks; their partial tiles go to scratch memory and a second kernel adds
 //            them in split order and runs the epilogue, so the sum's order is fixed.  That
 //            second kernel can also apply the RMSNorm that follows the product
@@ -658,6 +658,17 @@ tc5_reduce_kernel(const Tc5Params p, int bn) {
   }
 }
 
+// Where the partial sums of feature e of row j lie: those of split s are s * stride values on.  The swapped form's lie
+// by tile, [tile][split][row of bn][128 features], the pair kernel's (bn = 0) [split][row][feature].
+__device__ __forceinline__ const float* partial_sums(const Tc5Params& p, int bn, int j, int e, size_t& stride) {
+  if (bn == 0) {
+    stride = (size_t)p.M * p.N;
+    return p.scratch + (size_t)j * p.N + e;
+  }
+  stride = (size_t)bn * BM;
+  return p.scratch + (((size_t)(e / BM) * p.k_splits) * bn + j) * BM + e % BM;
+}
+
 // The same sum for a fused q|k|v product, followed by the rotation and the cache write that
 // rope_store_vec_kernel (elementwise.cu) does on the finished row: the float32 row is neither
 // written nor read again, and the step has one kernel less.  The same sums in the same order and
@@ -700,11 +711,11 @@ tc5_reduce_rope_kernel(const Tc5Params p, int bn, const SbRopeStore r) {
   bf16* cache = (bf16*)r.cache;
   // the sum over the splits of four consecutive features starting at feature n of token t, + bias
   auto sum4 = [&](int n, float (&acc)[4]) {
-    const int tile = n / BM, f = n % BM;
-    const float* base = p.scratch + (((size_t)tile * p.k_splits) * bn + t) * BM + f;
+    size_t stride;
+    const float* base = partial_sums(p, bn, t, n, stride);
     acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
     for (int s = 0; s < p.k_splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(base + (size_t)s * bn * BM);
+      const float4 v = *reinterpret_cast<const float4*>(base + s * stride);
       acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
     }
     if (p.epilogue == SB_EPI_BIAS) {
@@ -807,11 +818,12 @@ tc5_reduce_norm_kernel(const Tc5Params p, int bn, const TW* __restrict__ norm_w,
   for (int i = 0; i < RN_VEC; ++i) {
     const int g = g0 + threadIdx.x + i * RN_THREADS;
     if (g >= g1) continue;
-    const int e = g * 4, tile = e / BM, f = e % BM;
-    const float* base = p.scratch + (((size_t)tile * p.k_splits) * bn + j) * BM + f;
+    const int e = g * 4;
+    size_t stride;
+    const float* base = partial_sums(p, bn, j, e, stride);
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int s = 0; s < p.k_splits; ++s) {
-      const float4 t = *reinterpret_cast<const float4*>(base + (size_t)s * bn * BM);
+      const float4 t = *reinterpret_cast<const float4*>(base + s * stride);
       acc[0] += t.x; acc[1] += t.y; acc[2] += t.z; acc[3] += t.w;
     }
     if (p.epilogue == SB_EPI_BIAS) {
@@ -1037,13 +1049,14 @@ int pair_bn(int M, int N, int clusters) {
 
 namespace {
 int pair_splits(int M, int N, int K, int clusters);
-// Whether the many-rows product runs on pairs of SMs: from 129 rows on, and from 65 rows on when
-// it would split K there (one row tile either way, but the pairs share a tile's K blocks out,
-// while one block per tile would leave most SMs without work).
-bool pair_form(int M, int N, int K, int n_sms) {
-  if (N < 192 || n_sms <= 1 || !pair_enabled()) return false;
-  return M > BM || (M > 64 && pair_splits(M, N, K, n_sms / 2) > 1);
-}
+// Rows of the swapped form.  At 65 to 128 rows a tile of 128 weight rows times 128 tokens costs the tensor cores a
+// third of the time its weights take to arrive, so the product still runs at the weights' pace; on pairs of SMs with K
+// split the 97-row products of the 7B layers took 24 us (q|k|v), 22 (o) and 40 (down), and gate/up 80 us on
+// single SMs, and norm and rotation were kernels of their own: a prompt of 97 tokens 5.62 ms, now 4.07 (15, 15 and 27 us,
+// 63 us).
+constexpr int SWAPPED_ROWS = 128;
+// Whether the many-rows product runs on pairs of SMs.
+bool pair_form(int M, int N, int n_sms) { return M > BM && N >= 192 && n_sms > 1 && pair_enabled(); }
 // K splits of the pair kernel.  When even 256-column tiles leave at least half of the pairs of
 // SMs without one and the inner dimension is long enough, every tile's K blocks are shared out
 // over as many pairs as there are to spare (at most eight, at least eight K blocks each); the
@@ -1077,22 +1090,24 @@ extern "C" void sb_gemm_tc5_force_width(int bn) { g_forced_bn = valid_bn(bn); }
 // The tile width the product of these sizes runs with in its many-rows form (for tests that
 // want every width covered); 0 when that form does not run.
 extern "C" int sb_gemm_tc5_tile_width(int M, int N, int n_sms) {
-  if (M <= 64 || N < 192 || n_sms <= 0) return 0;
-  if (n_sms > 1 && M > BM && pair_enabled()) return pair_bn(M, N, n_sms / 2);
+  if (M <= SWAPPED_ROWS || N < 192 || n_sms <= 0) return 0;
+  if (n_sms > 1 && pair_enabled()) return pair_bn(M, N, n_sms / 2);
   return persistent_bn(M, N, n_sms);
 }
 
 namespace {
 
-int swapped_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : 64); }
+int swapped_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
 
 // How many blocks share one output tile of the swapped form: enough to give every SM two
-// blocks, at least four K tiles each, and no block without work.
-int choose_splits(int N, int K, int n_sms) {
+// blocks, at least four K tiles each (eight with more than 64 rows, whose partial tiles are as large as a weight
+// tile of four), and no block without work.
+int choose_splits(int M, int N, int K, int n_sms) {
   const int tiles = (N + BM - 1) / BM, n_k = (K + BK - 1) / BK;
   int splits = n_sms > 0 ? 2 * n_sms / tiles : 1;       // two blocks fit an SM
   if (splits > 16) splits = 16;
-  if (splits > n_k / 4) splits = n_k / 4;
+  const int least = M > 64 ? 8 : 4;
+  if (splits > n_k / least) splits = n_k / least;
   if (splits < 1) splits = 1;
   const int k_per = (n_k + splits - 1) / splits;
   return (n_k + k_per - 1) / k_per;
@@ -1103,23 +1118,28 @@ int choose_splits(int N, int K, int n_sms) {
 // Bytes of scratch (partial tiles) the swapped form needs for these sizes; 0 when K is not split.
 extern "C" size_t sb_gemm_tc5_scratch_bytes(int M, int N, int K, int n_sms) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (M > 64 && pair_form(M, N, K, n_sms)) {
+  if (pair_form(M, N, n_sms)) {
     // the many-rows form on pairs of SMs, when it splits K: [split][row][column]
     const int splits = pair_splits(M, N, K, n_sms / 2);
     return splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
   }
-  if (M > 64) return 0;
-  const int splits = choose_splits(N, K, n_sms);
+  if (M > SWAPPED_ROWS) return 0;
+  const int splits = choose_splits(M, N, K, n_sms);
   if (splits <= 1) return 0;
   const int tiles = (N + BM - 1) / BM;
   return (size_t)tiles * splits * swapped_bn(M) * BM * sizeof(float);
 }
 
-// Whether the swapped split-K form can finish these rows with the fused reduce + norm kernel.
+// K splits of a product in the form its sizes choose: the swapped form's, or the pair kernel's.
+static int splits_k(int M, int N, int K, int n_sms) {
+  if (M <= SWAPPED_ROWS) return choose_splits(M, N, K, n_sms);
+  return pair_form(M, N, n_sms) ? pair_splits(M, N, K, n_sms / 2) : 1;
+}
+
+// Whether these rows are finished by the fused reduce + norm kernel: every product that splits K.
 static bool norm_fuses(int M, int N, int K, int n_sms, int epilogue, int out_dtype, int form) {
-  const bool normal = form == 1 || (form == 0 && M > 64);
-  return !normal && M <= 64 && choose_splits(N, K, n_sms) > 1 && epilogue != SB_EPI_SWIGLU && epilogue != SB_EPI_RELU2 &&
-         out_dtype == SB_F32 && N % 4 == 0 && N <= RN_MAX_WIDTH;
+  if (epilogue == SB_EPI_SWIGLU || epilogue == SB_EPI_RELU2 || out_dtype != SB_F32 || N % 4 || N > RN_MAX_WIDTH) return false;
+  return form != 1 && splits_k(M, N, K, n_sms) > 1;
 }
 
 extern "C" int sb_gemm_tc5_fuses_norm(int M, int N, int K, int n_sms, int epilogue, int out_dtype,
@@ -1127,18 +1147,67 @@ extern "C" int sb_gemm_tc5_fuses_norm(int M, int N, int K, int n_sms, int epilog
   return norm_fuses(M, N, K, n_sms, epilogue, out_dtype, form) ? 1 : 0;
 }
 
-// Whether the swapped split-K form can finish these rows with the rotation and the cache write.
+// Whether these rows are finished with the rotation and the cache write.
 static bool rope_fuses(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_heads, int hd, int rot,
                        int has_kv) {
-  if (M <= 0 || M > 64 || N <= 0 || K <= 0 || n_q_heads <= 0 || hd <= 0 || (has_kv && n_kv_heads <= 0)) return false;
+  if (M <= 0 || N <= 0 || K <= 0 || n_q_heads <= 0 || hd <= 0 || (has_kv && n_kv_heads <= 0)) return false;
   if (N != (n_q_heads + (has_kv ? 2 * n_kv_heads : 0)) * hd) return false;
   if (rot < 0 || rot > hd || (rot & 7) || ((hd - rot) & 3) || (hd & 3)) return false;
-  return choose_splits(N, K, n_sms) > 1;
+  return splits_k(M, N, K, n_sms) > 1;
 }
 
 extern "C" int sb_gemm_tc5_fuses_rope(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_heads,
                                       int hd, int rot, int has_kv) {
   return rope_fuses(M, N, K, n_sms, n_q_heads, n_kv_heads, hd, rot, has_kv) ? 1 : 0;
+}
+
+// The kernels that finish a product whose K was split (`bn` as in partial_sums).  They take the pair kernel's partial
+// sums too: prompts of 180 and 300 tokens of the 7B model 5.91 to 4.90 and 7.62 to 7.20 ms, of 300 of the 1.5B 4.13 to 3.45.
+static int reduce_rope(const Tc5Params& p, int bn, const SbRopeStore& rope, int n_sms, cudaStream_t stream) {
+  const size_t smem = (size_t)(rope.rot > 0 ? rope.rot : 2) * sizeof(float);
+  // the heads of a token are shared out over enough blocks for two per SM, at least four
+  const int n_heads = rope.n_q_heads + (rope.cache ? 2 * rope.n_kv_heads : 0);
+  int shares = n_sms > 0 ? (2 * n_sms + p.M - 1) / p.M : 4;
+  shares = shares < 4 ? 4 : (shares > n_heads ? n_heads : shares);
+  sb_launch<SB_K_REDUCE>(tc5_reduce_rope_kernel, dim3((unsigned)p.M, (unsigned)shares), dim3(RR_THREADS), smem,
+                         stream, p, bn, rope);
+  SB_CHECK_LAUNCH("sb_gemm_tc5 (reduce + rotation)");
+  return SB_OK;
+}
+
+static int reduce_norm(const Tc5Params& p, int bn, const SbLinearExtras& norm, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(RN_CLUSTER, (unsigned)p.M);
+  cfg.blockDim = dim3(RN_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = RN_CLUSTER;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (sb_pdl_enabled() & SB_K_REDUCE) ? 2 : 1;
+  SB_DISPATCH_DTYPE(norm.norm_weight_dtype, TW, {
+    SB_DISPATCH_DTYPE(norm.norm_out_dtype, TN, {
+      cudaLaunchKernelEx(&cfg, tc5_reduce_norm_kernel<TW, TN>, p, bn, (const TW*)norm.norm_weight,
+                         norm.norm_eps, (TN*)norm.norm_out, (const TW*)norm.norm_weight2, (TN*)norm.norm_out2);
+    });
+  });
+  SB_CHECK_LAUNCH("sb_gemm_tc5 (reduce + norm)");
+  return SB_OK;
+}
+
+// Whether rows may be read and written 16 bytes at a time (SB_TC5_ROWWISE=0: never, for measurements).
+static bool rowwise_on() {
+  static const bool on = [] { const char* e = getenv("SB_TC5_ROWWISE"); return !(e && e[0] == '0'); }();
+  return on;
+}
+
+// Whether the workspace holds the pair kernel's partial sums.
+static bool pair_scratch(int M, int N, int splits, const void* scratch, size_t bytes) {
+  return scratch && bytes >= (size_t)splits * M * N * sizeof(float) && ((uintptr_t)scratch & 255) == 0;
 }
 
 static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N,
@@ -1169,7 +1238,10 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
         !sb_valid_dtype(norm->norm_out_dtype) || !(norm->norm_eps >= 0.0f))
       SB_FAIL(SB_ERR_ARG, "sb_gemm_tc5: norm output, dtype codes %d %d or eps %g",
               norm->norm_weight_dtype, norm->norm_out_dtype, norm->norm_eps);
+    const bool pairs = M > SWAPPED_ROWS && norm_fuses(M, N, K, n_sms, epilogue, out_dtype, form);
     if (!norm_fuses(M, N, K, n_sms, epilogue, out_dtype, form) ||
+        (pairs && (!rowwise_on() || pair_clusters<256, float>() <= 0 ||
+                   !pair_scratch(M, N, pair_splits(M, N, K, n_sms / 2), scratch, scratch_bytes))) ||
         (((uintptr_t)norm->norm_weight | (uintptr_t)norm->norm_out | (uintptr_t)norm->norm_weight2 |
           (uintptr_t)norm->norm_out2 | (uintptr_t)out |
           (uintptr_t)residual | (uintptr_t)bias) & 15)) {
@@ -1197,9 +1269,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
   p.M = M; p.N = N; p.K = K; p.epilogue = epilogue; p.bias = bias; p.bias_dtype = bias_dtype;
   p.residual = residual; p.out = out; p.k_splits = 1; p.scratch = nullptr;
   // rows of the output, the residual and the bias chunks start on 16-byte boundaries
-  // (SB_TC5_ROWWISE=0: never, for measurements)
-  static const bool rowwise_on = [] { const char* e = getenv("SB_TC5_ROWWISE"); return !(e && e[0] == '0'); }();
-  p.rowwise = rowwise_on && N % 16 == 0 && (((uintptr_t)out | (uintptr_t)residual | (uintptr_t)bias) & 15) == 0;
+  p.rowwise = rowwise_on() && N % 16 == 0 && (((uintptr_t)out | (uintptr_t)residual | (uintptr_t)bias) & 15) == 0;
   p.gate_limit = extras && epilogue == SB_EPI_SWIGLU ? extras->gate_limit : 0.0f;
   p.gate_slope = extras ? extras->gate_slope : 1.0f;
   p.gate_kind = extras && epilogue == SB_EPI_SWIGLU ? extras->gate_kind : SB_GATE_SILU;
@@ -1207,13 +1277,16 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
   p.warm_bytes = extras ? sb_warm_bytes(extras->warm, extras->warm_bytes) : 0;
   CUtensorMap ma, mb;
   // form: 0 picks by the number of rows, 1 forces the normal form, 2 the swapped form
-  const bool normal = form == 1 || (form == 0 && M > 64);
-  if (form == 2 && M > 64) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: the swapped form takes at most 64 rows");
-  if (normal && M > 64 && pair_form(M, N, K, n_sms)) {
+  const bool normal = form == 1 || (form == 0 && M > SWAPPED_ROWS);
+  if (form == 2 && M > SWAPPED_ROWS)
+    SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: the swapped form takes at most %d rows", SWAPPED_ROWS);
+  if (normal && pair_form(M, N, n_sms)) {
     // at least two row tiles, wide output: the persistent kernel on pairs of SMs
-    int splits = p.rowwise ? pair_splits(M, N, K, n_sms / 2) : 1;
-    if (splits > 1 && (!scratch || scratch_bytes < (size_t)splits * M * N * sizeof(float) || ((uintptr_t)scratch & 255)))
+    int splits = p.rowwise || rope ? pair_splits(M, N, K, n_sms / 2) : 1;
+    if (splits > 1 && !pair_scratch(M, N, splits, scratch, scratch_bytes)) {
+      if (rope) SB_FAIL(SB_ERR_ARG, "sb_gemm_tc5: scratch for the partial sums is missing");
       splits = 1;                                       // no room for the partial sums: the whole K per tile
+    }
     const int bn = splits > 1 ? 256 : pair_bn(M, N, n_sms / 2);
     p.k_splits = splits;
     p.scratch = splits > 1 ? (float*)scratch : nullptr;
@@ -1229,6 +1302,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
     SB_TC5_PAIR_CLUSTERS(192)
 #undef SB_TC5_PAIR_CLUSTERS
     if (splits > 1) clusters = pair_clusters<256, float>();   // the kernel that writes the partial sums
+    if (rope && clusters <= 0) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: no pairs of SMs for the fused rotation");
     if (clusters > 0) {                               // else: the one-block kernel below
       if (!make_map(&ma, A, M, K, BM) || !make_map(&mb, W, N, K, bn / 2))
         SB_FAIL(SB_ERR_CUDA, "sb_gemm_tc5: cuTensorMapEncodeTiled failed");
@@ -1236,6 +1310,8 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
       if (splits > 1) {
         // the partial sums, then their sum in split order with the epilogue
         if (int rc = launch_pair<256, float>(ma, mb, p, clusters, stream)) return rc;
+        if (rope) return reduce_rope(p, 0, *rope, n_sms, stream);
+        if (norm) return reduce_norm(p, 0, *norm, stream);
         const long work = (long)M * (N / 16);
         const dim3 rgrid((unsigned)((work + 255) / 256));
         if (out_dtype == SB_F32) sb_launch<SB_K_REDUCE>(tc5_splitk_reduce_kernel<float>, rgrid, dim3(256), 0, stream, p);
@@ -1287,7 +1363,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
   const int bn = swapped_bn(M);
   p.tiles_a = (N + BM - 1) / BM;
   p.tiles_b = 1;
-  const int splits = choose_splits(N, K, n_sms);
+  const int splits = choose_splits(M, N, K, n_sms);
   p.k_splits = splits;
   if (splits > 1) {
     const size_t need = sb_gemm_tc5_scratch_bytes(M, N, K, n_sms);
@@ -1314,43 +1390,12 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
                            : launch<BN_, ST_, true, bf16>(ma, mb, p, blocks, stream);
   if (bn == 16) { SB_TC5_SWAPPED(16, 4) }
   else if (bn == 32) { SB_TC5_SWAPPED(32, 5) }
-  else { SB_TC5_SWAPPED(64, 4) }
+  else if (bn == 64) { SB_TC5_SWAPPED(64, 4) }
+  else { SB_TC5_SWAPPED(128, 3) }
 #undef SB_TC5_SWAPPED
   if (rc != SB_OK || splits <= 1) return rc;
-  if (rope) {
-    const size_t smem = (size_t)(rope->rot > 0 ? rope->rot : 2) * sizeof(float);
-    // the heads of a token are shared out over enough blocks for two per SM, at least four
-    const int n_heads = rope->n_q_heads + (rope->cache ? 2 * rope->n_kv_heads : 0);
-    int shares = n_sms > 0 ? (2 * n_sms + M - 1) / M : 4;
-    shares = shares < 4 ? 4 : (shares > n_heads ? n_heads : shares);
-    sb_launch<SB_K_REDUCE>(tc5_reduce_rope_kernel, dim3((unsigned)M, (unsigned)shares), dim3(RR_THREADS), smem,
-                           stream, p, bn, *rope);
-    SB_CHECK_LAUNCH("sb_gemm_tc5 (reduce + rotation)");
-    return SB_OK;
-  }
-  if (norm) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(RN_CLUSTER, (unsigned)M);
-    cfg.blockDim = dim3(RN_THREADS);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = RN_CLUSTER;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (sb_pdl_enabled() & SB_K_REDUCE) ? 2 : 1;
-    SB_DISPATCH_DTYPE(norm->norm_weight_dtype, TW, {
-      SB_DISPATCH_DTYPE(norm->norm_out_dtype, TN, {
-        cudaLaunchKernelEx(&cfg, tc5_reduce_norm_kernel<TW, TN>, p, bn, (const TW*)norm->norm_weight,
-                           norm->norm_eps, (TN*)norm->norm_out, (const TW*)norm->norm_weight2, (TN*)norm->norm_out2);
-      });
-    });
-    SB_CHECK_LAUNCH("sb_gemm_tc5 (reduce + norm)");
-    return SB_OK;
-  }
+  if (rope) return reduce_rope(p, bn, *rope, n_sms, stream);
+  if (norm) return reduce_norm(p, bn, *norm, stream);
   const int n_out = epilogue == SB_EPI_SWIGLU ? N / 2 : N;
   const long work = (long)((n_out + 3) / 4) * M;
   const dim3 rgrid((unsigned)((work + 255) / 256));

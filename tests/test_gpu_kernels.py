@@ -283,6 +283,39 @@ def test_linear_followed_by_a_norm(M, N, K, ndtype):
     assert ops.tc5_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 520, 2048), (97, 3584, 1032), (128, 260, 4096), (129, 528, 2048), (300, 1040, 4096),
+                                   (512, 3584, 1200), (1500, 1536, 1536)])
+@pytest.mark.parametrize("pair", [False, True])
+def test_norms_ride_on_every_product_that_splits_k(M, N, K, pair):
+    """65 to 128 rows stream the weights past tiles of 128 tokens, more rows run on pairs of SMs; where either splits K
+    the kernel that adds the partial sums also writes the norm (or two), with the residual updated in place:
+    the product's bits are those without a norm, the norm's within the rounding of bfloat16 (half an ulp is 2^-8)."""
+    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, scale=K ** -0.5, seed=1)
+    res, bias = rnd(M, N, seed=3), rnd(N, dtype=torch.bfloat16, seed=2)
+    weights = [(1 + 0.3 * rnd(N, seed=4 + i)).to(torch.bfloat16) for i in range(2)]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for epi in (ops.EPI_NONE, ops.EPI_BIAS, ops.EPI_RESIDUAL):
+        assert bool(ops.lib().sb_gemm_tc5_fuses_norm(M, N, K, sms, epi, 0, 0))
+        out, plain = res.clone(), res.clone()
+        ops.linear(a, w, plain, epi, bias=bias if epi == ops.EPI_BIAS else None,
+                   residual=plain if epi == ops.EPI_RESIDUAL else None)
+        normed = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+        norm = (weights[0], 3e-5, normed[0]) + ((weights[1], normed[1]) if pair else ())
+        ops.linear(a, w, out, epi, bias=bias if epi == ops.EPI_BIAS else None,
+                   residual=out if epi == ops.EPI_RESIDUAL else None, norm=norm)
+        assert torch.equal(out, plain)
+        close(out, linear_ref(a, w, epi, bias, res), 1e-5)
+        for i in range(1 + pair):
+            close(normed[i], rmsnorm_ref(out, weights[i], 3e-5), 5e-3)
+    assert ops.tc5_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 1040, 200), (100, 272, 72), (127, 400, 520), (128, 1040, 4096)])
+def test_product_of_up_to_128_rows(M, N, K):
+    """Tiles of 128 tokens with one block a tile and with K split; rows and features that end inside a tile."""
+    _every_epilogue(M, N, K)
+
+
 def test_fused_gate_up_layout():
     gate, up = rnd(32, 8), rnd(32, 8, seed=1)
     f = interleave_gate_up(gate, up)
@@ -757,6 +790,41 @@ def test_fused_projection_rotation_and_cache_write(hq, hkv, hd, K, rot, rows):
     ops.linear(a, w[:hq * hd].contiguous(), qkv, ops.EPI_BIAS, bias=bias[:hq * hd].contiguous())
     ops.rope_store(qkv, hq, hkv, hd, rot, inv, plan.row_seq, plan.row_pos, None, None, 64, None, qb)
     assert pm.rel_err(qa.float().cpu(), qb.float().cpu()) < 4e-3
+    assert ops.tc5_status() == 0
+
+
+@pytest.mark.parametrize("rows,K", [(97, 3584), (128, 1536), (200, 3584), (500, 3584)])
+def test_rotation_rides_on_the_split_products_of_prompts(rows, K):
+    """The same fusion at a prompt's rows (tiles of 128 tokens, pairs of SMs with K split): 28 query and 4 key/value heads of
+    128, against the same product followed by `rope_store`, to an ulp of bfloat16."""
+    dt, hq, hkv, hd = torch.bfloat16, 28, 4, 128
+    N = (hq + 2 * hkv) * hd
+    a, w, bias = rnd(rows, K, dtype=dt), rnd(N, K, dtype=dt, scale=K ** -0.5, seed=1), rnd(N, dtype=dt, seed=2)
+    inv = torch.from_numpy((10000.0 ** (-np.arange(hd // 2) / (hd // 2))).astype(np.float32)).to(DEV)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert bool(ops.lib().sb_gemm_tc5_fuses_rope(rows, N, K, sms, hq, hkv, hd, hd, 1))
+    got = []
+    for fused in (True, False):
+        cache = make_cache(hkv, hd, 0, dt, max_tokens=1024)
+        slots = [cache.open() for _ in range(2)]
+        lens = [rows // 3, rows - rows // 3]
+        for i, (s, n) in enumerate(zip(slots, lens)):
+            cache.reserve(s, 37 * i + n)
+            cache.advance(s, 37 * i)
+        plan = StepPlan(cache, [StepEntry(s, [0] * n, []) for s, n in zip(slots, lens)], DEV)
+        g, storage = plan.groups[0], cache.groups[0].entry_storage(0)
+        q = torch.empty(rows, hq, hd, dtype=dt, device=DEV)
+        where = (hq, hkv, hd, hd, inv, plan.row_seq, plan.row_pos, g.page_off, g.page_ids, g.page_size, storage, q)
+        if fused:
+            ops.qkv_rope_store(a, w, bias, *where)
+        else:
+            qkv = torch.empty(rows, N, device=DEV)
+            ops.linear(a, w, qkv, ops.EPI_BIAS, bias=bias)
+            ops.rope_store(qkv, *where)
+        got.append((q.float().cpu(), storage.float().cpu()))
+    assert float(got[1][1].abs().max()) > 0
+    for x, y in zip(*got):
+        assert pm.rel_err(x, y) < 4e-3
     assert ops.tc5_status() == 0
 
 
