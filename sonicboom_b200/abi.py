@@ -36,6 +36,8 @@ CORE = {
     "sb_gemm_plain": ("i", _GEMM),
     "sb_gemm_skinny": ("i", _GEMM),
     "sb_gemm_skinny_gated": ("i", "pipiiiipiffis"),
+    "sb_gemm_skinny_takes_rope": ("i", "iiiiiii"),
+    "sb_gemm_skinny_rope": ("i", "pipiiiipips"),
     "sb_gemm_tiled": ("i", _GEMM),
     "sb_gemm_tc5": ("i", _GEMM[:-1] + "pziis"),
     "sb_gemm_tc5_ex": ("i", _GEMM[:-1] + "pziips"),

@@ -62,16 +62,28 @@ constexpr int SK_UNROLL = 8;
 // of its W rows and of its activation row; the four pairs feed two MMAs.  The MMA only needs
 // A and B to agree on which k sits in which slot, so this contiguous 16-byte-per-thread
 // assignment is as good as the canonical interleaved one.
-template <int NT, typename TO>
+//
+// ROPE (up to 8 rows): the product is a fused [q | k | v] projection and the rotation and the cache write that follow it
+// happen here.  A block then takes rows e ... e + 7 of a head and the rows half the rotated part further on, so that
+// the thread that adds up one value of a pair adds up both.  As a kernel of its own the rotation took 2.8 us between two
+// kernels that wait for each other (a decode step of eight 7B sequences 3.083 to 3.033 ms, of one 2.832 to 2.797).
+template <int NT, typename TO, bool ROPE>
 __global__ void __launch_bounds__(SK_WARPS * 32)
 gemm_skinny_kernel(const bf16* X, const bf16* __restrict__ W, int M, int N, int K,
                    int epilogue, const void* __restrict__ bias, int bias_dtype,
-                   const float* residual, TO* out, float gate_limit, float gate_slope) {
+                   const float* residual, TO* out, float gate_limit, float gate_slope, const SbRopeStore rope) {
   __shared__ float partial[SK_WARPS][NT][32][4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int m0 = blockIdx.x * 16;
+  int m0 = blockIdx.x * 16, m1 = m0 + 8;             // the first of the block's two groups of eight rows of W
+  bool rotated = false;
+  if (ROPE) {
+    const int per_head = rope.hd / 16, head0 = blockIdx.x / per_head * rope.hd, i = blockIdx.x % per_head;
+    rotated = i < rope.rot / 16;
+    m0 = head0 + (rotated ? 8 * i : 16 * i);
+    m1 = m0 + (rotated ? rope.rot / 2 : 8);
+  }
   const uint4* w0 = (const uint4*)(W + (size_t)min(m0 + g, N - 1) * K) + t;
-  const uint4* w1 = (const uint4*)(W + (size_t)min(m0 + g + 8, N - 1) * K) + t;
+  const uint4* w1 = (const uint4*)(W + (size_t)min(m1 + g, N - 1) * K) + t;
   const uint4* xp[NT];
   bool xok[NT];
 #pragma unroll
@@ -119,6 +131,46 @@ gemm_skinny_kernel(const bf16* X, const bf16* __restrict__ W, int M, int N, int 
     for (int i = 0; i < 4; ++i) partial[warp][nt][lane][i] = acc[nt][i];
   __syncthreads();
 
+  if constexpr (ROPE) {
+    // thread e: values n_lo and n_hi = the same place of the second group, of batch row e / 8
+    const int r = threadIdx.x & 7, b = threadIdx.x >> 3;
+    if (b >= M) return;
+    const int src_lane = r * 4 + ((b & 7) >> 1), reg = b & 1;
+    float lo = 0.0f, hi = 0.0f;
+#pragma unroll
+    for (int w = 0; w < SK_WARPS; ++w) {
+      lo += partial[w][0][src_lane][reg];
+      hi += partial[w][0][src_lane][reg + 2];
+    }
+    const int n_lo = m0 + r, n_hi = m1 + r, head = m0 / rope.hd, e_lo = n_lo - head * rope.hd, e_hi = n_hi - head * rope.hd;
+    if (epilogue == SB_EPI_BIAS) {
+      lo += bias_dtype == SB_F32 ? load_bias<float>(bias, n_lo) : load_bias<bf16>(bias, n_lo);
+      hi += bias_dtype == SB_F32 ? load_bias<float>(bias, n_hi) : load_bias<bf16>(bias, n_hi);
+    }
+    const int pos = rope.row_pos[b];
+    if (rotated && head < rope.n_q_heads + rope.n_kv_heads) {
+      const float theta = (float)pos * rope.inv_freq[e_lo], c = cosf(theta), s = sinf(theta);
+      const float a = lo;
+      lo = sb_rot_lo(a, hi, c, s);
+      hi = sb_rot_hi(a, hi, c, s);
+    }
+    bf16* dst;
+    if (head < rope.n_q_heads) {
+      dst = (bf16*)rope.q_out + ((size_t)b * rope.n_q_heads + head) * rope.hd;
+    } else {
+      // a position without a page in its own sequence's list writes no key and no value
+      const int seq = rope.row_seq[b], first = rope.page_off[seq], n_pages = rope.page_off[seq + 1] - first;
+      const int pi = pos / rope.page_size;
+      const int page = pos >= 0 && pi < n_pages ? rope.page_ids[first + pi] : -1;
+      if (page < 0) return;
+      const int kv = head - rope.n_q_heads, is_v = kv >= rope.n_kv_heads;       // k heads, then v heads
+      dst = (bf16*)rope.cache + ((((size_t)page * 2 + is_v) * rope.n_kv_heads + (kv - is_v * rope.n_kv_heads)) * rope.page_size
+                                 + pos % rope.page_size) * rope.hd;
+    }
+    dst[e_lo] = __float2bfloat16_rn(lo);
+    dst[e_hi] = __float2bfloat16_rn(hi);
+    return;
+  }
   // Epilogue: thread e takes W row r = e % 16 of batch row b = e / 16, sums the warps'
   // partial results in warp order, and applies the epilogue.
   for (int e = threadIdx.x; e < 16 * 8 * NT; e += SK_WARPS * 32) {
@@ -158,8 +210,8 @@ int launch_skinny(const bf16* X, const bf16* W, int M, int N, int K, int epilogu
                   int out_dtype, float gate_limit, float gate_slope, cudaStream_t stream) {
   const int blocks = (N + 15) / 16;
   SB_DISPATCH_DTYPE(out_dtype, TO, {
-    sb_launch<SB_K_SKINNY>(gemm_skinny_kernel<NT, TO>, dim3(blocks), dim3(SK_WARPS * 32), 0, stream,
-        X, W, M, N, K, epilogue, bias, bias_dtype, residual, (TO*)out, gate_limit, gate_slope);
+    sb_launch<SB_K_SKINNY>(gemm_skinny_kernel<NT, TO, false>, dim3(blocks), dim3(SK_WARPS * 32), 0, stream,
+        X, W, M, N, K, epilogue, bias, bias_dtype, residual, (TO*)out, gate_limit, gate_slope, SbRopeStore{});
   });
   SB_CHECK_LAUNCH("sb_gemm_skinny");
   return SB_OK;
@@ -359,6 +411,28 @@ extern "C" int sb_gemm_skinny_gated(const void* A, int a_dtype, const void* W, i
     SB_FAIL(SB_ERR_ARG, "sb_gemm_skinny_gated: limit %g must be positive", gate_limit);
   return gemm_skinny(A, a_dtype, W, w_dtype, M, N, K, SB_EPI_SWIGLU, nullptr, 0, nullptr, out, out_dtype,
                      gate_kind == SB_GATE_GELU_TANH ? -1.0f : gate_limit, gate_slope, stream);
+}
+
+extern "C" int sb_gemm_skinny_takes_rope(int M, int N, int n_q_heads, int n_kv_heads, int hd, int rot, int has_kv) {
+  return M > 0 && M <= 8 && n_q_heads > 0 && hd > 0 && hd % 16 == 0 && rot >= 0 && rot <= hd && rot % 16 == 0 &&
+         (!has_kv || n_kv_heads > 0) && N == (n_q_heads + (has_kv ? 2 * n_kv_heads : 0)) * hd;
+}
+
+extern "C" int sb_gemm_skinny_rope(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
+                                   const void* bias, int bias_dtype, const SbRopeStore* rope, cudaStream_t stream) {
+  if (int rc = check_bf16_product("sb_gemm_skinny_rope", a_dtype, w_dtype, K, A, W)) return rc;
+  if (!A || !W || K <= 0 || !rope) SB_FAIL(SB_ERR_ARG, "sb_gemm_skinny_rope: operands missing");
+  if (!sb_gemm_skinny_takes_rope(M, N, rope->n_q_heads, rope->n_kv_heads, rope->hd, rope->rot, rope->cache != nullptr))
+    SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_skinny_rope: these sizes do not take the fused rotation (see sb_gemm_skinny_takes_rope)");
+  if (!rope->q_out || !rope->inv_freq || !rope->row_pos ||
+      (rope->cache && (!rope->row_seq || !rope->page_off || !rope->page_ids || rope->page_size <= 0)))
+    SB_FAIL(SB_ERR_ARG, "sb_gemm_skinny_rope: rotation arguments missing");
+  if (bias && !sb_valid_dtype(bias_dtype)) SB_FAIL(SB_ERR_ARG, "sb_gemm_skinny_rope: bias dtype %d", bias_dtype);
+  sb_launch<SB_K_SKINNY>(gemm_skinny_kernel<1, bf16, true>, dim3(N / 16), dim3(SK_WARPS * 32), 0, stream, (const bf16*)A,
+                         (const bf16*)W, M, N, K, bias ? SB_EPI_BIAS : SB_EPI_NONE, bias, bias_dtype, (const float*)nullptr,
+                         (bf16*)nullptr, 0.0f, 1.0f, *rope);
+  SB_CHECK_LAUNCH("sb_gemm_skinny_rope");
+  return SB_OK;
 }
 
 extern "C" int sb_gemm_tiled(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N,

@@ -142,6 +142,11 @@ int sb_gemm_skinny(const void* A, int a_dtype, const void* W, int w_dtype, int M
 int sb_gemm_skinny_gated(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
                          void* out, int out_dtype, float gate_limit, float gate_slope, int gate_kind,
                          sb_stream_t stream);
+/* sb_gemm_skinny of a fused [q | k | v] projection whose rows are rotated and written by the same kernel (up to 8 rows,
+ * head and rotated sizes that are multiples of 16: sb_gemm_skinny_takes_rope).  bias may be null. */
+int sb_gemm_skinny_takes_rope(int M, int N, int n_q_heads, int n_kv_heads, int hd, int rot, int has_kv);
+int sb_gemm_skinny_rope(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
+                        const void* bias, int bias_dtype, const SbRopeStore* rope, sb_stream_t stream);
 int sb_gemm_tiled(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
                   int epilogue, const void* bias, int bias_dtype, const float* residual,
                   void* out, int out_dtype, sb_stream_t stream);

@@ -342,20 +342,25 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
                    q_out: torch.Tensor) -> torch.Tensor:
     """The fused [q | k | v] projection of the rows `h` (+ bias), the rotation of q and k, q into
     `q_out` [rows, heads, hd] and k, v into the cache pages (`cache=None`: the weight holds the
-    query rows only).  Where the split-K decode form of the tcgen05 product runs (9 to 64 rows of
-    bfloat16), its reduce kernel does the rotation and the cache write too and the float32 row
-    is never written; else the product and `rope_store` run one after the other."""
+    query rows only).  Where the weight-streaming kernel runs (up to 8 rows of bfloat16) or the tcgen05 product
+    splits K (9 to several hundred rows), the kernel that finishes the sums does the rotation and the cache write too
+    and the float32 row is never written; else the product and `rope_store` run one after the other."""
     M, K = h.shape
     N = w.shape[0]
     has_kv = cache is not None
     l = lib()
-    fused = (h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and q_out.dtype == torch.bfloat16
-             and (not has_kv or cache.dtype == torch.bfloat16) and K % 8 == 0
-             and (bias is None or bias.numel() == N)
-             and _pick_kernel(M, N, K, h.device) == "tc5"
-             and bool(l.sb_gemm_tc5_fuses_rope(M, N, K, _sm_count(h.device), n_q_heads, n_kv_heads, head_dim,
-                                              rotary_dim, 1 if has_kv else 0)))
-    if not fused:
+    fused = None
+    if (h.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and q_out.dtype == torch.bfloat16
+            and (not has_kv or cache.dtype == torch.bfloat16) and K % 8 == 0
+            and (bias is None or bias.numel() == N)):
+        kernel = _pick_kernel(M, N, K, h.device)
+        if kernel == "tc5" and l.sb_gemm_tc5_fuses_rope(M, N, K, _sm_count(h.device), n_q_heads, n_kv_heads, head_dim,
+                                                        rotary_dim, 1 if has_kv else 0):
+            fused = kernel
+        elif kernel == "skinny" and l.sb_gemm_skinny_takes_rope(M, N, n_q_heads, n_kv_heads, head_dim, rotary_dim,
+                                                                1 if has_kv else 0):
+            fused = kernel
+    if fused is None:
         qkv = torch.empty((M, N), dtype=torch.float32, device=h.device)
         linear(h, w, qkv, EPI_BIAS if bias is not None else EPI_NONE, bias=bias)
         return rope_store(qkv, n_q_heads, n_kv_heads, head_dim, rotary_dim, inv_freq, row_seq, row_pos,
@@ -366,6 +371,11 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
                      _i32(page_off, "page_off") if has_kv else None,
                      _i32(page_ids, "page_ids") if has_kv else None, page_size,
                      cache.data_ptr() if has_kv else None, _ptr(q_out))
+    if fused == "skinny":
+        _check(l.sb_gemm_skinny_rope(_ptr(h), BF16, _ptr(w), BF16, M, N, K, _ptr(bias),
+                                     _code(bias.dtype) if bias is not None else 0, ctypes.byref(rope), _stream()),
+               "q|k|v product with rotation (weight-streaming kernel)")
+        return q_out
     extras = LinearExtras()
     extras.rope = ctypes.pointer(rope)
     ws = _tc5_workspace(M, N, K, h.device)

@@ -793,6 +793,37 @@ def test_fused_projection_rotation_and_cache_write(hq, hkv, hd, K, rot, rows):
     assert ops.tc5_status() == 0
 
 
+@pytest.mark.parametrize("rows,hq,hkv,hd,rot", [(1, 12, 2, 128, 128), (8, 28, 4, 128, 128), (5, 3, 1, 16, 16), (7, 4, 2, 80, 48),
+                                                (8, 4, 4, 64, 0)])
+@pytest.mark.parametrize("bias_dtype", [None, "float32", "bfloat16"])
+def test_rotation_rides_on_the_weight_streaming_product(rows, hq, hkv, hd, rot, bias_dtype):
+    """Up to 8 rows, each of another sequence; the last one's position has no page of its own (its queries are written, its
+    keys and values nowhere).  The same bits as the weight-streaming product followed by `rope_store`."""
+    dt, K, N = torch.bfloat16, 520, (hq + 2 * hkv) * hd
+    a, w = rnd(rows, K, dtype=dt), rnd(N, K, dtype=dt, scale=K ** -0.5, seed=1)
+    bias = rnd(N, dtype=DT[bias_dtype], seed=2) if bias_dtype else None
+    inv = torch.from_numpy((10000.0 ** (-np.arange(max(rot // 2, 1)) / max(rot // 2, 1))).astype(np.float32)).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)             # noqa: E731
+    pages = 2 * rows
+    order = torch.randperm(pages, generator=torch.Generator().manual_seed(rows)).tolist()
+    pos = [(37 * i + 63) % 128 for i in range(rows - 1)] + [128]
+    where = (inv, i32(list(range(rows))), i32(pos), i32([2 * i for i in range(rows + 1)]), i32(order), 64)
+    assert bool(ops.lib().sb_gemm_skinny_takes_rope(rows, N, hq, hkv, hd, rot, 1))
+    got = []
+    for fused in (True, False):
+        cache = torch.zeros(pages, 2, hkv, 64, hd, dtype=dt, device=DEV)
+        q = torch.zeros(rows, hq, hd, dtype=dt, device=DEV)
+        if fused:
+            ops.qkv_rope_store(a, w, bias, hq, hkv, hd, rot, *where, cache, q)
+        else:
+            qkv = torch.empty(rows, N, device=DEV)
+            ops.linear(a, w, qkv, ops.EPI_BIAS if bias is not None else ops.EPI_NONE, bias=bias, kernel="skinny")
+            ops.rope_store(qkv, hq, hkv, hd, rot, *where, cache, q)
+        got.append((q, cache))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert int((got[0][1] != 0).any(-1).sum()) == 2 * hkv * (rows - 1)
+
+
 @pytest.mark.parametrize("rows,K", [(97, 3584), (128, 1536), (200, 3584), (500, 3584)])
 def test_rotation_rides_on_the_split_products_of_prompts(rows, K):
     """The same fusion at a prompt's rows (tiles of 128 tokens, pairs of SMs with K split): 28 query and 4 key/value heads of
