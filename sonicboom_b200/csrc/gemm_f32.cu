@@ -1,11 +1,12 @@
-// The float32 products of the 32-bit path: out[M,N] = A[M,K] . W[N,K]^T with float32 operands, FFMA
-// only (no tensor cores, no reduced-precision mode).  Two forms, chosen in sb_gemm_f32:
+// The float32 products of the 32-bit path: out[M,N] = A[M,K] . W[N,K]^T with float32 operands.  More than 32 rows (16 of wide
+// products) at K of 256 or more run on the tensor cores with operands split in two (gemm_f32_tc5.cu); here are two FFMA
+// forms, chosen in sb_gemm_f32:
 //
 // * gemm_f32_rows_kernel, few rows: bound by reading W once.  A block takes R weight rows; its warps share K in
 //   chunks of 128 values, a lane reads 16 bytes of every weight row past L1 and 16 bytes of every activation row
 //   (which the SM's blocks keep in L1), so that a warp's loads run along the rows.  Sums: a lane's terms in
 //   ascending order, then the lanes in a fixed tree, then the warps in order.
-// * gemm_f32_tile_kernel, many rows: bound by FFMA issue and shared-memory loads.  128 threads compute 16 TM x 128
+// * gemm_f32_tile_kernel, many rows at a short K: bound by FFMA issue and shared-memory loads.  128 threads compute 16 TM x 128
 //   outputs, TM x 16 a thread: a load from shared memory costs its bytes times its lanes whether lanes share the
 //   address or not, so a thread's tile is as large as the registers allow (TM 8: 24 values loaded for 128 FMA) and
 //   two products go into one packed FMA.  Tiles lie [k][row] in shared memory.  Where the tiles leave SMs idle a
@@ -393,12 +394,21 @@ int run_f32(const F32Args& p, TO* out, cudaStream_t stream) {
 
 }  // namespace
 
+// The tensor-core form (gemm_f32_tc5.cu).  Below this K its splitting of the operands (22 to 23 bits) would be its whole error,
+// 1.4e-7, where 256 float32 terms added one after the other have as much of their own.  From 17 rows on it takes the wide products,
+// whose tiles give every SM work (17 rows of 17920 x 1536: 51 us, streaming the weights 77; of 1536 x 1536 13 and 9).
+constexpr int SPLIT_MIN_K = 256, SPLIT_WIDE_ROWS = 16, SPLIT_WIDE_N = 8192;
+int sb_gemm_f32_tc5(const float* A, const float* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
+                    const float* residual, void* out, int out_dtype, cudaStream_t stream);
+
 bool sb_gemm_f32_takes(const void* A, const void* W, int K) {
   return K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
 }
 
 int sb_gemm_f32(const void* A, const void* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
                 const float* residual, void* out, int out_dtype, cudaStream_t stream) {
+  if (K >= SPLIT_MIN_K && (M > ROWS_MAX || (M > SPLIT_WIDE_ROWS && N >= SPLIT_WIDE_N)))
+    return sb_gemm_f32_tc5((const float*)A, (const float*)W, M, N, K, epilogue, bias, bias_dtype, residual, out, out_dtype, stream);
   const F32Args p{(const float*)A, (const float*)W, M, N, K, epilogue, bias, bias_dtype, residual};
   const int rc = out_dtype == SB_F32 ? run_f32(p, (float*)out, stream) : run_f32(p, (__nv_bfloat16*)out, stream);
   if (rc) return rc;

@@ -1076,9 +1076,13 @@ int pair_splits(int M, int N, int K, int clusters) {
 }  // namespace
 
 // 0 when no kernel has given up on a wait since the last call; else the code of the wait
-// (1 producer/empty, 2 producer drain, 3 MMA/full, 4 epilogue/accumulator).  Reading
+// (1 producer/empty, 2 producer drain, 3 MMA/full, 4 epilogue/accumulator; 11 to 16 the float32 product's).  Reading
 // synchronizes with the device.
-extern "C" int sb_tc5_status() { return tc5_read_status(); }
+int sb_gemm_f32_tc5_status();
+extern "C" int sb_tc5_status() {
+  const int v = tc5_read_status(), f32 = sb_gemm_f32_tc5_status();
+  return v ? v : f32;
+}
 
 // 1: products of more than 128 rows run on pairs of SMs, 0: on single SMs, -1: by the environment.
 extern "C" void sb_gemm_tc5_pairs(int mode) { g_pair_mode = mode; }

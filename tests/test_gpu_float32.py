@@ -49,6 +49,48 @@ def test_products(M, N, K):
         assert errs[0] <= 1.3 * errs[1] + 2 ** -24, (epi, errs)     # and no more than the plain kernel's
 
 
+# the tensor-core form: token tiles of 32 to 224, one more than a tile, three tiles; K of its least, with a ragged last stage, shared by
+# a cluster; weight rows that end inside a tile; 17 rows of a wide product
+@pytest.mark.parametrize("M,N,K", [(17, 8208, 256), (33, 8, 256), (64, 130, 260), (97, 1536, 1540), (128, 272, 8960), (193, 2048, 1536),
+                                   (224, 400, 1024), (225, 136, 516), (449, 1000, 300), (672, 16, 4100)])
+@pytest.mark.parametrize("scale", [1.0, 1e-12, 1e12])
+def test_products_of_split_operands(M, N, K, scale):
+    a, w, bias, res = rnd(M, K, scale=scale), rnd(N, K, seed=1, scale=K ** -0.5), rnd(N, seed=2, scale=scale), rnd(M, N, seed=3, scale=scale)
+    y = a.double() @ w.double().T
+    for epi in (ops.EPI_NONE, ops.EPI_BIAS, ops.EPI_RESIDUAL, ops.EPI_RELU2, ops.EPI_SWIGLU):
+        if epi == ops.EPI_SWIGLU and N % 16:
+            continue
+        want = {ops.EPI_BIAS: y + bias.double(), ops.EPI_RESIDUAL: y + res.double(), ops.EPI_RELU2: y.clamp(min=0) ** 2}.get(epi, y)
+        if epi == ops.EPI_SWIGLU:
+            z = y.view(M, -1, 2, 8)
+            want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2)
+        out = res.clone() if epi == ops.EPI_RESIDUAL else torch.full(want.shape, float("nan"), device=DEV)
+        ops.linear(a, w, out, epi, bias=bias if epi == ops.EPI_BIAS else None, residual=out if epi == ops.EPI_RESIDUAL else None)
+        # an operand is off by up to 2^-22, a sum's roundings by a few 2^-24; squares and products of two sums by twice that;
+        # a gate's exponential by 2^-24 of the gate's size
+        err = float((out.double() - want).norm() / want.norm()) if scale < 2 or epi != ops.EPI_SWIGLU else 0.0
+        assert bool(out.isfinite().all()) and err < 2 ** -20, (epi, err)
+    assert ops.tc5_status() == 0
+
+
+def test_split_operands_let_what_is_not_finite_through():
+    """Infinities, NaN of every pattern, values that round to infinity as TF32 and sums that overflow: as term by term."""
+    M, N, K = 96, 144, 512
+    a, w = rnd(M, K), rnd(N, K, seed=1)
+    a[3, 7], a[40, 200], a[60, 0], a[61, 5] = float("inf"), float("-inf"), float("nan"), torch.finfo(torch.float32).max
+    a[62, 9] = torch.tensor(0x7fffffff, dtype=torch.int32).view(torch.float32)
+    a[63, 9] = torch.tensor(0x7f800001, dtype=torch.int32).view(torch.float32)
+    w[:, 5].mul_(0.25).clamp_(-0.5, 0.5)
+    out = torch.empty(M, N, device=DEV)
+    ops.linear(a, w, out)
+    want = a.double() @ w.double().T
+    clean = [i for i in range(M) if i not in (3, 40, 60, 62, 63)]
+    assert bool(out[clean].isfinite().all()) and bool(out[[60, 62, 63]].isnan().all())
+    assert torch.equal(out[[3, 40]], want[[3, 40]].float())
+    assert float((out[61].double() - want[61]).norm() / want[61].norm()) < 2 ** -20
+    assert ops.tc5_status() == 0
+
+
 def test_products_let_infinities_through():
     a, w = rnd(40, 256), rnd(64, 256, seed=1).abs()
     a[3, 7], a[35, 200], a[39, 0] = float("inf"), float("-inf"), float("nan")
@@ -83,7 +125,8 @@ def attention_both(hq, hkv, hd, held, new, window=0, chunk=0, sink=None, softcap
 
 
 # one token's heads in the 16-row form (and one head more than fits), stretches in the 64-row form; head sizes below,
-# at and over each width; lengths around a tile of 64 keys and around all of a cluster's tiles
+# at and over each width; lengths around a tile of 64 keys and around all of a cluster's tiles.  Stretches take the 32-row form while
+# 64 rows a block would leave SMs without one
 @pytest.mark.parametrize("hq,hkv,hd", [(4, 2, 16), (12, 2, 128), (17, 1, 36), (16, 1, 64), (3, 3, 100), (2, 1, 256)])
 @pytest.mark.parametrize("held,new", [([0, 63, 64, 511, 513, 1100], [1] * 6), ([0, 5, 200], [63, 130, 17]), ([0], [201])])
 def test_attention(hq, hkv, hd, held, new):
