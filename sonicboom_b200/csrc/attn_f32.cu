@@ -1,15 +1,16 @@
 // Float32 attention over the paged cache for the 32-bit path: FFMA only, a block per tile of query rows of one
 // key/value head of one sequence.
 //
-// A query row is a (token, head in group) pair, so that all query heads of a key/value head share its tiles.  Two
-// forms: 16 rows (a decode step: one token's heads), 64 rows (prompts).  Keys come in tiles of 64 at absolute
+// A query row is a (token, head in group) pair, so that all query heads of a key/value head share its tiles.  Three
+// forms: 16 rows (a decode step: one token's heads), 64 rows (prompts), 32 rows (prompts whose 64-row tiles leave SMs idle).  Keys come in tiles of 64 at absolute
 // positions, which a cluster of blocks takes in turn (8 blocks for 16 rows, where a step has few blocks and the
-// sequence is long; 2 for 64 rows); the blocks' running softmaxes are merged in rank order through distributed shared
+// sequence is long; 4 for 32 rows, 2 for 64); the blocks' running softmaxes are merged in rank order through distributed shared
 // memory, so no workspace is needed and a row's sums depend on its own keys and the form alone.
 //
 // What attn_plain.cu says about masks, caps, biases and sinks holds here; that kernel (a block per row and head, a
 // warp per key) stays for head sizes this one does not take.  12/2 heads of 128: three single tokens at 100 to 400 keys
-// took 324 us there, bound by a block's dependent steps over its keys, and 19 here; a prompt of 201 tokens 183 and 67.
+// took 324 us there, bound by a block's dependent steps over its keys, and 16 here (19 when a tile's loads came one after
+// the other); a prompt of 201 tokens 183 and 50 (67 in 64-row tiles).
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -19,7 +20,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int THREADS = 256, KEYS = 64;
+constexpr int THREADS = 256, KEYS = 64, LOADS = 4;
 
 struct F32Attn {
   const float* q;
@@ -40,7 +41,7 @@ struct F32Attn {
 template <int TQ, int ND>
 struct Form {
   static constexpr int QB = 16 * TQ;
-  static constexpr int SPLITS = TQ == 1 ? 8 : 2;
+  static constexpr int SPLITS = TQ == 1 ? 8 : TQ == 2 ? 4 : 2;
   static int floats(int hd) {      // queries, keys (later probabilities), values, maximum and sum, their merge
     const int kp = KEYS * (hd + 4), pp = QB * (KEYS + 4), op = QB * hd;
     const int first = kp > pp ? kp : pp;
@@ -66,7 +67,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
   const int rank = blockIdx.z, tid = threadIdx.x;
   const int seq = blockIdx.x / tiles_per_seq, tile = blockIdx.x % tiles_per_seq, g = blockIdx.y;
   const int group = p.n_q_heads / p.n_kv_heads;
-  sb_pdl_wait();
+  // the step's plan was written before the step's first kernel
   const int row0 = p.seq_row0[seq], n_new = p.seq_row0[seq + 1] - row0, pos0 = p.seq_pos0[seq];
   const int pairs = n_new * group, pair0 = tile * QB;
   if (pair0 >= pairs) return;                           // the same for the whole cluster
@@ -90,6 +91,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
                        p.chunk > 0 ? max(first_pos, 0) / p.chunk * p.chunk : 0);
   const int k_hi = min(last_pos, held - 1);
 
+  sb_pdl_wait();
   const int quads = hd / 4;
   for (int i = tid; i < QB * quads; i += THREADS) {
     const int r = i / quads, c = i % quads, pair = pair0 + r;
@@ -115,19 +117,34 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
     if (tid == 0) bad_values = 0;
     __syncthreads();
     bool bad = false;
-    for (int i = tid; i < KEYS * quads; i += THREADS) {
-      const int r = i / quads, c = i % quads, j = base + r;
-      float4 kv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv = kv;
-      const int page = j >= k_lo && j <= k_hi ? pages[j / p.page_size] : -1;
-      if (page >= 0 && page < p.n_pages) {
-        const float* at = p.cache + (((size_t)page * 2 * p.n_kv_heads + g) * p.page_size + j % p.page_size) * hd + 4 * c;
-        kv = *reinterpret_cast<const float4*>(at);
-        vv = *reinterpret_cast<const float4*>(at + (size_t)p.n_kv_heads * p.page_size * hd);
+    // LOADS keys' and values' 16 bytes a thread at once: one after the other they were most of a decode step's time
+    for (int i0 = tid; i0 < KEYS * quads; i0 += LOADS * THREADS) {
+      float4 kv[LOADS], vv[LOADS];
+      int page[LOADS];
+#pragma unroll
+      for (int u = 0; u < LOADS; ++u) {
+        const int i = i0 + u * THREADS, j = base + i / quads;
+        page[u] = i < KEYS * quads && j >= k_lo && j <= k_hi ? pages[j / p.page_size] : -1;
       }
-      *reinterpret_cast<float4*>(ks + r * kpitch + 4 * c) = kv;
-      *reinterpret_cast<float4*>(vs + r * hd + 4 * c) = vv;
-      const float s = fabsf(vv.x) + fabsf(vv.y) + fabsf(vv.z) + fabsf(vv.w);
-      bad |= !(s < INFINITY);
+#pragma unroll
+      for (int u = 0; u < LOADS; ++u) {
+        const int i = i0 + u * THREADS, j = base + i / quads, c = i % quads;
+        kv[u] = vv[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (page[u] >= 0 && page[u] < p.n_pages) {
+          const float* at = p.cache + (((size_t)page[u] * 2 * p.n_kv_heads + g) * p.page_size + j % p.page_size) * hd + 4 * c;
+          kv[u] = *reinterpret_cast<const float4*>(at);
+          vv[u] = *reinterpret_cast<const float4*>(at + (size_t)p.n_kv_heads * p.page_size * hd);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < LOADS; ++u) {
+        const int i = i0 + u * THREADS, r = i / quads, c = i % quads;
+        if (i >= KEYS * quads) continue;
+        *reinterpret_cast<float4*>(ks + r * kpitch + 4 * c) = kv[u];
+        *reinterpret_cast<float4*>(vs + r * hd + 4 * c) = vv[u];
+        const float s = fabsf(vv[u].x) + fabsf(vv[u].y) + fabsf(vv[u].z) + fabsf(vv[u].w);
+        bad |= !(s < INFINITY);
+      }
     }
     if (bad) bad_values = 1;
     __syncthreads();
@@ -313,9 +330,15 @@ extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_se
     SB_FAIL(SB_ERR_UNSUPPORTED, "sb_attention_f32: head size %d (a multiple of 4 up to 256), %d key/value heads", hd, n_kv_heads);
   const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
                   chunk, bias_len, scale, softcap, sink, bias};
-  // one token's heads fit the 16-row form; a row of a longer stretch sees up to 64 rows' keys loaded once
-  const bool few = (long)max_new * (n_q_heads / n_kv_heads) <= 16;
-  if (hd <= 64) return few ? launch<1, 1>(p, n_seqs, max_new, stream) : launch<4, 1>(p, n_seqs, max_new, stream);
-  if (hd <= 128) return few ? launch<1, 2>(p, n_seqs, max_new, stream) : launch<4, 2>(p, n_seqs, max_new, stream);
-  return few ? launch<1, 4>(p, n_seqs, max_new, stream) : launch<4, 4>(p, n_seqs, max_new, stream);
+  // one token's heads fit the 16-row form; a row of a longer stretch sees up to 64 rows' keys loaded once, or 32 where 64
+  // leave SMs without a block (a prompt of 201 tokens: 76 blocks that go through two tiles of keys each, or 304 with one)
+  const long rows = (long)max_new * (n_q_heads / n_kv_heads), blocks = (rows + 63) / 64 * n_kv_heads * n_seqs * 2;
+#define SB_F32_FORMS(ND)                                              \
+  if (rows <= 16) return launch<1, ND>(p, n_seqs, max_new, stream);   \
+  if (blocks < 148) return launch<2, ND>(p, n_seqs, max_new, stream); \
+  return launch<4, ND>(p, n_seqs, max_new, stream);
+  if (hd <= 64) { SB_F32_FORMS(1) }
+  if (hd <= 128) { SB_F32_FORMS(2) }
+  SB_F32_FORMS(4)
+#undef SB_F32_FORMS
 }
