@@ -58,11 +58,11 @@ __host__ __device__ constexpr uint32_t instr_desc(int bn) {
 }
 
 // SiLU of a value that is rounded to TO afterwards: for bfloat16 outputs with the hardware's
-// exponential and division (relative error about 1e-6 against bfloat16's 4e-3; a gate so negative that the
-// exponential overflows gives 0, as it should); for float32 outputs the accurate one.
+// exponential (relative error about 1e-6 against bfloat16's 4e-3; a gate so negative that the
+// exponential overflows gives 1 / inf = 0, as it should); for float32 outputs the accurate one.
 template <typename TO>
 __device__ __forceinline__ float sb_silu_out(float x) {
-  if (sizeof(TO) == 2) return __fdividef(x, 1.0f + __expf(-x));
+  if (sizeof(TO) == 2) return x * __frcp_rn(1.0f + __expf(-x));
   return sb_silu(x);
 }
 
@@ -875,6 +875,76 @@ tc5_reduce_norm_kernel(const Tc5Params p, int bn, const TW* __restrict__ norm_w,
   }
 }
 
+// The same with a block a row, for more than 64 rows, which are enough blocks: no cluster to wait for, and the sum of squares is
+// added as rmsnorm_vec_kernel adds it, so the normed row is the one that the norm as a kernel of its own gives.
+constexpr int RNR_MAX_WIDTH = RN_THREADS * RN_VEC * 4;
+template <typename TW, typename TN>
+__global__ void __launch_bounds__(RN_THREADS)
+tc5_reduce_norm_row_kernel(const Tc5Params p, int bn, const TW* __restrict__ norm_w, float eps,
+                           TN* __restrict__ norm_out, const TW* __restrict__ norm_w2, TN* __restrict__ norm_out2) {
+  __shared__ float warp_sums[RN_THREADS / 32];
+  __shared__ float inv_shared;
+  sb_pdl_launch();
+  const int j = blockIdx.x;                                             // token
+  float wv[RN_VEC][4];
+#pragma unroll
+  for (int i = 0; i < RN_VEC; ++i) {                 // the norm's weights wait for nobody
+    const int e = (threadIdx.x + i * RN_THREADS) * 4;
+    if (e < p.N) rn_load4(norm_w + e, wv[i]);
+  }
+  sb_pdl_wait();
+  float v[RN_VEC][4];
+  float sq = 0.0f;
+#pragma unroll
+  for (int i = 0; i < RN_VEC; ++i) {
+    const int e = (threadIdx.x + i * RN_THREADS) * 4;
+    if (e >= p.N) continue;
+    size_t stride;
+    const float* base = partial_sums(p, bn, j, e, stride);
+    float add[4] = {0.0f, 0.0f, 0.0f, 0.0f}, acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (p.epilogue == SB_EPI_BIAS) {
+      if (p.bias_dtype == SB_F32) rn_load4((const float*)p.bias + e, add);
+      else rn_load4((const bf16*)p.bias + e, add);
+    } else if (p.epilogue == SB_EPI_RESIDUAL) {
+      rn_load4(p.residual + (size_t)j * p.N + e, add);
+    }
+    for (int s = 0; s < p.k_splits; ++s) {
+      const float4 t = *reinterpret_cast<const float4*>(base + s * stride);
+      acc[0] += t.x; acc[1] += t.y; acc[2] += t.z; acc[3] += t.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[i][k] = p.epilogue == SB_EPI_NONE ? acc[k] : acc[k] + add[k];
+    rn_store4((float*)p.out + (size_t)j * p.N + e, v[i]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sq = fmaf(v[i][k], v[i][k], sq);
+  }
+  sq = sb_warp_sum(sq);
+  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = sq;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float total = 0.0f;
+    for (int i = 0; i < RN_THREADS / 32; ++i) total += warp_sums[i];
+    inv_shared = 1.0f / sqrtf(total / (float)p.N + eps);
+  }
+  __syncthreads();
+  const float inv = inv_shared;
+#pragma unroll
+  for (int i = 0; i < RN_VEC; ++i) {
+    const int e = (threadIdx.x + i * RN_THREADS) * 4;
+    if (e >= p.N) continue;
+    float y[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) y[k] = (v[i][k] * inv) * wv[i][k];
+    rn_store4(norm_out + (size_t)j * p.N + e, y);
+    if (norm_w2) {                                   // the same rows with a second weight
+      rn_load4(norm_w2 + e, wv[i]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[k] = (v[i][k] * inv) * wv[i][k];
+      rn_store4(norm_out2 + (size_t)j * p.N + e, y);
+    }
+  }
+}
+
 // --------------------------------------------------------------------------- host side
 // A [rows, K] bfloat16 row-major matrix as a tensor map with boxes of box_rows x 64.
 bool make_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows) {
@@ -1104,14 +1174,15 @@ namespace {
 int swapped_bn(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
 
 // How many blocks share one output tile of the swapped form: enough to give every SM two
-// blocks, at least four K tiles each (eight with more than 64 rows, whose partial tiles are as large as a weight
-// tile of four), and no block without work.
+// blocks, at least four K tiles each, and no block without work.  More than 64 rows take the splits of the
+// pair kernel, which is about a block an SM with twice the stages: the partial sums are half as many, and a prompt's values
+// are those that the pair kernel gives.
 int choose_splits(int M, int N, int K, int n_sms) {
+  if (M > 64) return N >= 192 && n_sms > 1 && pair_enabled() ? pair_splits(M, N, K, n_sms / 2) : 1;
   const int tiles = (N + BM - 1) / BM, n_k = (K + BK - 1) / BK;
   int splits = n_sms > 0 ? 2 * n_sms / tiles : 1;       // two blocks fit an SM
   if (splits > 16) splits = 16;
-  const int least = M > 64 ? 8 : 4;
-  if (splits > n_k / least) splits = n_k / least;
+  if (splits > n_k / 4) splits = n_k / 4;
   if (splits < 1) splits = 1;
   const int k_per = (n_k + splits - 1) / splits;
   return (n_k + k_per - 1) / k_per;
@@ -1143,7 +1214,7 @@ static int splits_k(int M, int N, int K, int n_sms) {
 // Whether these rows are finished by the fused reduce + norm kernel: every product that splits K.
 static bool norm_fuses(int M, int N, int K, int n_sms, int epilogue, int out_dtype, int form) {
   if (epilogue == SB_EPI_SWIGLU || epilogue == SB_EPI_RELU2 || out_dtype != SB_F32 || N % 4 || N > RN_MAX_WIDTH) return false;
-  return form != 1 && splits_k(M, N, K, n_sms) > 1;
+  return form != 1 && (M <= 64 || N <= RNR_MAX_WIDTH) && splits_k(M, N, K, n_sms) > 1;
 }
 
 extern "C" int sb_gemm_tc5_fuses_norm(int M, int N, int K, int n_sms, int epilogue, int out_dtype,
@@ -1180,6 +1251,17 @@ static int reduce_rope(const Tc5Params& p, int bn, const SbRopeStore& rope, int 
 }
 
 static int reduce_norm(const Tc5Params& p, int bn, const SbLinearExtras& norm, cudaStream_t stream) {
+  if (p.M > 64) {
+    SB_DISPATCH_DTYPE(norm.norm_weight_dtype, TW, {
+      SB_DISPATCH_DTYPE(norm.norm_out_dtype, TN, {
+        sb_launch<SB_K_REDUCE>(tc5_reduce_norm_row_kernel<TW, TN>, dim3((unsigned)p.M), dim3(RN_THREADS), 0, stream, p, bn,
+                               (const TW*)norm.norm_weight, norm.norm_eps, (TN*)norm.norm_out, (const TW*)norm.norm_weight2,
+                               (TN*)norm.norm_out2);
+      });
+    });
+    SB_CHECK_LAUNCH("sb_gemm_tc5 (reduce + norm of a row)");
+    return SB_OK;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(RN_CLUSTER, (unsigned)p.M);
   cfg.blockDim = dim3(RN_THREADS);
@@ -1395,6 +1477,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
   if (bn == 16) { SB_TC5_SWAPPED(16, 4) }
   else if (bn == 32) { SB_TC5_SWAPPED(32, 5) }
   else if (bn == 64) { SB_TC5_SWAPPED(64, 4) }
+  else if (blocks <= n_sms) { SB_TC5_SWAPPED(128, 6) }
   else { SB_TC5_SWAPPED(128, 3) }
 #undef SB_TC5_SWAPPED
   if (rc != SB_OK || splits <= 1) return rc;

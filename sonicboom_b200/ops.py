@@ -217,16 +217,17 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 
 
     `norm` = (weight, eps, norm_out[, weight2, norm_out2]) also writes norm_out = rmsnorm(out, weight, eps) [M,N]
     (and norm_out2 with the second weight)
-    (out must be float32): in the kernel that finishes the product where one does (the split-K
-    decode form of the tcgen05 kernel), else with the norm kernel after it.
+    (out must be float32): in the kernel that finishes the product where one does (wherever the tcgen05 kernel
+    splits K: decode steps and prompts of up to some hundred rows), else with the norm kernel after it.
     `warm`: weights that a later kernel streams; the blocks of the tcgen05 kernel ask for them
     into L2 as they end (other kernels ignore it).  A hint: it changes no result.  It pays only
     for a consumer that cannot request its own weights early (see `requests_weights_late`).
 
     bfloat16 operands run on tensor cores: `kernel` "tc5" (TMA + tcgen05), "skinny" (weights
     streamed into mma.sync fragments, at most SKINNY_MAX_ROWS rows), "tiled" (mma.sync tiles),
-    or "auto", which picks between the first two (see `_pick_kernel`).  float32 operands, inner
-    sizes that are not multiples of 8, and `kernel="plain"` run the plain FFMA kernel.  A
+    or "auto", which picks between the first two (see `_pick_kernel`).  float32 operands run
+    sb_gemm_plain's float32 forms (FFMA, or tensor cores with every operand split in two), inner
+    sizes that are not multiples of 8 and bfloat16 with `kernel="plain"` its plain FFMA kernel.  A
     bfloat16 activation with a float32 weight is cast to float32 first.  The split-K decode
     form keeps one workspace per device, so products on one device must be ordered in a stream.
     """

@@ -283,13 +283,13 @@ def test_linear_followed_by_a_norm(M, N, K, ndtype):
     assert ops.tc5_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(65, 520, 2048), (97, 3584, 1032), (128, 260, 4096), (129, 528, 2048), (300, 1040, 4096),
+@pytest.mark.parametrize("M,N,K", [(65, 520, 2048), (97, 3584, 1032), (128, 272, 4096), (129, 528, 2048), (300, 1040, 4096),
                                    (512, 3584, 1200), (1500, 1536, 1536)])
 @pytest.mark.parametrize("pair", [False, True])
 def test_norms_ride_on_every_product_that_splits_k(M, N, K, pair):
     """65 to 128 rows stream the weights past tiles of 128 tokens, more rows run on pairs of SMs; where either splits K
     the kernel that adds the partial sums also writes the norm (or two), with the residual updated in place:
-    the product's bits are those without a norm, the norm's within the rounding of bfloat16 (half an ulp is 2^-8)."""
+    the product's bits are those without a norm, the norm's those of the norm kernel on these rows."""
     a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, scale=K ** -0.5, seed=1)
     res, bias = rnd(M, N, seed=3), rnd(N, dtype=torch.bfloat16, seed=2)
     weights = [(1 + 0.3 * rnd(N, seed=4 + i)).to(torch.bfloat16) for i in range(2)]
@@ -306,7 +306,8 @@ def test_norms_ride_on_every_product_that_splits_k(M, N, K, pair):
         assert torch.equal(out, plain)
         close(out, linear_ref(a, w, epi, bias, res), 1e-5)
         for i in range(1 + pair):
-            close(normed[i], rmsnorm_ref(out, weights[i], 3e-5), 5e-3)
+            close(normed[i], rmsnorm_ref(out, weights[i], 3e-5), 5e-3)     # half an ulp of bfloat16 is 2^-8
+            assert torch.equal(normed[i], ops.rmsnorm(out, weights[i], 3e-5, torch.empty_like(normed[i])))
     assert ops.tc5_status() == 0
 
 
@@ -827,7 +828,7 @@ def test_rotation_rides_on_the_weight_streaming_product(rows, hq, hkv, hd, rot, 
 @pytest.mark.parametrize("rows,K", [(97, 3584), (128, 1536), (200, 3584), (500, 3584)])
 def test_rotation_rides_on_the_split_products_of_prompts(rows, K):
     """The same fusion at a prompt's rows (tiles of 128 tokens, pairs of SMs with K split): 28 query and 4 key/value heads of
-    128, against the same product followed by `rope_store`, to an ulp of bfloat16."""
+    128: the bits of the same product followed by `rope_store`."""
     dt, hq, hkv, hd = torch.bfloat16, 28, 4, 128
     N = (hq + 2 * hkv) * hd
     a, w, bias = rnd(rows, K, dtype=dt), rnd(N, K, dtype=dt, scale=K ** -0.5, seed=1), rnd(N, dtype=dt, seed=2)
@@ -852,10 +853,10 @@ def test_rotation_rides_on_the_split_products_of_prompts(rows, K):
             qkv = torch.empty(rows, N, device=DEV)
             ops.linear(a, w, qkv, ops.EPI_BIAS, bias=bias)
             ops.rope_store(qkv, *where)
-        got.append((q.float().cpu(), storage.float().cpu()))
-    assert float(got[1][1].abs().max()) > 0
+        got.append((q, storage))
+    assert float(got[1][1].float().abs().max()) > 0
     for x, y in zip(*got):
-        assert pm.rel_err(x, y) < 4e-3
+        assert torch.equal(x, y)
     assert ops.tc5_status() == 0
 
 
