@@ -48,16 +48,12 @@ constexpr int LDS = HD + 8;            // shared-memory row stride: an odd numbe
 constexpr int BM = HD <= 128 ? 128 : 64;  // prefill rows per block (16 per warp); registers bound it
 constexpr int PREFILL_THREADS = BM / 16 * 32;
 constexpr int DEC_WARPS = 4;           // decode: warps per block, 16 keys of every tile each
-// decode: pages per split.  128 keys while a sequence is at most SHORT_LEN long (a block then goes through two tiles one
-// after the other, not four: eight tokens of one 1.5B conversation at 333 keys 9.91 to 9.62 ms, 8 and 64 sequences of
-// 300 to 1,500 keys as before), 256 while it is at most LONG_LEN long, 512 beyond: a
+// decode: pages per split.  256 keys while a sequence is at most LONG_LEN long, 512 beyond: a
 // longer split spreads a block's fixed costs over more keys (32,768 keys at batch 8: 110 us
 // against 130 us per layer), a shorter one gives short sequences enough blocks (3,072 keys at
 // batch 8: 14.9 us against 18.2 us).  It depends on the sequence's own length only.
-constexpr int SHORT_SPLIT_PAGES = 2, SPLIT_PAGES = 4, LONG_SPLIT_PAGES = 8, SHORT_LEN = 1024, LONG_LEN = 4096;
-__host__ __device__ constexpr int split_pages_for(int len) {
-  return len > LONG_LEN ? LONG_SPLIT_PAGES : len > SHORT_LEN ? SPLIT_PAGES : SHORT_SPLIT_PAGES;
-}
+constexpr int SPLIT_PAGES = 4, LONG_SPLIT_PAGES = 8, LONG_LEN = 4096;
+__host__ __device__ constexpr int split_pages_for(int len) { return len > LONG_LEN ? LONG_SPLIT_PAGES : SPLIT_PAGES; }
 constexpr int DEC_ROWS = 16;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int BIAS_PAD = 64;
@@ -671,15 +667,10 @@ constexpr int MAX_MERGE_SPLITS = 4 * LDS;
 
 // Splits the grid needs when no sequence is longer than max_len: short sequences use short splits.
 int n_splits_for(int max_len) {
-  int most = 0;
-  const int lens[3] = {SHORT_LEN, LONG_LEN, max_len}, pages[3] = {SHORT_SPLIT_PAGES, SPLIT_PAGES, LONG_SPLIT_PAGES};
-  for (int i = 0; i < 3; ++i) {                 // the longest sequence of every split length
-    const int len = lens[i] < max_len ? lens[i] : max_len;
-    if (i > 0 && max_len <= lens[i - 1]) break;
-    const int n = (len + pages[i] * KT - 1) / (pages[i] * KT);
-    most = n > most ? n : most;
-  }
-  return most;
+  if (max_len <= LONG_LEN) return (max_len + SPLIT_PAGES * KT - 1) / (SPLIT_PAGES * KT);
+  const int most_short = LONG_LEN / (SPLIT_PAGES * KT);
+  const int longs = (max_len + LONG_SPLIT_PAGES * KT - 1) / (LONG_SPLIT_PAGES * KT);
+  return longs > most_short ? longs : most_short;
 }
 
 // Shared memory opt-ins of the mma.sync kernels, once per instantiation.
