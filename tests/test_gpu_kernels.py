@@ -283,7 +283,7 @@ def test_linear_followed_by_a_norm(M, N, K, ndtype):
     assert ops.tc5_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(65, 520, 2048), (97, 3584, 1032), (128, 272, 4096), (129, 528, 2048), (300, 1040, 4096),
+@pytest.mark.parametrize("M,N,K", [(65, 528, 2048), (97, 3584, 1032), (128, 272, 4096), (129, 528, 2048), (300, 1040, 4096),
                                    (512, 3584, 1200), (1500, 1536, 1536)])
 @pytest.mark.parametrize("pair", [False, True])
 def test_norms_ride_on_every_product_that_splits_k(M, N, K, pair):
