@@ -14,9 +14,9 @@
 //   so no workspace is needed.
 //
 // Measured on one B200 inside a step of the 1.5B layers (28 layers: 2048, 1536 and 17920 x 1536, 1536 x 8960): three rows
-// 15.5 us a product on average where the plain kernel took 636 (one row of 151936 x 1536: 140 us, 6.6 TB/s); 201 rows
-// 193 us where it took 821 (17920 x 1536: 330 us, 34 TFLOP/s of 74).  The rows form wins up to 32 rows (1536 x 8960 at
-// 32 rows 64 against 110 us, at 64 rows 113 against 117; 17920 x 1536 at 24 rows 82 against 100 us, at 32 104 against 100).
+// 15.5 us a product on average where the plain kernel took 636 (one row of 151936 x 1536: 140 us, 6.6 TB/s).  The tile form at
+// 201 rows took 193 us where the plain kernel took 821 (17920 x 1536: 330 us, 34 TFLOP/s of 74), and the tensor cores 56.
+// Rows against tensor cores at 24 rows: 1536 x 8960 40 and 38 us, 2048 x 1536 11 and 14, 17920 x 1536 77 and 50; hence the lines.
 // Error against float64 at K = 8960: 1.2e-7 and 4.3e-7, the plain kernel's terms one after the other 9e-7.
 //
 // Epilogues as in gemm_plain.cu, which computes the same sums in another order and takes the sizes and

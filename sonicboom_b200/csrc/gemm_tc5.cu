@@ -91,8 +91,8 @@ __device__ __forceinline__ float sb_gated(const P& p, float gate, float up) {
 
 // The same for N outputs (gates v[0..7], their up values v[8..15], and so on): one branch for all of them, so that
 // their exponentials and divisions overlap.  (With a branch an output the gate/up epilogue of a prompt took 35
-// instructions an output one after the other: at K = 1,536 longer than the next tile's MMAs, 110 us for 2,048
-// rows of 17,920 x 1,536 where it is now 100.)
+// instructions an output one after the other: at K = 1,536 longer than the next tile's MMAs, 99 us for 2,048
+// rows of 17,920 x 1,536 where it is now 89.)
 template <typename TO, int N, typename P>
 __device__ __forceinline__ void sb_gated_row(const P& p, const float* v, float* o) {
   if (p.gate_kind == SB_GATE_GELU_TANH) {
