@@ -67,7 +67,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
   const int rank = blockIdx.z, tid = threadIdx.x;
   const int seq = blockIdx.x / tiles_per_seq, tile = blockIdx.x % tiles_per_seq, g = blockIdx.y;
   const int group = p.n_q_heads / p.n_kv_heads;
-  // the step's plan was written before the step's first kernel
+  // the step's plan was written before the step's first kernel, which triggers after its own wait
   const int row0 = p.seq_row0[seq], n_new = p.seq_row0[seq + 1] - row0, pos0 = p.seq_pos0[seq];
   const int pairs = n_new * group, pair0 = tile * QB;
   if (pair0 >= pairs) return;                           // the same for the whole cluster

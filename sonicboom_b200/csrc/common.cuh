@@ -98,6 +98,9 @@ __device__ __forceinline__ float sb_warp_max(float v) {
 // its successor may be scheduled: small kernels at their start, the products and the attention
 // once their own operands have been requested, so that a successor does not take resources the
 // kernel still wants.  Without the launch attribute both are no-ops.
+// Starting is transitive: behind kernels that trigger at their first instruction a kernel can start while one several
+// places before it still runs.  A step's plan (positions, page lists) may be read ahead of the wait all the same, because
+// the step's first kernel, the embedding, triggers after its own wait.
 __device__ __forceinline__ void sb_pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void sb_pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

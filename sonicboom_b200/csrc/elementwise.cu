@@ -13,11 +13,14 @@ extern "C" int sb_abi_version() { return 1; }
 // the non-coherent load path that `const __restrict__` selects could then return stale lines.
 // An id outside the table (the sampler's -1 for a row of logits that are not finite, when ids are
 // fed back on the device) reads nothing and gives a row of NaN, which stays visible downstream.
+// The embedding is a step's first kernel, so it lets its successor start only after its own wait: what a loop on the
+// device wrote between two steps (positions, token ids) is then finished before any later kernel of the step starts, and
+// those may read the step's plan ahead of their own waits.
 template <typename TW>
 __global__ void embed_kernel(const int32_t* tokens, const TW* __restrict__ table, int vocab,
                              int width, float scale, float* __restrict__ out) {
-  sb_pdl_launch();
   sb_pdl_wait();
+  sb_pdl_launch();
   const int t = blockIdx.x;
   const int id = tokens[t];
   float* o = out + (size_t)t * width;
@@ -216,14 +219,14 @@ extern "C" int sb_rmsnorm_pair(const float* x, int n_rows, int width, const void
 }
 
 // The embedding row, times `scale`, RMS-normed with the weight `w`: what a model hands its first layer when it norms its
-// embeddings.  An id outside the table gives a row of NaN.
+// embeddings.  An id outside the table gives a row of NaN.  A step's first kernel: the wait comes first (see embed_kernel).
 template <typename TW, typename TN>
 __global__ void __launch_bounds__(256)
 embed_norm_kernel(const int32_t* tokens, const TW* __restrict__ table, int vocab, int width, float scale,
                   const TN* __restrict__ w, float eps, float* __restrict__ out) {
   __shared__ float warp_sums[8];
-  sb_pdl_launch();
   sb_pdl_wait();
+  sb_pdl_launch();
   const int t = blockIdx.x, id = tokens[t];
   float* o = out + (size_t)t * width;
   if ((unsigned)id >= (unsigned)vocab) {

@@ -675,12 +675,14 @@ __device__ __forceinline__ const float* partial_sums(const Tc5Params& p, int bn,
 // the same rotation formulas as the two kernels.  A block takes a
 // token and a share of its heads; a task is four pairs (e, e + half) of one head, or four of the
 // values beyond the rotated part.  cos and sin of the token's position are worked out once a
-// block (from the step's plan, before the wait for the product).
+// block (from the step's plan, before the wait for the swapped product; the pair kernel lets this one start at its first
+// instruction, so behind it the wait comes first).
 constexpr int RR_THREADS = 256;
 __global__ void __launch_bounds__(RR_THREADS)
 tc5_reduce_rope_kernel(const Tc5Params p, int bn, const SbRopeStore r) {
   extern __shared__ float rr_cs[];                   // cos[rot/2], then sin[rot/2]
   sb_pdl_launch();
+  if (bn == 0) sb_pdl_wait();
   const int t = blockIdx.x;
   const int pos = r.row_pos[t];
   const int half = r.rot >> 1, hd = r.hd;

@@ -38,8 +38,8 @@ __global__ void embed_pair_kernel(const int32_t* tokens, const int32_t* row_seq,
                                   const int32_t* seq_row0, const int32_t* seq_slot, const int32_t* prev_token,
                                   const T* __restrict__ table, int vocab, const T* __restrict__ pair, int buckets,
                                   int mul_prev, int mul_cur, int width, float scale, float* out) {
-  sb_pdl_launch();
-  sb_pdl_wait();
+  sb_pdl_wait();                                    // a step's first kernel waits before it lets the next one start
+  sb_pdl_launch();                                  // (embed_kernel says why)
   const int r = blockIdx.x;
   const int tok = tokens[r];
   float* o = out + (size_t)r * width;

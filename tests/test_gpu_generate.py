@@ -354,3 +354,31 @@ def test_trace_replay_three_cuts(model_dirs, oracles, tmp_path, name, dtype):
     assert len(by_step[last]) == expect[last].shape[0] and all(len(r) == 2 for r in by_step[last])
     first_decode = len(reqs) + 1                  # the step after request r0's prefix step
     assert by_step[first_decode] == [["r0x", len(reqs["r0"]) - 32]]
+
+
+@pytest.mark.parametrize("n_seqs", [130, 3])
+def test_a_device_loop_without_a_graph(tmp_path, n_seqs):
+    """The same loop as launches of its own: nothing but the kernels' own waits lies between the kernel that moves the
+    positions on and those that read them, at rows that finish the q|k|v product behind the pair kernel and at few."""
+    import sonicboom_b200 as sb
+    from sonicboom_b200 import ops
+    from sonicboom_b200.engine.decode import DecodeLoop
+    cfg = dict(TINY["B"], hidden_size=1536, num_attention_heads=12, num_key_value_heads=2, head_dim=128)
+    sb.write_random_model(tmp_path, cfg, seed=3, std=0.02, bias_std=0.1, norm_std=0.1)
+    engine = sb.Engine(sb.load_model(str(tmp_path), dtype="bfloat16"), max_tokens=64 * n_seqs)
+    if n_seqs > 128:
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        assert bool(ops.lib().sb_gemm_tc5_fuses_rope(n_seqs, 2048, 1536, sms, 12, 2, 128, 128, 1))
+    prompts = [[(7 * i + j) % 1000 for j in range(1 + i % 5)] for i in range(n_seqs)]
+    seen = []
+    for graph in (True, False):
+        slots = [engine.open() for _ in prompts]
+        engine.step([(s, p, []) for s, p in zip(slots, prompts)])
+        loop = DecodeLoop(engine, slots, 24, use_graph=graph)
+        loop.run_device([(3 * i) % 1000 for i in range(n_seqs)], 20)
+        assert loop.plan.row_pos.tolist() == [len(p) + 20 for p in prompts]
+        seen.append(loop.plan.tokens.clone())
+        loop.close()
+        for s in slots:
+            engine.close(s)
+    assert torch.equal(seen[0], seen[1])
