@@ -1230,6 +1230,7 @@ static bool rope_fuses(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_h
   if (M <= 0 || N <= 0 || K <= 0 || n_q_heads <= 0 || hd <= 0 || (has_kv && n_kv_heads <= 0)) return false;
   if (N != (n_q_heads + (has_kv ? 2 * n_kv_heads : 0)) * hd) return false;
   if (rot < 0 || rot > hd || (rot & 7) || ((hd - rot) & 3) || (hd & 3)) return false;
+  if (M > SWAPPED_ROWS && pair_clusters<256, float>() <= 0) return false;      // no pairs of SMs to split K over
   return splits_k(M, N, K, n_sms) > 1;
 }
 

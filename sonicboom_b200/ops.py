@@ -355,8 +355,10 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
             and (not has_kv or cache.dtype == torch.bfloat16) and K % 8 == 0
             and (bias is None or bias.numel() == N)):
         kernel = _pick_kernel(M, N, K, h.device)
-        if kernel == "tc5" and l.sb_gemm_tc5_fuses_rope(M, N, K, _sm_count(h.device), n_q_heads, n_kv_heads, head_dim,
-                                                        rotary_dim, 1 if has_kv else 0):
+        # the kernel behind the tcgen05 product reads and writes 16 and 8 bytes at a time
+        aligned = inv_freq.data_ptr() % 16 == 0 and (q_out.data_ptr() | (cache.data_ptr() if has_kv else 0)) % 8 == 0
+        if kernel == "tc5" and aligned and l.sb_gemm_tc5_fuses_rope(M, N, K, _sm_count(h.device), n_q_heads, n_kv_heads,
+                                                                    head_dim, rotary_dim, 1 if has_kv else 0):
             fused = kernel
         elif kernel == "skinny" and l.sb_gemm_skinny_takes_rope(M, N, n_q_heads, n_kv_heads, head_dim, rotary_dim,
                                                                 1 if has_kv else 0):

@@ -825,6 +825,44 @@ def test_rotation_rides_on_the_weight_streaming_product(rows, hq, hkv, hd, rot, 
     assert int((got[0][1] != 0).any(-1).sum()) == 2 * hkv * (rows - 1)
 
 
+def rope_problem(rows, hq=12, hkv=2, hd=128, K=1536):
+    """Operands of a q|k|v product of one sequence with its rotation: (h, w, bias), what comes between, (cache, q)."""
+    dt = torch.bfloat16
+    N = (hq + 2 * hkv) * hd
+    ops3 = rnd(rows, K, dtype=dt), rnd(N, K, dtype=dt, scale=K ** -0.5, seed=1), rnd(N, dtype=dt, seed=2)
+    inv = torch.from_numpy((10000.0 ** (-np.arange(hd // 2) / (hd // 2))).astype(np.float32)).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)             # noqa: E731
+    pages = (rows + 63) // 64
+    where = (inv, i32([0] * rows), i32(list(range(rows))), i32([0, pages]), i32(list(range(pages))), 64)
+    return ops3, (hq, hkv, hd, hd), where, (torch.zeros(pages, 2, hkv, 64, hd, dtype=dt, device=DEV),
+                                            torch.zeros(rows, hq, hd, dtype=dt, device=DEV))
+
+
+def shifted(t, by):
+    """The same values `by` elements further on than an aligned address."""
+    flat = torch.zeros(t.numel() + by, dtype=t.dtype, device=DEV)
+    flat[by:] = t.reshape(-1)
+    return flat[by:].view(t.shape)
+
+
+@pytest.mark.parametrize("rows", [5, 33, 97, 200])
+@pytest.mark.parametrize("what", ["inv_freq", "q", "cache"])
+def test_rotation_takes_operands_off_the_fused_kernels_alignment(rows, what):
+    """A frequency table off 16 bytes, queries or a cache off 8: the values of the aligned call."""
+    (h, w, bias), sizes, where, (cache, q) = rope_problem(rows)
+    ops.qkv_rope_store(h, w, bias, *sizes, *where, cache, q)
+    cache2, q2 = torch.zeros_like(cache), torch.zeros_like(q)
+    if what == "inv_freq":
+        where = (shifted(where[0], 1), *where[1:])
+    elif what == "q":
+        q2 = shifted(q2, 1)
+    else:
+        cache2 = shifted(cache2, 1)
+    ops.qkv_rope_store(h, w, bias, *sizes, *where, cache2, q2)
+    # the same sums; cos and sin of the same float32 angles
+    assert pm.rel_err(q2.float().cpu(), q.float().cpu()) < 4e-3 and pm.rel_err(cache2.float().cpu(), cache.float().cpu()) < 4e-3
+
+
 @pytest.mark.parametrize("rows,K", [(97, 3584), (128, 1536), (200, 3584), (500, 3584)])
 def test_rotation_rides_on_the_split_products_of_prompts(rows, K):
     """The same fusion at a prompt's rows (tiles of 128 tokens, pairs of SMs with K split): 28 query and 4 key/value heads of
