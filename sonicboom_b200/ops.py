@@ -348,6 +348,7 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
     and the float32 row is never written; else the product and `rope_store` run one after the other."""
     M, K = h.shape
     N = w.shape[0]
+    assert w.shape[1] == K, f"qkv_rope_store: h is [{M},{K}], w is {tuple(w.shape)}"
     has_kv = cache is not None
     l = lib()
     fused = None
@@ -369,11 +370,11 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
         return rope_store(qkv, n_q_heads, n_kv_heads, head_dim, rotary_dim, inv_freq, row_seq, row_pos,
                           page_off, page_ids, page_size, cache, q_out)
     assert inv_freq.dtype == torch.float32 and inv_freq.numel() >= rotary_dim // 2
-    rope = RopeStore(n_q_heads, n_kv_heads, head_dim, rotary_dim, inv_freq.data_ptr(),
+    rope = RopeStore(n_q_heads, n_kv_heads, head_dim, rotary_dim, _ptr(inv_freq),
                      _i32(row_seq, "row_seq"), _i32(row_pos, "row_pos"),
                      _i32(page_off, "page_off") if has_kv else None,
                      _i32(page_ids, "page_ids") if has_kv else None, page_size,
-                     cache.data_ptr() if has_kv else None, _ptr(q_out))
+                     _ptr(cache), _ptr(q_out))
     if fused == "skinny":
         _check(l.sb_gemm_skinny_rope(_ptr(h), BF16, _ptr(w), BF16, M, N, K, _ptr(bias),
                                      _code(bias.dtype) if bias is not None else 0, ctypes.byref(rope), _stream()),

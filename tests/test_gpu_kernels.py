@@ -863,6 +863,15 @@ def test_rotation_takes_operands_off_the_fused_kernels_alignment(rows, what):
     assert pm.rel_err(q2.float().cpu(), q.float().cpu()) < 4e-3 and pm.rel_err(cache2.float().cpu(), cache.float().cpu()) < 4e-3
 
 
+@pytest.mark.parametrize("rows", [5, 33, 200])
+def test_fused_rotation_refuses_what_the_two_kernels_refuse(rows):
+    """Weights of another inner size, a frequency table on the host, a cache that is not contiguous: before any launch."""
+    (h, w, bias), sizes, where, (cache, q) = rope_problem(rows)
+    for bad in (dict(w=w[:, :1024].contiguous()), dict(inv=where[0].cpu()), dict(cache=torch.cat([cache, cache], -1)[..., :128])):
+        with pytest.raises((AssertionError, ops.KernelError)):
+            ops.qkv_rope_store(h, bad.get("w", w), bias, *sizes, bad.get("inv", where[0]), *where[1:], bad.get("cache", cache), q)
+
+
 @pytest.mark.parametrize("rows,K", [(97, 3584), (128, 1536), (200, 3584), (500, 3584)])
 def test_rotation_rides_on_the_split_products_of_prompts(rows, K):
     """The same fusion at a prompt's rows (tiles of 128 tokens, pairs of SMs with K split): 28 query and 4 key/value heads of
