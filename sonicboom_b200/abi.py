@@ -34,6 +34,7 @@ CORE = {
     "sb_cast": ("i", "pipizs"),
     "sb_rope_store": ("i", "piiiiipppppipipiis"),
     "sb_gemm_plain": ("i", _GEMM),
+    "sb_gemm_f32": ("i", "ppiiiipippiis"),
     "sb_gemm_skinny": ("i", _GEMM),
     "sb_gemm_skinny_gated": ("i", "pipiiiipiffis"),
     "sb_gemm_skinny_takes_rope": ("i", "iiiiiii"),

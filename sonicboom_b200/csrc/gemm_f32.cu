@@ -53,7 +53,6 @@ __device__ __forceinline__ void f32_store(const F32Args& p, TO* out, int m, int 
 // ---------------------------------------------------------------------------- few rows
 constexpr int ROWS_WARPS = 4;
 constexpr int ROWS_MAX = 32;              // rows that stream the weights, in groups of eight
-constexpr int SMS = 148;
 
 __device__ __forceinline__ float4 load_weights(const float* p) {       // read once: past L1
   float4 v;
@@ -338,7 +337,7 @@ int launch_tile(const F32Args& p, TO* out, int splits, cudaStream_t stream) {
   const size_t smem = Tile<TM>::FLOATS * sizeof(float);
   // every call sets it, as it belongs to the current device's copy of the kernel; it costs nothing beside the product
   if (cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<TM, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))
-    SB_FAIL(SB_ERR_CUDA, "sb_gemm_plain: %s", cudaGetErrorString(e));
+    SB_FAIL(SB_ERR_CUDA, "sb_gemm_f32: %s", cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((p.M + Tile<TM>::BM - 1) / Tile<TM>::BM) * (unsigned)((p.N + BN - 1) / BN), 1, splits);
   cfg.blockDim = dim3(TILE_THREADS);
@@ -359,12 +358,12 @@ int launch_tile(const F32Args& p, TO* out, int splits, cudaStream_t stream) {
 // Rows of a thread's tile and blocks that share K.  A K tile of a block costs its FMAs (16 TM) or the loads that feed
 // them (4 (TM + 16)), whichever is more; an SM's blocks follow each other, and one alone on its SM (four warps) leaves
 // about a third of the time unused.  At least four K tiles are worth a block.
-void pick_tile(int M, int N, int K, int& tm, int& splits) {
+void pick_tile(int M, int N, int K, int n_sms, int& tm, int& splits) {
   const long tiles_n = (N + BN - 1) / BN, tiles_k = (K + BK - 1) / BK;
   double least = 0.0;
   for (int t : {8, 7, 6, 5, 4, 2})
     for (int s = 1; s <= 8 && (s == 1 || tiles_k >= 4 * s); ++s) {
-      const long blocks = (M + 16 * t - 1) / (16 * t) * tiles_n * s, each = (blocks + SMS - 1) / SMS;
+      const long blocks = (M + 16 * t - 1) / (16 * t) * tiles_n * s, each = (blocks + n_sms - 1) / n_sms;
       const double block = (double)(16 * t > 4 * (t + 16) ? 16 * t : 4 * (t + 16)) * (double)((tiles_k + s - 1) / s);
       const double cost = block * (double)each * (each == 1 ? 1.5 : 1.0);
       if (least == 0.0 || cost < least * 0.99) { least = cost; tm = t; splits = s; }
@@ -372,7 +371,7 @@ void pick_tile(int M, int N, int K, int& tm, int& splits) {
 }
 
 template <typename TO>
-int run_f32(const F32Args& p, TO* out, cudaStream_t stream) {
+int run_f32(const F32Args& p, TO* out, int n_sms, cudaStream_t stream) {
   if (p.M <= ROWS_MAX) {
     if (p.M == 1) launch_rows<1, 4, TO>(p, out, stream);
     else if (p.M == 2) launch_rows<2, 4, TO>(p, out, stream);
@@ -381,7 +380,7 @@ int run_f32(const F32Args& p, TO* out, cudaStream_t stream) {
     return SB_OK;
   }
   int tm = 8, splits = 1;
-  pick_tile(p.M, p.N, p.K, tm, splits);
+  pick_tile(p.M, p.N, p.K, n_sms, tm, splits);
   switch (tm) {
     case 8: return launch_tile<8, TO>(p, out, splits, stream);
     case 7: return launch_tile<7, TO>(p, out, splits, stream);
@@ -399,19 +398,24 @@ int run_f32(const F32Args& p, TO* out, cudaStream_t stream) {
 // whose tiles give every SM work (17 rows of 17920 x 1536: 51 us, streaming the weights 77; of 1536 x 1536 13 and 9).
 constexpr int SPLIT_MIN_K = 256, SPLIT_WIDE_ROWS = 16, SPLIT_WIDE_N = 8192;
 int sb_gemm_f32_tc5(const float* A, const float* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
-                    const float* residual, void* out, int out_dtype, cudaStream_t stream);
+                    const float* residual, void* out, int out_dtype, int n_sms, cudaStream_t stream);
 
-bool sb_gemm_f32_takes(const void* A, const void* W, int K) {
-  return K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-}
+int sb_check_linear_args(const char* who, int M, int N, int K, int epilogue, const void* bias, const float* residual, int out_dtype);
 
-int sb_gemm_f32(const void* A, const void* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
-                const float* residual, void* out, int out_dtype, cudaStream_t stream) {
+extern "C" int sb_gemm_f32(const float* A, const float* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
+                           const float* residual, void* out, int out_dtype, int n_sms, cudaStream_t stream) {
+  if (!sb_valid_dtype(out_dtype) || (bias && !sb_valid_dtype(bias_dtype)))
+    SB_FAIL(SB_ERR_ARG, "sb_gemm_f32: dtype codes %d %d", out_dtype, bias_dtype);
+  if (int rc = sb_check_linear_args("sb_gemm_f32", M, N, K, epilogue, bias, residual, out_dtype)) return rc;
+  if (!A || !W || n_sms <= 0) SB_FAIL(SB_ERR_ARG, "sb_gemm_f32: operands missing, or %d SMs", n_sms);
+  if (K % 4 || (((uintptr_t)A | (uintptr_t)W) & 15))
+    SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_f32: rows must start on 16 bytes (K = %d): sb_gemm_plain takes the others", K);
+  if (M > 65535 * 64) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_f32: M=%d is too many rows", M);
   if (K >= SPLIT_MIN_K && (M > ROWS_MAX || (M > SPLIT_WIDE_ROWS && N >= SPLIT_WIDE_N)))
-    return sb_gemm_f32_tc5((const float*)A, (const float*)W, M, N, K, epilogue, bias, bias_dtype, residual, out, out_dtype, stream);
-  const F32Args p{(const float*)A, (const float*)W, M, N, K, epilogue, bias, bias_dtype, residual};
-  const int rc = out_dtype == SB_F32 ? run_f32(p, (float*)out, stream) : run_f32(p, (__nv_bfloat16*)out, stream);
+    return sb_gemm_f32_tc5(A, W, M, N, K, epilogue, bias, bias_dtype, residual, out, out_dtype, n_sms, stream);
+  const F32Args p{A, W, M, N, K, epilogue, bias, bias_dtype, residual};
+  const int rc = out_dtype == SB_F32 ? run_f32(p, (float*)out, n_sms, stream) : run_f32(p, (__nv_bfloat16*)out, n_sms, stream);
   if (rc) return rc;
-  SB_CHECK_LAUNCH("sb_gemm_plain (float32)");
+  SB_CHECK_LAUNCH("sb_gemm_f32");
   return SB_OK;
 }

@@ -288,14 +288,14 @@ bool tc_map(CUtensorMap* map, const float* base, int rows, int K, int box_rows) 
 }
 
 // Blocks that share a tile's K: as many as run at once, at most eight, with at least four stages of K each.  A block has an SM
-// to itself and a cluster's blocks lie in one group of SMs, so fewer than 148 / 8 clusters of eight may fit: 16 tiles with eight
+// to itself and a cluster's blocks lie in one group of SMs, so fewer than (SMs / 8) clusters of eight may fit: 16 tiles with eight
 // blocks each ran in two waves.  (The counts belong to the kernel on this kind of device.)
 template <typename TO>
-int tc_splits(long tiles, int K) {
+int tc_splits(long tiles, int K, int n_sms) {
   static int most[9] = {0};
   const long k_tiles = (K + TC_K - 1) / TC_K;
   for (int s = 8; s > 1; --s) {
-    if (k_tiles < 4 * s || tiles * s > 148) continue;
+    if (k_tiles < 4 * s || tiles * s > n_sms) continue;
     if (most[s] == 0) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(1, 1, s);
@@ -317,21 +317,21 @@ int tc_splits(long tiles, int K) {
 }
 
 template <typename TO>
-int tc_launch(TcArgs p, TO* out, cudaStream_t stream) {
+int tc_launch(TcArgs p, TO* out, int n_sms, cudaStream_t stream) {
   p.tiles_m = (p.M + TC_MAX_TOKENS - 1) / TC_MAX_TOKENS;
   p.tokens = ((p.M + p.tiles_m - 1) / p.tiles_m + 31) / 32 * 32;
   p.tiles_m = (p.M + p.tokens - 1) / p.tokens;
   const long tiles = (long)p.tiles_m * ((p.N + TC_ROWS - 1) / TC_ROWS);
-  if (tiles > 2147483647L) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_plain: too many tiles");
+  if (tiles > 2147483647L) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_f32: too many tiles");
   p.stages = (TC_SMEM - 1024) / tc_stage_bytes(p.tokens) - 2;
   if (p.stages > TC_MAX_STAGES) p.stages = TC_MAX_STAGES;
   CUtensorMap map_w, map_a;
   if (!tc_map(&map_w, p.W, p.N, p.K, TC_ROWS) || !tc_map(&map_a, p.A, p.M, p.K, p.tokens))
-    SB_FAIL(SB_ERR_CUDA, "sb_gemm_plain: cuTensorMapEncodeTiled failed");
+    SB_FAIL(SB_ERR_CUDA, "sb_gemm_f32: cuTensorMapEncodeTiled failed");
   // every call sets it, as it belongs to the current device's copy of the kernel; it costs nothing beside the product
   if (cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc5_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM))
-    SB_FAIL(SB_ERR_CUDA, "sb_gemm_plain: %s", cudaGetErrorString(e));
-  const int splits = tc_splits<TO>(tiles, p.K);
+    SB_FAIL(SB_ERR_CUDA, "sb_gemm_f32: %s", cudaGetErrorString(e));
+  const int splits = tc_splits<TO>(tiles, p.K, n_sms);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)tiles, 1, splits);
   cfg.blockDim = dim3(TC_THREADS);
@@ -352,12 +352,12 @@ int tc_launch(TcArgs p, TO* out, cudaStream_t stream) {
 }  // namespace
 
 int sb_gemm_f32_tc5(const float* A, const float* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
-                    const float* residual, void* out, int out_dtype, cudaStream_t stream) {
+                    const float* residual, void* out, int out_dtype, int n_sms, cudaStream_t stream) {
   TcArgs p{};
   p.A = A; p.W = W; p.M = M; p.N = N; p.K = K; p.epilogue = epilogue; p.bias = bias; p.bias_dtype = bias_dtype; p.residual = residual;
-  const int rc = out_dtype == SB_F32 ? tc_launch(p, (float*)out, stream) : tc_launch(p, (__nv_bfloat16*)out, stream);
+  const int rc = out_dtype == SB_F32 ? tc_launch(p, (float*)out, n_sms, stream) : tc_launch(p, (__nv_bfloat16*)out, n_sms, stream);
   if (rc) return rc;
-  SB_CHECK_LAUNCH("sb_gemm_plain (float32, tensor cores)");
+  SB_CHECK_LAUNCH("sb_gemm_f32 (tensor cores)");
   return SB_OK;
 }
 

@@ -1,7 +1,7 @@
 // Plain CUDA-core matrix product with float32 accumulation: out[M,N] = A[M,K] . W[N,K]^T (FFMA only, no tensor
-// cores, no reduced-precision mode).  It takes every size, alignment and mix of operand types; float32 operands whose
-// rows start on 16 bytes go on to gemm_f32.cu, and bfloat16 operands run here where the tensor-core kernels are
-// checked against it.  Each output element is one thread's sum over K in ascending order, so a row's result does not
+// cores, no reduced-precision mode).  It takes every size, alignment and mix of operand types, and is what the other
+// product kernels are checked against; float32 operands whose rows start on 16 bytes run gemm_f32.cu unless a caller asks
+// for this kernel.  Each output element is one thread's sum over K in ascending order, so a row's result does not
 // depend on what else is in the launch.
 //
 // Epilogues (the fusions the reference's passes make on its graphs: bias into the product,
@@ -113,11 +113,6 @@ int sb_check_linear_args(const char* who, int M, int N, int K, int epilogue, con
   return SB_OK;
 }
 
-// gemm_f32.cu: the same product of float32 operands whose rows start on 16 bytes
-bool sb_gemm_f32_takes(const void* A, const void* W, int K);
-int sb_gemm_f32(const void* A, const void* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
-                const float* residual, void* out, int out_dtype, cudaStream_t stream);
-
 extern "C" int sb_gemm_plain(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N,
                              int K, int epilogue, const void* bias, int bias_dtype,
                              const float* residual, void* out, int out_dtype,
@@ -130,8 +125,6 @@ extern "C" int sb_gemm_plain(const void* A, int a_dtype, const void* W, int w_dt
     return rc;
   const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
   if (grid.y > 65535) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_plain: M=%d is too many rows", M);
-  if (a_dtype == SB_F32 && w_dtype == SB_F32 && sb_gemm_f32_takes(A, W, K))
-    return sb_gemm_f32(A, W, M, N, K, epilogue, bias, bias_dtype, residual, out, out_dtype, stream);
   SB_DISPATCH_DTYPE(a_dtype, TA, {
     SB_DISPATCH_DTYPE(w_dtype, TW, {
       SB_DISPATCH_DTYPE(out_dtype, TO, {

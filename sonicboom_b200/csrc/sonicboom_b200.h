@@ -134,6 +134,10 @@ int sb_rope_store(const float* qkv, int n_rows, int n_q_heads, int n_kv_heads, i
 int sb_gemm_plain(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
                   int epilogue, const void* bias, int bias_dtype, const float* residual,
                   void* out, int out_dtype, sb_stream_t stream);
+/* The same for float32 operands whose rows start on 16 bytes (K a multiple of 4): few rows stream the weights with FFMA,
+ * many run on the tensor cores with every operand split into two TF32 values. */
+int sb_gemm_f32(const float* A, const float* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
+                const float* residual, void* out, int out_dtype, int n_sms, sb_stream_t stream);
 int sb_gemm_skinny(const void* A, int a_dtype, const void* W, int w_dtype, int M, int N, int K,
                    int epilogue, const void* bias, int bias_dtype, const float* residual,
                    void* out, int out_dtype, sb_stream_t stream);

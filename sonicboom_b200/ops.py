@@ -225,9 +225,9 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 
 
     bfloat16 operands run on tensor cores: `kernel` "tc5" (TMA + tcgen05), "skinny" (weights
     streamed into mma.sync fragments, at most SKINNY_MAX_ROWS rows), "tiled" (mma.sync tiles),
-    or "auto", which picks between the first two (see `_pick_kernel`).  float32 operands run
-    sb_gemm_plain's float32 forms (FFMA, or tensor cores with every operand split in two), inner
-    sizes that are not multiples of 8 and bfloat16 with `kernel="plain"` its plain FFMA kernel.  A
+    or "auto", which picks between the first two (see `_pick_kernel`).  float32 operands whose rows start on 16
+    bytes run sb_gemm_f32 (FFMA for few rows, else tensor cores with every operand split in two); `kernel="plain"`, other
+    alignments and bfloat16 at inner sizes that are not multiples of 8 run the plain FFMA kernel.  A
     bfloat16 activation with a float32 weight is cast to float32 first.  The split-K decode
     form keeps one workspace per device, so products on one device must be ordered in a stream.
     """
@@ -312,6 +312,9 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 
         _check(l.sb_gemm_skinny(*args), "linear (weight-streaming kernel)")
     elif fast and kernel == "tiled":
         _check(l.sb_gemm_tiled(*args), "linear (tiled kernel)")
+    elif a.dtype == torch.float32 and kernel != "plain" and K % 4 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0:
+        _check(l.sb_gemm_f32(_ptr(a), _ptr(w), M, N, K, *args[7:-1], _sm_count(a.device), _stream()),
+               "linear (float32 kernels)")
     elif kernel in ("plain", "auto") or not fast:
         _check(l.sb_gemm_plain(*args), "linear (plain kernel)")
     else:

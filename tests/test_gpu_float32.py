@@ -15,13 +15,6 @@ def rnd(*shape, seed=0, scale=1.0):
     return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).mul_(scale).to(DEV)
 
 
-def off_by_one(t):
-    """The same values at an address that is no multiple of 16: the plain kernel takes them."""
-    flat = torch.empty(t.numel() + 1, device=DEV)
-    flat[1:] = t.reshape(-1)
-    return flat[1:].view(t.shape)
-
-
 # rows: one to 32 stream the weights (1, 2, 4 and groups of 8), 33 on are tiled (2 to 8 rows a thread); K: one lane's
 # 16 bytes, less and more than a warp's 128 values, odd numbers of K tiles; N: less than a block's rows or columns
 @pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 32, 33, 48, 81, 112, 129, 201])
@@ -38,15 +31,28 @@ def test_products(M, N, K):
             z = y.view(M, -1, 2, 8)
             want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2)
         errs = []
-        for x in (a, off_by_one(a)):
+        for kernel in ("auto", "plain"):
             out = res.clone() if epi == ops.EPI_RESIDUAL else torch.full(want.shape, float("nan"), device=DEV, dtype=dtype)
-            ops.linear(x, w, out, epi, bias=bias if epi == ops.EPI_BIAS else None,
-                       residual=out if epi == ops.EPI_RESIDUAL else None)
+            ops.linear(a, w, out, epi, bias=bias if epi == ops.EPI_BIAS else None,
+                       residual=out if epi == ops.EPI_RESIDUAL else None, kernel=kernel)
             errs.append(float((out.double() - want).norm() / want.norm()))
         # sums of K terms that are rounded one after the other are off by about sqrt(K) / 2 * 2^-24 of their terms'
         # root mean square sum, squared or multiplied by about twice that
         assert errs[0] < (2 ** -8 if dtype == torch.bfloat16 else (K ** 0.5 + 8) * 2 ** -24 * 2), (epi, errs)
         assert errs[0] <= 1.3 * errs[1] + 2 ** -24, (epi, errs)     # and no more than the plain kernel's
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 40, 64), (33, 40, 64), (40, 272, 512), (201, 1536, 1540)])
+def test_plain_is_the_plain_kernel(M, N, K):
+    """Every output one chain over K, to the bit, in float32 as in the sums of bfloat16 operands of the same values; and at an
+    address off 16 bytes, where "auto" takes it too."""
+    a, w = rnd(M, K).bfloat16(), rnd(N, K, seed=1).bfloat16()
+    got = [torch.empty(M, N, device=DEV) for _ in range(3)]
+    ops.linear(a, w, got[0], kernel="plain")
+    ops.linear(a.float(), w.float(), got[1], kernel="plain")
+    off = torch.empty(M * K + 1, device=DEV)[1:].view(M, K)
+    ops.linear(off.copy_(a), w.float(), got[2])
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
 
 
 # the tensor-core form: token tiles of 32 to 224, one more than a tile, three tiles; K of its least, with a ragged last stage, shared by
