@@ -30,7 +30,7 @@ struct F32Attn {
   const int32_t* page_off;
   const int32_t* page_ids;
   const float* cache;
-  int page_size, n_pages, n_q_heads, n_kv_heads, hd, window, chunk, bias_len;
+  int n_rows, page_size, n_pages, n_q_heads, n_kv_heads, hd, window, chunk, bias_len;
   float scale, softcap;
   const float* sink;
   const float* bias;
@@ -68,7 +68,8 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
   const int seq = blockIdx.x / tiles_per_seq, tile = blockIdx.x % tiles_per_seq, g = blockIdx.y;
   const int group = p.n_q_heads / p.n_kv_heads;
   // the step's plan was written before the step's first kernel, which triggers after its own wait
-  const int row0 = p.seq_row0[seq], n_new = p.seq_row0[seq + 1] - row0, pos0 = p.seq_pos0[seq];
+  // (n_rows may be less than the plan's: the caller wants its first rows)
+  const int row0 = p.seq_row0[seq], n_new = min(p.seq_row0[seq + 1], p.n_rows) - row0, pos0 = p.seq_pos0[seq];
   const int pairs = n_new * group, pair0 = tile * QB;
   if (pair0 >= pairs) return;                           // the same for the whole cluster
   const int32_t* pages = p.page_ids + p.page_off[seq];
@@ -328,7 +329,7 @@ extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_se
   if (n_seqs <= 0 || max_new <= 0) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: %d sequences, at most %d new rows", n_seqs, max_new);
   if (hd % 4 || hd > 256 || n_kv_heads > 65535)
     SB_FAIL(SB_ERR_UNSUPPORTED, "sb_attention_f32: head size %d (a multiple of 4 up to 256), %d key/value heads", hd, n_kv_heads);
-  const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
+  const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, n_rows, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
                   chunk, bias_len, scale, softcap, sink, bias};
   // one token's heads fit the 16-row form; a row of a longer stretch sees up to 64 rows' keys loaded once, or 32 where 64
   // leave SMs without a block (a prompt of 201 tokens: 76 blocks that go through two tiles of keys each, or 304 with one)

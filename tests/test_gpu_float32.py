@@ -153,3 +153,21 @@ def test_attention_of_values_that_are_not_finite():
     got, want = attention_both(4, 2, 32, [10], [120], edit=edit)
     assert torch.equal(got.isfinite(), want.isfinite()) and bool(got[:74].isfinite().all())
     assert pm.rel_err(got[:74].cpu(), want[:74].cpu()) < 16 * 2 ** -24 * 2
+
+
+def test_attention_of_a_plans_first_rows():
+    """Queries for fewer rows than the plan has, as the plain kernel takes them: the others are neither read nor written."""
+    cache = Cache([KVNeed(2, 32, 0, 0, 0)], [None], 64 * 4, torch.float32, DEV)
+    storage = cache.groups[0].entry_storage(0)
+    storage.copy_(rnd(*storage.shape))
+    slots = [cache.open() for _ in range(2)]
+    for s, h in zip(slots, (5, 40)):
+        cache.reserve(s, h + 9)
+        cache.advance(s, h)
+    plan = StepPlan(cache, [StepEntry(s, [0] * 9, []) for s in slots], DEV)
+    for n in (4, 9, 13):
+        q = rnd(n, 4, 32, seed=1)
+        out = torch.full((2, 18, 128), float("nan"), device=DEV)
+        for o, kernel in zip(out, ("auto", "plain")):
+            ops.attention(q, o[:n], plan, 0, storage, 4, 2, 32, 0, 32 ** -0.5, kernel=kernel)
+        assert pm.rel_err(out[0, :n].cpu(), out[1, :n].cpu()) < 16 * 2 ** -24 * 2 and bool(out[0, n:].isnan().all())
