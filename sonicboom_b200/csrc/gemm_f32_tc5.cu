@@ -25,6 +25,7 @@
 #include <cooperative_groups.h>
 #include <float.h>
 
+#include "device_cache.h"
 #include "tc5.cuh"
 
 namespace cg = cooperative_groups;
@@ -287,32 +288,38 @@ bool tc_map(CUtensorMap* map, const float* base, int rows, int K, int box_rows) 
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Clusters of `blocks` blocks that the current device runs at once.
+template <typename TO>
+int tc_clusters(int blocks) {
+  static SbDeviceCache most[9];
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) device = -1;
+  return most[blocks].get(device, [&] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, blocks);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = TC_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = blocks;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_tc5_kernel<TO>, &cfg) == cudaSuccess) return n;
+    cudaGetLastError();
+    return -1;
+  });
+}
+
 // Blocks that share a tile's K: as many as run at once, at most eight, with at least four stages of K each.  A block has an SM
 // to itself and a cluster's blocks lie in one group of SMs, so fewer than (SMs / 8) clusters of eight may fit: 16 tiles with eight
-// blocks each ran in two waves.  (The counts belong to the kernel on this kind of device.)
+// blocks each ran in two waves.
 template <typename TO>
 int tc_splits(long tiles, int K, int n_sms) {
-  static int most[9] = {0};
   const long k_tiles = (K + TC_K - 1) / TC_K;
-  for (int s = 8; s > 1; --s) {
-    if (k_tiles < 4 * s || tiles * s > n_sms) continue;
-    if (most[s] == 0) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(1, 1, s);
-      cfg.blockDim = dim3(TC_THREADS);
-      cfg.dynamicSmemBytes = TC_SMEM;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = s;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_tc5_kernel<TO>, &cfg) != cudaSuccess) cudaGetLastError();
-      most[s] = n > 0 ? n : -1;
-    }
-    if (tiles <= most[s]) return s;
-  }
+  for (int s = 8; s > 1; --s)
+    if (k_tiles >= 4 * s && tiles * s <= n_sms && tiles <= tc_clusters<TO>(s)) return s;
   return 1;
 }
 
