@@ -6,26 +6,18 @@
 //   chunks of 128 values, a lane reads 16 bytes of every weight row past L1 and 16 bytes of every activation row
 //   (which the SM's blocks keep in L1), so that a warp's loads run along the rows.  Sums: a lane's terms in
 //   ascending order, then the lanes in a fixed tree, then the warps in order.
-// * gemm_f32_tile_kernel, many rows at a short K: bound by FFMA issue and shared-memory loads.  128 threads compute 16 TM x 128
+// * gemm_f32_tile_kernel, many rows at a K below 256: bound by FFMA issue and shared-memory loads.  128 threads compute 16 TM x 128
 //   outputs, TM x 16 a thread: a load from shared memory costs its bytes times its lanes whether lanes share the
 //   address or not, so a thread's tile is as large as the registers allow (TM 8: 24 values loaded for 128 FMA) and
-//   two products go into one packed FMA.  Tiles lie [k][row] in shared memory.  Where the tiles leave SMs idle a
-//   cluster of blocks shares K; its partial tiles meet in distributed shared memory and are added in rank order,
-//   so no workspace is needed.
+//   two products go into one packed FMA.  Tiles lie [k][row] in shared memory.  Every output is one chain over K in
+//   ascending order: the bits of the plain kernel.
 //
 // Measured on one B200 inside a step of the 1.5B layers (28 layers: 2048, 1536 and 17920 x 1536, 1536 x 8960): three rows
-// 15.5 us a product on average where the plain kernel took 636 (one row of 151936 x 1536: 140 us, 6.6 TB/s).  The tile form at
-// 201 rows took 193 us where the plain kernel took 821 (17920 x 1536: 330 us, 34 TFLOP/s of 74), and the tensor cores 56.
-// Rows against tensor cores at 24 rows: 1536 x 8960 40 and 38 us, 2048 x 1536 11 and 14, 17920 x 1536 77 and 50; hence the lines.
-// Error against float64 at K = 8960: 1.2e-7 and 4.3e-7, the plain kernel's terms one after the other 9e-7.
-//
+// 15.5 us a product on average where the plain kernel took 636 (one row of 151936 x 1536: 140 us, 6.6 TB/s).
+// Error against float64 at K = 8960: 1.2e-7 (the plain kernel's terms one after the other 9e-7).
 // Epilogues as in gemm_plain.cu, which computes the same sums in another order and takes the sizes and
 // alignments that these forms do not (K a multiple of 4, rows on 16 bytes).
-#include <cooperative_groups.h>
-
 #include "common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -163,7 +155,7 @@ template <int TM>
 struct Tile {
   static constexpr int BM = 16 * TM, PITCH = BM + 4;
   static constexpr int STAGE = BK * (PITCH + W_PITCH);
-  static constexpr int FLOATS = 2 * STAGE > BM * W_PITCH ? 2 * STAGE : BM * W_PITCH;     // the partial tile lies over the stages
+  static constexpr int FLOATS = 2 * STAGE > BM * W_PITCH ? 2 * STAGE : BM * W_PITCH;     // the finished tile lies over the stages
   static constexpr int A_UNITS = BM / 16 * 2, W_UNITS = BN / 16 * 2;      // 16 rows x 2 columns of 16 bytes, a warp's load
   static constexpr int A_LOADS = (A_UNITS + 3) / 4, W_LOADS = W_UNITS / 4;
 };
@@ -191,9 +183,7 @@ gemm_f32_tile_kernel(F32Args p, TO* out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tiles_m = (p.M + T::BM - 1) / T::BM;       // tiles of the same weight rows follow each other
   const int m0 = (int)(blockIdx.x % tiles_m) * T::BM, n0 = (int)(blockIdx.x / tiles_m) * BN;
-  // this block's share of the K tiles
-  const int tiles = (p.K + BK - 1) / BK, splits = gridDim.z, rank = blockIdx.z;
-  const int t0 = (int)((long)tiles * rank / splits), t1 = (int)((long)tiles * (rank + 1) / splits);
+  const int tiles = (p.K + BK - 1) / BK;
   const int r_in = lane >> 1, c_in = lane & 1;          // a warp's load: 16 rows, two neighbouring 16-byte columns
 
   float4 ra[T::A_LOADS], rw[T::W_LOADS];
@@ -244,14 +234,12 @@ gemm_f32_tile_kernel(F32Args p, TO* out) {
     for (int j = 0; j < 8; ++j) acc[i][j] = pack(0.0f, 0.0f);
 
   sb_pdl_wait();
-  if (t0 < t1) {
-    fetch(t0);
-    put(0);
-  }
+  fetch(0);
+  put(0);
   __syncthreads();
-  for (int t = t0; t < t1; ++t) {
-    const int stage = (t - t0) & 1;
-    if (t + 1 < t1) fetch(t + 1);
+  for (int t = 0; t < tiles; ++t) {
+    const int stage = t & 1;
+    if (t + 1 < tiles) fetch(t + 1);
     const float* sa = smem + stage * T::STAGE + ty * TM;
     const float* sw = smem + stage * T::STAGE + BK * T::PITCH + tx * 4;
 #pragma unroll
@@ -282,12 +270,12 @@ gemm_f32_tile_kernel(F32Args p, TO* out) {
         for (int j = 0; j < 8; ++j) fma_pair(acc[i][j], a[i], w[j]);
     }
     // the other stage was last read before the barrier that ended the previous round
-    if (t + 1 < t1) put(stage ^ 1);
+    if (t + 1 < tiles) put(stage ^ 1);
     __syncthreads();
   }
   sb_pdl_launch();
 
-  // the partial tile, then the cluster's blocks share out its rows
+  // the tile through shared memory, so that a warp writes along a row
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -297,32 +285,16 @@ gemm_f32_tile_kernel(F32Args p, TO* out) {
       unpack(acc[i][2 * j + 1], v.z, v.w);
       *reinterpret_cast<float4*>(smem + (ty * TM + i) * W_PITCH + tx * 4 + 32 * j) = v;
     }
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  const float* peer[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) peer[s] = s < splits ? cluster.map_shared_rank(smem, s) : smem;
-  auto sum_at = [&](int at) {
-    float v = 0.0f;
-#pragma unroll
-    for (int s = 0; s < 8; ++s)
-      if (s < splits) v += peer[s][at];
-    return v;
-  };
+  __syncthreads();
   if (p.epilogue == SB_EPI_SWIGLU) {
-    for (int r = rank * 2 + (tid >> 6); r < T::BM; r += 2 * splits) {
-      const int c = tid & 63, at = r * W_PITCH + c / SB_SWIGLU_BLOCK * 2 * SB_SWIGLU_BLOCK + c % SB_SWIGLU_BLOCK;
-      const int m = m0 + r, j = n0 / 2 + c;
-      if (m < p.M && j < p.N / 2)
-        out[(size_t)m * (p.N / 2) + j] = sb_from_f32<TO>(sb_silu(sum_at(at)) * sum_at(at + SB_SWIGLU_BLOCK));
-    }
-  } else {
-    for (int r = rank; r < T::BM; r += splits) {
-      const int m = m0 + r, n = n0 + tid;
-      if (m < p.M && n < p.N) f32_store(p, out, m, n, sum_at(r * W_PITCH + tid));
-    }
+    const int c = tid & 63, at = c / SB_SWIGLU_BLOCK * 2 * SB_SWIGLU_BLOCK + c % SB_SWIGLU_BLOCK, j = n0 / 2 + c;
+    if (j < p.N / 2)
+      for (int r = tid >> 6; r < T::BM && m0 + r < p.M; r += 2)
+        out[(size_t)(m0 + r) * (p.N / 2) + j] =
+            sb_from_f32<TO>(sb_silu(smem[r * W_PITCH + at]) * smem[r * W_PITCH + at + SB_SWIGLU_BLOCK]);
+  } else if (n0 + tid < p.N) {
+    for (int r = 0; r < T::BM && m0 + r < p.M; ++r) f32_store(p, out, m0 + r, n0 + tid, smem[r * W_PITCH + tid]);
   }
-  cluster.sync();                                      // nobody's tile goes while another block reads it
 }
 
 template <int MT, int R, typename TO>
@@ -332,42 +304,17 @@ void launch_rows(const F32Args& p, TO* out, cudaStream_t stream) {
                         stream, p, out);
 }
 
+template <int TM>
+long tile_blocks(const F32Args& p) { return (long)((p.M + Tile<TM>::BM - 1) / Tile<TM>::BM) * ((p.N + BN - 1) / BN); }
+
 template <int TM, typename TO>
-int launch_tile(const F32Args& p, TO* out, int splits, cudaStream_t stream) {
+int launch_tile(const F32Args& p, TO* out, cudaStream_t stream) {
   const size_t smem = Tile<TM>::FLOATS * sizeof(float);
   // every call sets it, as it belongs to the current device's copy of the kernel; it costs nothing beside the product
   if (cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<TM, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))
     SB_FAIL(SB_ERR_CUDA, "sb_gemm_f32: %s", cudaGetErrorString(e));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((p.M + Tile<TM>::BM - 1) / Tile<TM>::BM) * (unsigned)((p.N + BN - 1) / BN), 1, splits);
-  cfg.blockDim = dim3(TILE_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = splits;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (sb_pdl_enabled() & SB_K_OTHER) ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<TM, TO>, p, out);
+  sb_launch<SB_K_OTHER>(gemm_f32_tile_kernel<TM, TO>, dim3((unsigned)tile_blocks<TM>(p)), dim3(TILE_THREADS), smem, stream, p, out);
   return SB_OK;
-}
-
-// Rows of a thread's tile and blocks that share K.  A K tile of a block costs its FMAs (16 TM) or the loads that feed
-// them (4 (TM + 16)), whichever is more; an SM's blocks follow each other, and one alone on its SM (four warps) leaves
-// about a third of the time unused.  At least four K tiles are worth a block.
-void pick_tile(int M, int N, int K, int n_sms, int& tm, int& splits) {
-  const long tiles_n = (N + BN - 1) / BN, tiles_k = (K + BK - 1) / BK;
-  double least = 0.0;
-  for (int t : {8, 7, 6, 5, 4, 2})
-    for (int s = 1; s <= 8 && (s == 1 || tiles_k >= 4 * s); ++s) {
-      const long blocks = (M + 16 * t - 1) / (16 * t) * tiles_n * s, each = (blocks + n_sms - 1) / n_sms;
-      const double block = (double)(16 * t > 4 * (t + 16) ? 16 * t : 4 * (t + 16)) * (double)((tiles_k + s - 1) / s);
-      const double cost = block * (double)each * (each == 1 ? 1.5 : 1.0);
-      if (least == 0.0 || cost < least * 0.99) { least = cost; tm = t; splits = s; }
-    }
 }
 
 template <typename TO>
@@ -379,16 +326,10 @@ int run_f32(const F32Args& p, TO* out, int n_sms, cudaStream_t stream) {
     else launch_rows<8, 4, TO>(p, out, stream);
     return SB_OK;
   }
-  int tm = 8, splits = 1;
-  pick_tile(p.M, p.N, p.K, n_sms, tm, splits);
-  switch (tm) {
-    case 8: return launch_tile<8, TO>(p, out, splits, stream);
-    case 7: return launch_tile<7, TO>(p, out, splits, stream);
-    case 6: return launch_tile<6, TO>(p, out, splits, stream);
-    case 5: return launch_tile<5, TO>(p, out, splits, stream);
-    case 4: return launch_tile<4, TO>(p, out, splits, stream);
-    default: return launch_tile<2, TO>(p, out, splits, stream);
-  }
+  // the largest tile that gives every SM a block, else the smallest
+  if (tile_blocks<8>(p) >= n_sms) return launch_tile<8, TO>(p, out, stream);
+  if (tile_blocks<4>(p) >= n_sms) return launch_tile<4, TO>(p, out, stream);
+  return launch_tile<2, TO>(p, out, stream);
 }
 
 }  // namespace

@@ -15,8 +15,9 @@ def rnd(*shape, seed=0, scale=1.0):
     return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).mul_(scale).to(DEV)
 
 
-# rows: one to 32 stream the weights (1, 2, 4 and groups of 8), 33 on are tiled (2 to 8 rows a thread); K: one lane's
-# 16 bytes, less and more than a warp's 128 values, odd numbers of K tiles; N: less than a block's rows or columns
+# rows: one to 32 stream the weights (1, 2, 4 and groups of 8), 33 on are tiled at a K below 256 and run on the tensor
+# cores from there on; K: one lane's 16 bytes, less and more than a warp's 128 values, odd numbers of K tiles; N: less than a
+# block's rows or columns
 @pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 32, 33, 48, 81, 112, 129, 201])
 @pytest.mark.parametrize("N,K", [(16, 4), (48, 132), (1536, 1540), (272, 8960), (130, 100)])
 def test_products(M, N, K):
@@ -53,6 +54,31 @@ def test_plain_is_the_plain_kernel(M, N, K):
     off = torch.empty(M * K + 1, device=DEV)[1:].view(M, K)
     ops.linear(off.copy_(a), w.float(), got[2])
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+# tiles of 128, 64 and 32 rows (the largest that gives each of 148 SMs a block), rows and columns that end inside a tile, K of
+# one 16-byte column, of whole and of ragged tiles of 16
+@pytest.mark.parametrize("M,N,tile", [(1000, 2400, 128), (897, 2450, 128), (500, 2400, 64), (1000, 1160, 64), (33, 130, 32), (97, 1536, 32)])
+@pytest.mark.parametrize("K", [4, 48, 132, 252])
+def test_tiled_products(M, N, tile, K):
+    """Every output one chain over K, as the plain kernel adds it: the same bits."""
+    blocks = lambda t: -(-M // t) * -(-N // 128)                               # noqa: E731
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:
+        assert tile == next((t for t in (128, 64) if blocks(t) >= sms), 32)
+    a, w, bias, res = rnd(M, K), rnd(N, K, seed=1), rnd(N, seed=2), rnd(M, N, seed=3)
+    for epi, dtype in [(ops.EPI_NONE, torch.float32), (ops.EPI_BIAS, torch.float32), (ops.EPI_RESIDUAL, torch.float32),
+                       (ops.EPI_RELU2, torch.float32), (ops.EPI_SWIGLU, torch.float32), (ops.EPI_BIAS, torch.bfloat16)]:
+        if epi == ops.EPI_SWIGLU and N % 16:
+            continue
+        got = []
+        for kernel in ("auto", "plain"):
+            out = res.clone() if epi == ops.EPI_RESIDUAL else \
+                torch.full((M, N // 2 if epi == ops.EPI_SWIGLU else N), float("nan"), device=DEV, dtype=dtype)
+            ops.linear(a, w, out, epi, bias=bias if epi == ops.EPI_BIAS else None, residual=out if epi == ops.EPI_RESIDUAL else None,
+                       kernel=kernel)
+            got.append(out)
+        assert torch.equal(got[0], got[1]) and bool(got[0].isfinite().all()), epi
 
 
 # the tensor-core form: token tiles of 32 to 224, one more than a tile, three tiles; K of its least, with a ragged last stage, shared by
@@ -97,15 +123,15 @@ def test_split_operands_let_what_is_not_finite_through():
     assert ops.tc5_status() == 0
 
 
-def test_products_let_infinities_through():
-    a, w = rnd(40, 256), rnd(64, 256, seed=1).abs()
+@pytest.mark.parametrize("rows,K", [(4, 256), (40, 252), (40, 256)])           # streamed, tiled, on the tensor cores
+def test_products_let_infinities_through(rows, K):
+    a, w = rnd(40, K), rnd(64, K, seed=1).abs()
     a[3, 7], a[35, 200], a[39, 0] = float("inf"), float("-inf"), float("nan")
-    for rows in (40, 4):                               # tiled, streamed
-        out = torch.empty(rows, 64, device=DEV)
-        ops.linear(a[:rows].contiguous(), w, out)
-        assert bool((out[3] == float("inf")).all()) and bool(out[:3].isfinite().all())
-        if rows == 40:
-            assert bool((out[35] == float("-inf")).all()) and bool(out[39].isnan().all()) and bool(out[36:39].isfinite().all())
+    out = torch.empty(rows, 64, device=DEV)
+    ops.linear(a[:rows].contiguous(), w, out)
+    assert bool((out[3] == float("inf")).all()) and bool(out[:3].isfinite().all())
+    if rows == 40:
+        assert bool((out[35] == float("-inf")).all()) and bool(out[39].isnan().all()) and bool(out[36:39].isfinite().all())
 
 
 def attention_both(hq, hkv, hd, held, new, window=0, chunk=0, sink=None, softcap=0.0, bias=None, edit=None, seed=0):
