@@ -2,15 +2,18 @@
 // key/value head of one sequence.
 //
 // A query row is a (token, head in group) pair, so that all query heads of a key/value head share its tiles.  Three
-// forms: 16 rows (a decode step: one token's heads), 64 rows (prompts), 32 rows (prompts whose 64-row tiles leave SMs idle).  Keys come in tiles of 64 at absolute
-// positions, which a cluster of blocks takes in turn (8 blocks for 16 rows, where a step has few blocks and the
-// sequence is long; 4 for 32 rows, 2 for 64); the blocks' running softmaxes are merged in rank order through distributed shared
-// memory, so no workspace is needed and a row's sums depend on its own keys and the form alone.
+// forms: 16 rows (a decode step: one token's heads), 64 rows (prompts), 32 rows (prompts whose 64-row tiles leave SMs idle).
+// Keys come in tiles of 64 at absolute positions.  Tile t belongs to part t % 8; every part has a running softmax of its own
+// and the eight are merged in order, in every form, so a row's bits depend on its own keys and position alone: not on the
+// form, and so not on the cut or on what else the step holds.  A cluster of blocks shares the parts out (8 blocks for
+// 16 rows, where a step has few blocks and the sequence is long; else 4, each with two parts one after the other) and merges
+// them through distributed shared memory; no workspace is needed.
 //
 // What attn_plain.cu says about masks, caps, biases and sinks holds here; that kernel (a block per row and head, a
 // warp per key) stays for head sizes this one does not take.  12/2 heads of 128: three single tokens at 100 to 400 keys
 // took 324 us there, bound by a block's dependent steps over its keys, and 16 here (19 when a tile's loads came one after
-// the other); a prompt of 201 tokens 183 and 50 (67 in 64-row tiles).
+// the other); a prompt of 201 tokens 183 and 50 (67 in 64-row tiles).  The eight parts in every form, where each form had as many
+// as blocks and so bits of its own, cost 201 tokens 40.0 to 41.3 us (the kernel alone), 4,000 tokens 2,465 to 2,502.
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -20,7 +23,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int THREADS = 256, KEYS = 64, LOADS = 4;
+constexpr int THREADS = 256, KEYS = 64, LOADS = 4, PARTS = 8;
 
 struct F32Attn {
   const float* q;
@@ -41,16 +44,16 @@ struct F32Attn {
 template <int TQ, int ND>
 struct Form {
   static constexpr int QB = 16 * TQ;
-  static constexpr int SPLITS = TQ == 1 ? 8 : TQ == 2 ? 4 : 2;
+  static constexpr int SPLITS = TQ == 1 ? 8 : 4, MINE = PARTS / SPLITS;       // blocks of a cluster, parts of a block
   static int floats(int hd) {      // queries, keys (later probabilities), values, maximum and sum, their merge
     const int kp = KEYS * (hd + 4), pp = QB * (KEYS + 4), op = QB * hd;
     const int first = kp > pp ? kp : pp;
-    return QB * hd + (first > op ? first : op) + KEYS * hd + 2 * QB;
+    return QB * hd + (first > op ? first : op) + KEYS * hd + 2 * MINE * QB;
   }
 };
 
 template <int TQ, int ND>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, ND <= 2 ? 2 : 1)           // two blocks fit an SM's shared memory at head sizes up to 128
 attn_f32_kernel(F32Attn p, int tiles_per_seq) {
   using F = Form<TQ, ND>;
   constexpr int QB = F::QB;
@@ -61,7 +64,8 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
   float* ps = ks;                                       // over the keys, once the scores are made
   const int first = max(max(KEYS * kpitch, QB * ppitch), QB * hd);
   float* vs = ks + first;
-  float* stat = vs + KEYS * hd;                         // maximum and sum per row, for the merge
+  float* stat = vs + KEYS * hd;                         // maximum and sum per part and row, for the merge
+  static_assert(F::MINE <= 2 && QB <= KEYS, "a block's parts lie over its keys and values");
   __shared__ int bad_values;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = blockIdx.z, tid = threadIdx.x;
@@ -104,6 +108,19 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 
   float m[TQ], l[TQ];
   float4 acc[TQ][ND];
+  const int t_lo = k_lo / KEYS, t_hi = k_hi >= k_lo ? k_hi / KEYS : -1;
+  // the first tile of a part (none: beyond t_hi)
+  auto first_tile = [&](int part) { return t_lo + (part - t_lo % PARTS + PARTS) % PARTS; };
+  // This block's parts, rank and rank + SPLITS, the empty ones left out.  The first of two is set aside in local memory (an index that
+  // the compiler does not know): kept in registers, or in a copy of the loop each, it cost 4,000 tokens 13 and 10 % more.
+  const bool two = F::MINE > 1 && first_tile(rank) <= t_hi && first_tile(rank + F::SPLITS) <= t_hi;
+  float4 kept[F::MINE][TQ][ND];
+  float2 kept_stat[F::MINE][TQ];
+  int last = 0;                                         // the part whose sums are in registers
+#pragma unroll 1
+  for (int j = 0; j < F::MINE; ++j) {
+  if (j > 0 && first_tile(rank + j * F::SPLITS) > t_hi) break;
+  last = j;
 #pragma unroll
   for (int i = 0; i < TQ; ++i) {
     m[i] = -INFINITY;
@@ -111,8 +128,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 #pragma unroll
     for (int d = 0; d < ND; ++d) acc[i][d] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
-
-  for (int t = k_lo / KEYS + rank; t <= k_hi / KEYS && k_hi >= k_lo; t += F::SPLITS) {
+  for (int t = first_tile(rank + j * F::SPLITS); t <= t_hi; t += PARTS) {
     const int base = t * KEYS;
     __syncthreads();                                    // the tile before this one has been read
     if (tid == 0) bad_values = 0;
@@ -235,34 +251,52 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
       }
     }
   }
+  if (two && j == 0) {
+#pragma unroll
+    for (int i = 0; i < TQ; ++i) {
+      kept_stat[j][i] = make_float2(m[i], l[i]);
+#pragma unroll
+      for (int d = 0; d < ND; ++d) kept[j][i][d] = acc[i][d];
+    }
+  }
+  }
 
-  // merge: every block leaves its sums over its keys' space, then takes a share of the rows
+  // merge: every block leaves its parts' sums over its keys' space, then takes a share of the rows
   sb_pdl_launch();
   __syncthreads();
   float* os = ks;
+  auto leave = [&](int j, const float4 (&sums)[TQ][ND], auto stat_of) {
 #pragma unroll
-  for (int i = 0; i < TQ; ++i) {
-    const int r = ty * TQ + i;
+    for (int i = 0; i < TQ; ++i) {
+      const int r = j * QB + ty * TQ + i;
 #pragma unroll
-    for (int d = 0; d < ND; ++d)
-      if (tx * 4 + 64 * d < hd) *reinterpret_cast<float4*>(os + r * hd + tx * 4 + 64 * d) = acc[i][d];
-    if (tx == 0) { stat[2 * r] = m[i]; stat[2 * r + 1] = l[i]; }
-  }
+      for (int d = 0; d < ND; ++d)
+        if (tx * 4 + 64 * d < hd) *reinterpret_cast<float4*>(os + r * hd + tx * 4 + 64 * d) = sums[i][d];
+      if (tx == 0) *reinterpret_cast<float2*>(stat + 2 * r) = stat_of(i);
+    }
+  };
+  leave(last, acc, [&](int i) { return make_float2(m[i], l[i]); });
+  if (two) leave(0, kept[last - 1], [&](int i) { return kept_stat[last - 1][i]; });
+  // part s is the (s / SPLITS)-th of block s % SPLITS
   cluster.sync();
   for (int r = rank * (QB / F::SPLITS) + ty; r < (rank + 1) * (QB / F::SPLITS); r += 16) {
     const int pair = pair0 + r;
     if (pair >= pairs) continue;
     const int h = g * group + pair % group, at = pos0 + pair / group;
     const bool row_live = at >= 0 && at / p.page_size < held / p.page_size;
-    float m_all = -INFINITY, total = 0.0f;
-    for (int s = 0; s < F::SPLITS; ++s) m_all = fmaxf(m_all, cluster.map_shared_rank(stat, s)[2 * r]);
-    if (p.sink) m_all = fmaxf(m_all, p.sink[h]);
-    float f[F::SPLITS];
+    float2 st[PARTS];
 #pragma unroll
-    for (int s = 0; s < F::SPLITS; ++s) {
-      const float* st = cluster.map_shared_rank(stat, s);
-      f[s] = st[2 * r] == -INFINITY ? 0.0f : expf(st[2 * r] - m_all);
-      total += st[2 * r + 1] * f[s];
+    for (int s = 0; s < PARTS; ++s)
+      st[s] = first_tile(s) <= t_hi ? *reinterpret_cast<const float2*>(cluster.map_shared_rank(stat, s % F::SPLITS) + 2 * (s / F::SPLITS * QB + r))
+                                    : make_float2(-INFINITY, 0.0f);
+    float m_all = p.sink ? p.sink[h] : -INFINITY, total = 0.0f;
+#pragma unroll
+    for (int s = 0; s < PARTS; ++s) m_all = fmaxf(m_all, st[s].x);
+    float f[PARTS];
+#pragma unroll
+    for (int s = 0; s < PARTS; ++s) {
+      f[s] = st[s].x == -INFINITY ? 0.0f : expf(st[s].x - m_all);
+      total += st[s].y * f[s];
     }
     if (p.sink) total += expf(p.sink[h] - m_all);
     const float inv = 1.0f / total;
@@ -274,8 +308,10 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
       float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (row_live) {
 #pragma unroll
-        for (int s = 0; s < F::SPLITS; ++s) {
-          const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(os, s) + r * hd + at_d);
+        for (int s = 0; s < PARTS; ++s) {
+          float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (first_tile(s) <= t_hi)
+            v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(os, s % F::SPLITS) + (s / F::SPLITS * QB + r) * hd + at_d);
           o.x = fmaf(v.x, f[s], o.x); o.y = fmaf(v.y, f[s], o.y); o.z = fmaf(v.z, f[s], o.z); o.w = fmaf(v.w, f[s], o.w);
         }
         o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
@@ -321,7 +357,7 @@ extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_se
                                 const int32_t* seq_pos0, const int32_t* page_off, const int32_t* page_ids, int page_size,
                                 const float* cache, int n_pages, int n_q_heads, int n_kv_heads, int hd, int window,
                                 float scale, const float* sink, float softcap, int chunk, const float* bias, int bias_len,
-                                cudaStream_t stream) {
+                                int n_sms, cudaStream_t stream) {
   if (chunk < 0 || (bias && bias_len < 1))
     SB_FAIL(SB_ERR_ARG, "sb_attention_f32: chunk %d, a distance bias of %d entries", chunk, bias_len);
   if (softcap < 0.0f) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: score cap %g (0: none)", softcap);
@@ -331,12 +367,13 @@ extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_se
     SB_FAIL(SB_ERR_UNSUPPORTED, "sb_attention_f32: head size %d (a multiple of 4 up to 256), %d key/value heads", hd, n_kv_heads);
   const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, n_rows, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
                   chunk, bias_len, scale, softcap, sink, bias};
+  if (n_sms <= 0) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: %d SMs", n_sms);
   // one token's heads fit the 16-row form; a row of a longer stretch sees up to 64 rows' keys loaded once, or 32 where 64
-  // leave SMs without a block (a prompt of 201 tokens: 76 blocks that go through two tiles of keys each, or 304 with one)
-  const long rows = (long)max_new * (n_q_heads / n_kv_heads), blocks = (rows + 63) / 64 * n_kv_heads * n_seqs * 2;
+  // leave SMs idle (a prompt of 201 tokens: 38 tiles of 64 rows, 152 blocks with a tile of keys each, or 304 with half the work)
+  const long rows = (long)max_new * (n_q_heads / n_kv_heads), tiles = (rows + 63) / 64 * n_kv_heads * n_seqs;
 #define SB_F32_FORMS(ND)                                              \
   if (rows <= 16) return launch<1, ND>(p, n_seqs, max_new, stream);   \
-  if (blocks < 148) return launch<2, ND>(p, n_seqs, max_new, stream); \
+  if (2 * tiles < n_sms) return launch<2, ND>(p, n_seqs, max_new, stream); \
   return launch<4, ND>(p, n_seqs, max_new, stream);
   if (hd <= 64) { SB_F32_FORMS(1) }
   if (hd <= 128) { SB_F32_FORMS(2) }

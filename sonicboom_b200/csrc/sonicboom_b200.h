@@ -265,7 +265,8 @@ int sb_attention_plain(const void* q, void* out, int act_dtype, int n_rows, cons
 int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, const int32_t* seq_row0,
                      const int32_t* seq_pos0, const int32_t* page_off, const int32_t* page_ids, int page_size,
                      const float* cache, int n_pages, int n_q_heads, int n_kv_heads, int hd, int window, float scale,
-                     const float* sink, float softcap, int chunk, const float* bias, int bias_len, sb_stream_t stream);
+                     const float* sink, float softcap, int chunk, const float* bias, int bias_len, int n_sms,
+                     sb_stream_t stream);
 
 /* ---- the stream, the feed-forward and mixers with projections of their own kind ----
  * out[r] = x[r] + add[r] + vec (add [rows, width] float32 and vec [width] are optional; out may be

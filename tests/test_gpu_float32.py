@@ -197,3 +197,33 @@ def test_attention_of_a_plans_first_rows():
         for o, kernel in zip(out, ("auto", "plain")):
             ops.attention(q, o[:n], plan, 0, storage, 4, 2, 32, 0, 32 ** -0.5, kernel=kernel)
         assert pm.rel_err(out[0, :n].cpu(), out[1, :n].cpu()) < 16 * 2 ** -24 * 2 and bool(out[0, n:].isnan().all())
+
+
+@pytest.mark.parametrize("hq,hkv,hd", [(12, 2, 128), (3, 1, 64), (2, 1, 256), (16, 16, 32)])
+@pytest.mark.parametrize("kw", [dict(), dict(window=150), dict(chunk=320, softcap=3.0)])
+def test_attention_of_a_row_does_not_depend_on_the_launch(hq, hkv, hd, kw):
+    """One sequence of 1,300 tokens whole (tiles of 64 rows), its rows in portions of one (16 rows) and of 20 (32 rows), and a portion
+    beside other sequences: the same bits."""
+    n, others = 1300, 30
+    cache = Cache([KVNeed(hkv, hd, 0, 0, 0)], [None], 64 * (21 + others * 4), torch.float32, DEV)
+    storage = cache.groups[0].entry_storage(0)
+    storage.copy_(rnd(*storage.shape))
+    seq, slots = cache.open(), [cache.open() for _ in range(others)]
+    cache.reserve(seq, n)
+    for s in slots:
+        cache.reserve(s, 200)
+    q = rnd(n, hq, hd, seed=1)
+
+    def run(entries):
+        plan = StepPlan(cache, [StepEntry(s, [0] * (hi - lo), []) for s, lo, hi in entries], DEV)
+        rows = torch.cat([q[lo:hi] for _, lo, hi in entries]).contiguous()
+        out = torch.empty(len(rows), hq * hd, device=DEV)
+        ops.attention(rows, out, plan, 0, storage, hq, hkv, hd, kw.get("window", 0), hd ** -0.5, softcap=kw.get("softcap", 0.0),
+                      chunk=kw.get("chunk", 0))
+        return out
+
+    whole = run([(seq, 0, n)])
+    for lo, hi in [(0, 1), (63, 83), (511, 512), (512, 532), (777, 1100), (1280, 1300)]:
+        cache.advance(seq, lo)
+        alone, beside = run([(seq, lo, hi)]), run([(slots[0], 0, 7), (seq, lo, hi)] + [(s, 0, 200) for s in slots[1:]])
+        assert torch.equal(alone, whole[lo:hi]) and torch.equal(beside[7:7 + hi - lo], whole[lo:hi]), (lo, hi)
