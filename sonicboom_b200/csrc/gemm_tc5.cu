@@ -39,7 +39,7 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
 constexpr int THREADS = 192;
-// The decode form with 32 or 64 tokens has two groups of four epilogue warps: a warp reaches only
+// The swapped form with 32 tokens and more has two groups of four epilogue warps: a warp reaches only
 // its own quarter of the tensor memory's lanes (weight rows), so the second group takes the
 // second half of the columns (tokens).  With one group the epilogue of the last wave of blocks,
 // beside which nothing else runs, took 5 of the fused gate/up product's 46 microseconds at 64
@@ -660,13 +660,14 @@ tc5_reduce_kernel(const Tc5Params p, int bn) {
 
 // Where the partial sums of feature e of row j lie: those of split s are s * stride values on.  The swapped form's lie
 // by tile, [tile][split][row of bn][128 features], the pair kernel's (bn = 0) [split][row][feature].
-__device__ __forceinline__ const float* partial_sums(const Tc5Params& p, int bn, int j, int e, size_t& stride) {
-  if (bn == 0) {
-    stride = (size_t)p.M * p.N;
-    return p.scratch + (size_t)j * p.N + e;
-  }
+__device__ __forceinline__ const float* swapped_sums(const Tc5Params& p, int bn, int j, int e, size_t& stride) {
   stride = (size_t)bn * BM;
   return p.scratch + (((size_t)(e / BM) * p.k_splits) * bn + j) * BM + e % BM;
+}
+__device__ __forceinline__ const float* partial_sums(const Tc5Params& p, int bn, int j, int e, size_t& stride) {
+  if (bn != 0) return swapped_sums(p, bn, j, e, stride);
+  stride = (size_t)p.M * p.N;
+  return p.scratch + (size_t)j * p.N + e;
 }
 
 // The same sum for a fused q|k|v product, followed by the rotation and the cache write that
@@ -765,7 +766,7 @@ tc5_reduce_rope_kernel(const Tc5Params p, int bn, const SbRopeStore r) {
 }
 
 // The same sum for a row-wise epilogue, followed by the RMSNorm of the finished rows: what a
-// pre-norm block's next product reads.  A cluster of RN_CLUSTER blocks takes one token; a block
+// pre-norm block's next product reads (up to 64 rows, the swapped form's).  A cluster of RN_CLUSTER blocks takes one token; a block
 // adds the partial tiles of its part of the row, writes the float32 result, and the blocks
 // exchange their sums of squares through each other's shared memory, so that the row is neither
 // written and read again for the norm nor waits for another launch.  The sum of squares is added
@@ -822,7 +823,7 @@ tc5_reduce_norm_kernel(const Tc5Params p, int bn, const TW* __restrict__ norm_w,
     if (g >= g1) continue;
     const int e = g * 4;
     size_t stride;
-    const float* base = partial_sums(p, bn, j, e, stride);
+    const float* base = swapped_sums(p, bn, j, e, stride);
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int s = 0; s < p.k_splits; ++s) {
       const float4 t = *reinterpret_cast<const float4*>(base + s * stride);
