@@ -383,8 +383,8 @@ def attention_ref(qkv, pos0, hq, hkv, hd, window, history=None, theta=10000.0, s
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("kernel", ["plain", "auto", "mma", "tma"])
 def test_rotation_cache_and_attention(hq, hkv, hd, dtype, kernel):
-    if dtype == "float32" and kernel != "plain":
-        pytest.skip("float32 has the plain kernel only")
+    if dtype == "float32" and kernel in ("mma", "tma"):
+        pytest.skip("these kernels take bfloat16")
     if kernel == "tma" and hd not in (64, 128):
         pytest.skip("the persistent decode kernel is written for head sizes 64 and 128")
     if kernel == "mma" and hd not in (64, 128):
@@ -415,8 +415,6 @@ def test_rotation_cache_and_attention(hq, hkv, hd, dtype, kernel):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("kernel", ["plain", "auto"])
 def test_partial_rotation_and_no_rotation(dtype, kernel):
-    if dtype == "float32" and kernel == "auto":
-        pytest.skip("float32 has the plain kernel only")
     hq, hkv, hd = 4, 2, 32
     x = torch.randn(9, (hq + 2 * hkv) * hd, generator=torch.Generator().manual_seed(1))
     for rot in (0, 16):
@@ -444,8 +442,6 @@ def standout(n, hq, hkv, hd, key_pos, big=60.0):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("kernel", ["plain", "auto"])
 def test_a_far_key_among_hundreds_is_found(dtype, kernel):
-    if dtype == "float32" and kernel == "auto":
-        pytest.skip("float32 has the plain kernel only")
     hq, hkv, hd, n = 6, 2, 32, 700
     for key_pos in (3, 64, 255, 256, 511, 640):
         cache = make_cache(hkv, hd, 0, DT[dtype])
@@ -462,8 +458,6 @@ def test_a_far_key_among_hundreds_is_found(dtype, kernel):
 @pytest.mark.parametrize("kernel", ["plain", "auto"])
 def test_window_edges(dtype, kernel):
     """Query i sees key j iff i - j < window: the key at i - window + 1 counts, i - window not."""
-    if dtype == "float32" and kernel == "auto":
-        pytest.skip("float32 has the plain kernel only")
     hq, hkv, hd, window = 4, 2, 16, 70
     for n in (71, 135, 200):                              # the last row is the query
         i = n - 1
@@ -489,8 +483,6 @@ def test_window_edges(dtype, kernel):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("kernel", ["plain", "auto"])
 def test_every_sequence_reads_its_own_pages(dtype, kernel):
-    if dtype == "float32" and kernel == "auto":
-        pytest.skip("float32 has the plain kernel only")
     hq, hkv, hd = 4, 1, 16
     cache = make_cache(hkv, hd, 0, DT[dtype], max_tokens=64 * 40)
     # interleave the sequences' growth so that their pages are interleaved in the pool
