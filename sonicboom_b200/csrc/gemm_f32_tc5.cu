@@ -21,7 +21,12 @@
 // loading, splitting, MMAs and draining: 2 us for 32 values of K at 224 tokens, of which the MMAs take 0.7.
 //
 // A value that is not finite, or that rounds to infinity as TF32, makes its sums NaN here (infinity times a lo of 0): a result that is not
-// finite is computed once more term by term in float32, and is then what the plain kernel gives.
+// finite is computed once more term by term in float32, and is then what the plain kernel gives.  So is a result below TC_SMALL:
+// below 2^-112 an operand is off by up to 2^-136, its last bit as TF32, more than the 2^-24 of it that a float32 result may be off
+// (512 terms with operands around 2^-126: 3.0e-4, term by term 4.0e-7).  Over K terms that is at most K 2^-135 times the largest
+// operand: below 2^-24 of a result of TC_SMALL for operands up to 2^41 / K.  What is left are products of operands beyond that
+// with ones below 2^-112, and operands below 2^-136, which count as 0 where nothing else is in the sum.  (Looking for small operands
+// while they are split closes that too, but cost the gate/up product of 201 rows 5 % and the down product 7.)
 #include <cooperative_groups.h>
 #include <float.h>
 
@@ -38,6 +43,8 @@ constexpr int TC_W_BYTES = TC_ROWS * TC_ROW_BYTES;
 constexpr int TC_WARPS = 8, TC_THREADS = 64 + 32 * TC_WARPS;
 constexpr int TC_PITCH = TC_ROWS + 4;                               // of a token's sums in the partial tile
 constexpr int TC_MAX_STAGES = 6, TC_SMEM = 225 * 1024;
+
+constexpr float TC_SMALL = 0x1p-70f;
 
 struct TcArgs {
   const float* A;
@@ -243,11 +250,12 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
     for (int s = 0; s < 8; ++s)
       if (s < splits) v += peer[s][r * TC_PITCH + c];
-    if (!(fabsf(v) <= FLT_MAX)) {
-      const float* a = p.A + (size_t)(m0 + r) * p.K;
-      const float* w = p.W + (size_t)(n0 + c) * p.K;
+    const float size = fabsf(v);
+    if (!(size <= FLT_MAX) || (size < TC_SMALL && size > 0.0f)) {
+      const float4* a = reinterpret_cast<const float4*>(p.A + (size_t)(m0 + r) * p.K);
+      const float4* w = reinterpret_cast<const float4*>(p.W + (size_t)(n0 + c) * p.K);
       v = 0.0f;
-      for (int k = 0; k < p.K; ++k) v = fmaf(a[k], w[k], v);
+      for (int k = 0; k < p.K / 4; ++k) v = fmaf(a[k].w, w[k].w, fmaf(a[k].z, w[k].z, fmaf(a[k].y, w[k].y, fmaf(a[k].x, w[k].x, v))));
     }
     return v;
   };

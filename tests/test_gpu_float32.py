@@ -123,6 +123,31 @@ def test_products_of_split_operands(M, N, K, scale):
     assert ops.tc5_status() == 0
 
 
+# operands scaled by powers of two down to the subnormal range: rows, weights; rows of ordinary size, of zeros and of tiny values side
+# by side (None)
+@pytest.mark.parametrize("ea,ew", [(-60, 0), (-72, 0), (-100, 0), (-110, 0), (-116, 0), (-126, 0), (-130, 0), (-70, -70), (-110, 20), (0, -120),
+                                   (20, -126), (None, 0), (None, -60)])
+@pytest.mark.parametrize("M,N,K", [(40, 144, 512), (225, 136, 1028)])
+def test_split_operands_of_any_size(M, N, K, ea, ew):
+    """As close to 64 bits as the plain kernel, row by row."""
+    a, w = rnd(M, K), rnd(N, K, seed=1).mul_(2.0 ** ew)
+    if ea is None:
+        sizes = torch.tensor([0.0, 2.0 ** -120, 1.0, 2.0 ** -50, 0.0, 2.0 ** -90, 2.0 ** 30], device=DEV)
+        a *= sizes[torch.arange(M, device=DEV) % len(sizes)][:, None]
+    else:
+        a *= 2.0 ** (ea / 2)
+        a *= 2.0 ** (ea - ea / 2)
+    want = a.double() @ w.double().T
+    err = []
+    for kernel in ("auto", "plain"):
+        out = torch.full((M, N), float("nan"), device=DEV)
+        ops.linear(a, w, out, kernel=kernel)
+        err.append((out.double() - want).norm(dim=1))
+    # 2^-22 of an operand, a few 2^-24 of the sums, half a unit of the subnormal range for each
+    assert bool((err[0] <= 1.3 * err[1] + 2 ** -22 * want.norm(dim=1) + N ** 0.5 * 2.0 ** -149).all())
+    assert ops.tc5_status() == 0
+
+
 def test_split_operands_let_what_is_not_finite_through():
     """Infinities, NaN of every pattern, values that round to infinity as TF32 and sums that overflow: as term by term."""
     M, N, K = 96, 144, 512
