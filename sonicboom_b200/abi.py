@@ -61,7 +61,7 @@ CORE = {
     "sb_mlstm_scan": ("i", "pippiiippiffipipps"),
     "sb_mlstm_out": ("i", "pppiiiipifpis"),
     "sb_attention_plain": ("i", "ppiippppipiiiiifpfipis"),
-    "sb_attention_f32": ("i", "ppiiippppipiiiiifpfipiis"),
+    "sb_attention_f32": ("i", "ppiiiippppipiiiiifpfipiis"),
     "sb_stream_add": ("i", "pppiiippifpipps"),
     "sb_polynorm": ("i", "piipifpis"),
     "sb_attn_prep": ("i", "piiiiiiiiiiiippppiiffppppipipiis"),

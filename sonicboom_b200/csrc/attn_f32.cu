@@ -5,17 +5,19 @@
 // forms: 16 rows (a decode step: one token's heads), 64 rows (prompts), 32 rows (prompts whose 64-row tiles leave SMs idle).
 // Keys come in tiles of 64 at absolute positions.  Tile t belongs to part t % 8; every part has a running softmax of its own
 // and the eight are merged in order, in every form, so a row's bits depend on its own keys and position alone: not on the
-// form, and so not on the cut or on what else the step holds.  A cluster of blocks shares the parts out (8 blocks for
-// 16 rows, where a step has few blocks and the sequence is long; else 4, each with two parts one after the other) and merges
-// them through distributed shared memory; no workspace is needed.
+// form, and so not on the cut or on what else the step holds.  A cluster of blocks shares the parts out and merges
+// them through distributed shared memory; no workspace is needed.  Its size, which changes no bit either, is the number of
+// key tiles that the step's longest sequence has, up to 8 blocks for 16 rows, where a step has few blocks and the sequence is
+// long, else up to 4, with two parts each, one after the other; a row that sees one tile of keys takes one block, and the others leave.
 //
 // What attn_plain.cu says about masks, caps, biases and sinks holds here; that kernel (a block per row and head, a
-// warp per key) stays for head sizes this one does not take.  12/2 heads of 128: three single tokens at 100 to 400 keys
-// took 324 us there, bound by a block's dependent steps over its keys, and 16 here (19 when a tile's loads came one after
-// the other); a prompt of 201 tokens 183 and 50 (67 in 64-row tiles).  The eight parts in every form, where each form had as many
-// as blocks and so bits of its own, cost 201 tokens 40.0 to 41.3 us (the kernel alone), 4,000 tokens 2,465 to 2,502.
+// warp per key) stays for head sizes this one does not take.  The kernel alone, us, there / here, 12/2 heads of 128: one token at 20, 64
+// keys 16.4 / 7.3, 36.4 / 12.6; 256 tokens at 30 keys 73.6 / 21.0 (225 with clusters of eight whatever the length); three at 100 to 400
+// 324 / 13.9; prompts of 10 in 64 sequences 69 / 17.8, of 201 183 / 24 (40 while blocks without a tile of keys stayed to the end), of
+// 4,000 2,467.  8/8 heads of 256, one row a tile of 16: 256 tokens at 30 keys 105 / 184, 64 at 50 51 / 71, a sequence of 64 47 / 19.5.
 #include <cooperative_groups.h>
 #include <math.h>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -33,7 +35,7 @@ struct F32Attn {
   const int32_t* page_off;
   const int32_t* page_ids;
   const float* cache;
-  int n_rows, page_size, n_pages, n_q_heads, n_kv_heads, hd, window, chunk, bias_len;
+  int n_rows, max_len, page_size, n_pages, n_q_heads, n_kv_heads, hd, window, chunk, bias_len;
   float scale, softcap;
   const float* sink;
   const float* bias;
@@ -44,7 +46,7 @@ struct F32Attn {
 template <int TQ, int ND>
 struct Form {
   static constexpr int QB = 16 * TQ;
-  static constexpr int SPLITS = TQ == 1 ? 8 : 4, MINE = PARTS / SPLITS;       // blocks of a cluster, parts of a block
+  static constexpr int MOST = TQ == 1 ? 8 : 4, MINE = PARTS / MOST;           // blocks of a cluster, parts of a block
   static int floats(int hd) {      // queries, keys (later probabilities), values, maximum and sum, their merge
     const int kp = KEYS * (hd + 4), pp = QB * (KEYS + 4), op = QB * hd;
     const int first = kp > pp ? kp : pp;
@@ -94,10 +96,16 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
   const int first_pos = pos0 + pair0 / group, last_pos = pos0 + (min(pair0 + QB, pairs) - 1) / group;
   const int k_lo = max(p.window > 0 ? max(0, first_pos - p.window + 1) : 0,
                        p.chunk > 0 ? max(first_pos, 0) / p.chunk * p.chunk : 0);
-  const int k_hi = min(last_pos, held - 1);
+  const int k_hi = min(min(last_pos, held - 1), p.max_len - 1);
+  // Tile t_lo + i is block (t_lo + i) % splits's; `mine` is this block's first i.  Fewer blocks than MOST have no second part: there
+  // are no more tiles than blocks.
+  const int t_lo = k_lo / KEYS, t_hi = k_hi >= k_lo ? k_hi / KEYS : -1;
+  const int splits = gridDim.z, used = min(max(t_hi - t_lo + 1, 1), splits), mine = (rank - t_lo) & (splits - 1);
+  if (used == 1 && mine != 0) return;                   // a block alone meets nobody
 
   sb_pdl_wait();
   const int quads = hd / 4;
+  if (mine < used)
   for (int i = tid; i < QB * quads; i += THREADS) {
     const int r = i / quads, c = i % quads, pair = pair0 + r;
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -108,18 +116,15 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 
   float m[TQ], l[TQ];
   float4 acc[TQ][ND];
-  const int t_lo = k_lo / KEYS, t_hi = k_hi >= k_lo ? k_hi / KEYS : -1;
-  // the first tile of a part (none: beyond t_hi)
-  auto first_tile = [&](int part) { return t_lo + (part - t_lo % PARTS + PARTS) % PARTS; };
-  // This block's parts, rank and rank + SPLITS, the empty ones left out.  The first of two is set aside in local memory (an index that
-  // the compiler does not know): kept in registers, or in a copy of the loop each, it cost 4,000 tokens 13 and 10 % more.
-  const bool two = F::MINE > 1 && first_tile(rank) <= t_hi && first_tile(rank + F::SPLITS) <= t_hi;
+  // The block's parts.  The first of two is set aside in local memory (an index that the compiler does not know): kept in
+  // registers, or in a copy of the loop each, it cost 4,000 tokens 13 and 10 % more.
+  const bool two = F::MINE > 1 && splits == F::MOST && t_lo + mine + splits <= t_hi;
   float4 kept[F::MINE][TQ][ND];
   float2 kept_stat[F::MINE][TQ];
   int last = 0;                                         // the part whose sums are in registers
 #pragma unroll 1
   for (int j = 0; j < F::MINE; ++j) {
-  if (j > 0 && first_tile(rank + j * F::SPLITS) > t_hi) break;
+  if (j > 0 && !two) break;
   last = j;
 #pragma unroll
   for (int i = 0; i < TQ; ++i) {
@@ -128,20 +133,21 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 #pragma unroll
     for (int d = 0; d < ND; ++d) acc[i][d] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
-  for (int t = first_tile(rank + j * F::SPLITS); t <= t_hi; t += PARTS) {
-    const int base = t * KEYS;
+  for (int t = t_lo + mine + j * splits; t <= t_hi; t += PARTS) {
+    const int base = t * KEYS, n_keys = min(KEYS, k_hi - base + 1);     // the rest of the tile is neither loaded nor looked at
+    const int load = (n_keys + 15) / 16 * 16 * quads;
     __syncthreads();                                    // the tile before this one has been read
     if (tid == 0) bad_values = 0;
     __syncthreads();
     bool bad = false;
     // LOADS keys' and values' 16 bytes a thread at once: one after the other they were most of a decode step's time
-    for (int i0 = tid; i0 < KEYS * quads; i0 += LOADS * THREADS) {
+    for (int i0 = tid; i0 < load; i0 += LOADS * THREADS) {
       float4 kv[LOADS], vv[LOADS];
       int page[LOADS];
 #pragma unroll
       for (int u = 0; u < LOADS; ++u) {
         const int i = i0 + u * THREADS, j = base + i / quads;
-        page[u] = i < KEYS * quads && j >= k_lo && j <= k_hi ? pages[j / p.page_size] : -1;
+        page[u] = i < load && j >= k_lo && j <= k_hi ? pages[j / p.page_size] : -1;
       }
 #pragma unroll
       for (int u = 0; u < LOADS; ++u) {
@@ -156,7 +162,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 #pragma unroll
       for (int u = 0; u < LOADS; ++u) {
         const int i = i0 + u * THREADS, r = i / quads, c = i % quads;
-        if (i >= KEYS * quads) continue;
+        if (i >= load) continue;
         *reinterpret_cast<float4*>(ks + r * kpitch + 4 * c) = kv[u];
         *reinterpret_cast<float4*>(vs + r * hd + 4 * c) = vv[u];
         const float s = fabsf(vv[u].x) + fabsf(vv[u].y) + fabsf(vv[u].z) + fabsf(vv[u].w);
@@ -168,22 +174,27 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 
     // scores: rows ty * TQ + i, keys tx + 16 j
     float s[TQ][4] = {};
-    for (int c = 0; c < quads; ++c) {
-      float4 kq[4];
+    auto scores = [&](auto columns) {                   // of the first 16 `columns` keys
+      constexpr int NJ = decltype(columns)::value;
+      for (int c = 0; c < quads; ++c) {
+        float4 kq[NJ];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) kq[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * kpitch + 4 * c);
+        for (int j = 0; j < NJ; ++j) kq[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * kpitch + 4 * c);
 #pragma unroll
-      for (int i = 0; i < TQ; ++i) {
-        const float4 qv = *reinterpret_cast<const float4*>(qs + (ty * TQ + i) * hd + 4 * c);
+        for (int i = 0; i < TQ; ++i) {
+          const float4 qv = *reinterpret_cast<const float4*>(qs + (ty * TQ + i) * hd + 4 * c);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          s[i][j] = fmaf(qv.x, kq[j].x, s[i][j]);
-          s[i][j] = fmaf(qv.y, kq[j].y, s[i][j]);
-          s[i][j] = fmaf(qv.z, kq[j].z, s[i][j]);
-          s[i][j] = fmaf(qv.w, kq[j].w, s[i][j]);
+          for (int j = 0; j < NJ; ++j) {
+            s[i][j] = fmaf(qv.x, kq[j].x, s[i][j]);
+            s[i][j] = fmaf(qv.y, kq[j].y, s[i][j]);
+            s[i][j] = fmaf(qv.z, kq[j].z, s[i][j]);
+            s[i][j] = fmaf(qv.w, kq[j].w, s[i][j]);
+          }
         }
       }
-    }
+    };
+    if (TQ == 1 && n_keys <= 32) scores(std::integral_constant<int, 2>());
+    else scores(std::integral_constant<int, 4>());
     __syncthreads();                                    // the keys have been read: the probabilities take their place
 #pragma unroll
     for (int i = 0; i < TQ; ++i) {
@@ -225,7 +236,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
     // output: rows ty * TQ + i, dimensions tx * 4 + 64 d.  A value that is not finite must not reach rows that do not
     // see its key, so a tile that holds one takes the keys one by one.
     const bool check = bad_values != 0;
-    for (int k4 = 0; k4 < KEYS; k4 += 4) {
+    for (int k4 = 0; k4 < n_keys; k4 += 4) {
       float4 pr[TQ];
 #pragma unroll
       for (int i = 0; i < TQ; ++i) pr[i] = *reinterpret_cast<const float4*>(ps + (ty * TQ + i) * ppitch + k4);
@@ -275,11 +286,16 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
       if (tx == 0) *reinterpret_cast<float2*>(stat + 2 * r) = stat_of(i);
     }
   };
-  leave(last, acc, [&](int i) { return make_float2(m[i], l[i]); });
+  if (mine < used) leave(last, acc, [&](int i) { return make_float2(m[i], l[i]); });
   if (two) leave(0, kept[last - 1], [&](int i) { return kept_stat[last - 1][i]; });
-  // part s is the (s / SPLITS)-th of block s % SPLITS
-  cluster.sync();
-  for (int r = rank * (QB / F::SPLITS) + ty; r < (rank + 1) * (QB / F::SPLITS); r += 16) {
+  // part s begins with tile t_lo + i and is the (i / splits)-th of block s % splits (i beyond the last tile: the part is empty)
+  auto begins = [&](int s) { return (s - t_lo) & (PARTS - 1); };
+  auto holds = [&](int s) { return t_lo + begins(s) <= t_hi; };
+  auto row_of = [&](int s, int r) { return (begins(s) >= splits ? QB : 0) + r; };
+  if (used > 1) cluster.sync();
+  else __syncthreads();
+  const int share = (QB + used - 1) / used;
+  for (int r = mine * share + ty; r < min((mine + 1) * share, QB); r += 16) {
     const int pair = pair0 + r;
     if (pair >= pairs) continue;
     const int h = g * group + pair % group, at = pos0 + pair / group;
@@ -287,8 +303,8 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
     float2 st[PARTS];
 #pragma unroll
     for (int s = 0; s < PARTS; ++s)
-      st[s] = first_tile(s) <= t_hi ? *reinterpret_cast<const float2*>(cluster.map_shared_rank(stat, s % F::SPLITS) + 2 * (s / F::SPLITS * QB + r))
-                                    : make_float2(-INFINITY, 0.0f);
+      st[s] = holds(s) ? *reinterpret_cast<const float2*>(cluster.map_shared_rank(stat, s & (splits - 1)) + 2 * row_of(s, r))
+                       : make_float2(-INFINITY, 0.0f);
     float m_all = p.sink ? p.sink[h] : -INFINITY, total = 0.0f;
 #pragma unroll
     for (int s = 0; s < PARTS; ++s) m_all = fmaxf(m_all, st[s].x);
@@ -310,8 +326,8 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
 #pragma unroll
         for (int s = 0; s < PARTS; ++s) {
           float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (first_tile(s) <= t_hi)
-            v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(os, s % F::SPLITS) + (s / F::SPLITS * QB + r) * hd + at_d);
+          if (holds(s))
+            v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(os, s & (splits - 1)) + row_of(s, r) * hd + at_d);
           o.x = fmaf(v.x, f[s], o.x); o.y = fmaf(v.y, f[s], o.y); o.z = fmaf(v.z, f[s], o.z); o.w = fmaf(v.w, f[s], o.w);
         }
         o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
@@ -319,7 +335,7 @@ attn_f32_kernel(F32Attn p, int tiles_per_seq) {
       *reinterpret_cast<float4*>(to + at_d) = o;
     }
   }
-  cluster.sync();                                       // nobody's sums go while another block reads them
+  if (used > 1) cluster.sync();                         // nobody's sums go while another block reads them
 }
 
 template <int TQ, int ND>
@@ -332,14 +348,17 @@ int launch(const F32Attn& p, int n_seqs, int max_new, cudaStream_t stream) {
                                            F::floats(64 * ND) * (int)sizeof(float)))
     SB_FAIL(SB_ERR_CUDA, "sb_attention_f32: %s", cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)n_seqs * (unsigned)tiles, p.n_kv_heads, F::SPLITS);
+  const int key_tiles = (p.max_len + KEYS - 1) / KEYS;
+  int splits = 1;
+  while (splits < key_tiles && splits < F::MOST) splits *= 2;
+  cfg.gridDim = dim3((unsigned)n_seqs * (unsigned)tiles, p.n_kv_heads, splits);
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = F::SPLITS;
+  attr[0].val.clusterDim.z = splits;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
@@ -353,7 +372,7 @@ int launch(const F32Attn& p, int n_seqs, int max_new, cudaStream_t stream) {
 
 int sb_check_attention_args(const char* who, int n_rows, int n_q_heads, int n_kv_heads, int hd, int window, int page_size);
 
-extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, const int32_t* seq_row0,
+extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, int max_len, const int32_t* seq_row0,
                                 const int32_t* seq_pos0, const int32_t* page_off, const int32_t* page_ids, int page_size,
                                 const float* cache, int n_pages, int n_q_heads, int n_kv_heads, int hd, int window,
                                 float scale, const float* sink, float softcap, int chunk, const float* bias, int bias_len,
@@ -362,10 +381,11 @@ extern "C" int sb_attention_f32(const float* q, float* out, int n_rows, int n_se
     SB_FAIL(SB_ERR_ARG, "sb_attention_f32: chunk %d, a distance bias of %d entries", chunk, bias_len);
   if (softcap < 0.0f) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: score cap %g (0: none)", softcap);
   if (int rc = sb_check_attention_args("sb_attention_f32", n_rows, n_q_heads, n_kv_heads, hd, window, page_size)) return rc;
-  if (n_seqs <= 0 || max_new <= 0) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: %d sequences, at most %d new rows", n_seqs, max_new);
+  if (n_seqs <= 0 || max_new <= 0 || max_len <= 0)
+    SB_FAIL(SB_ERR_ARG, "sb_attention_f32: %d sequences, at most %d new rows and %d positions", n_seqs, max_new, max_len);
   if (hd % 4 || hd > 256 || n_kv_heads > 65535)
     SB_FAIL(SB_ERR_UNSUPPORTED, "sb_attention_f32: head size %d (a multiple of 4 up to 256), %d key/value heads", hd, n_kv_heads);
-  const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, n_rows, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
+  const F32Attn p{q, out, seq_row0, seq_pos0, page_off, page_ids, cache, n_rows, max_len, page_size, n_pages, n_q_heads, n_kv_heads, hd, window,
                   chunk, bias_len, scale, softcap, sink, bias};
   if (n_sms <= 0) SB_FAIL(SB_ERR_ARG, "sb_attention_f32: %d SMs", n_sms);
   // one token's heads fit the 16-row form; a row of a longer stretch sees up to 64 rows' keys loaded once, or 32 where 64

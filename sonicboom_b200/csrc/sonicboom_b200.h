@@ -260,9 +260,9 @@ int sb_attention_plain(const void* q, void* out, int act_dtype, int n_rows, cons
                        sb_stream_t stream);
 
 /* The same attention for float32 rows over a float32 cache of n_pages pages, by tiles of query rows: the step's
- * sequences own the rows seq_row0[s] ... seq_row0[s + 1] - 1 at positions from seq_pos0[s] on, at most max_new each;
- * head sizes that are multiples of 4 up to 256. */
-int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, const int32_t* seq_row0,
+ * sequences own the rows seq_row0[s] ... seq_row0[s + 1] - 1 at positions from seq_pos0[s] on, at most max_new each, below
+ * max_len; head sizes that are multiples of 4 up to 256. */
+int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, int max_len, const int32_t* seq_row0,
                      const int32_t* seq_pos0, const int32_t* page_off, const int32_t* page_ids, int page_size,
                      const float* cache, int n_pages, int n_q_heads, int n_kv_heads, int hd, int window, float scale,
                      const float* sink, float softcap, int chunk, const float* bias, int bias_len, int n_sms,

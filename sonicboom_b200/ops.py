@@ -617,7 +617,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, plan, group_index: int, cache:
     elif (q.dtype == out.dtype == cache.dtype == torch.float32 and kernel != "plain" and head_dim % 4 == 0 and head_dim <= 256
           and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0):
         _check(lib().sb_attention_f32(
-            _ptr(q), _ptr(out), n, plan.n_seqs, plan.max_new, _i32(plan.seq_row0, "seq_row0"),
+            _ptr(q), _ptr(out), n, plan.n_seqs, plan.max_new, plan.max_len, _i32(plan.seq_row0, "seq_row0"),
             _i32(plan.seq_pos0, "seq_pos0"), _i32(g.page_off, "page_off"), _i32(g.page_ids, "page_ids"), g.page_size,
             _ptr(cache), cache.shape[0], n_q_heads, n_kv_heads, head_dim, window, ctypes.c_float(scale), _ptr(sink),
             ctypes.c_float(softcap), int(chunk), _ptr(bias.values) if bias is not None else None, bias_len, _sm_count(q.device),

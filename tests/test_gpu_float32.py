@@ -199,11 +199,13 @@ def attention_both(hq, hkv, hd, held, new, window=0, chunk=0, sink=None, softcap
     return outs
 
 
-# one token's heads in the 16-row form (and one head more than fits), stretches in the 64-row form; head sizes below,
-# at and over each width; lengths around a tile of 64 keys and around all of a cluster's tiles.  Stretches take the 32-row form while
-# 64 rows a block would leave SMs without one
+# one token's heads in the 16-row form (and one head more than fits), stretches in the 64- and 32-row forms; head sizes below,
+# at and over each width; lengths around a tile of 64 keys and around all of a cluster's tiles, and longest lengths that make clusters
+# of one, two and four blocks
 @pytest.mark.parametrize("hq,hkv,hd", [(4, 2, 16), (12, 2, 128), (17, 1, 36), (16, 1, 64), (3, 3, 100), (2, 1, 256)])
-@pytest.mark.parametrize("held,new", [([0, 63, 64, 511, 513, 1100], [1] * 6), ([0, 5, 200], [63, 130, 17]), ([0], [201])])
+@pytest.mark.parametrize("held,new", [([0, 63, 64, 511, 513, 1100], [1] * 6), ([0, 5, 200], [63, 130, 17]), ([0], [201]),
+                                      ([0, 20, 63], [1] * 3), ([0, 64, 127], [1] * 3), ([3, 190, 255], [1] * 3), ([0, 10], [64, 30]),
+                                      ([40, 0], [60, 128]), ([0] * 40, [200] * 40)])
 def test_attention(hq, hkv, hd, held, new):
     sink = rnd(hq, seed=5)
     bias = ops.DistanceBias(rnd(hq, 33, seed=6))
