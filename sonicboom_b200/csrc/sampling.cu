@@ -5,8 +5,8 @@
 // a value that at least CANDIDATES of the row reach, and only those that reach it (about 400 of a row of
 // random logits) are collected in the first block and sorted.  Rows where more than MAX_LIST reach it (many equal logits) go through a
 // radix select in the first block instead, with the same result.  Measured at a vocabulary of 152,064 on one B200, us: 8
-// rows sampled at temperature 0.7 23.5, 64 rows 54 (one block per row, five passes over it for a radix select and the
-// filters by one thread took 382 and 393); one greedy row 5.4 (12).
+// rows sampled at temperature 0.7 23.3, 64 rows 36 (one block per row, five passes over it for a radix select and the
+// filters by one thread took 342 and 389); greedy, one row 4.0, 64 rows 7.2, 256 rows 31 (7.0, 10.0 and 30).
 //
 // The order of stages is the reference's (capi/include/sonicboom/capi.h:629-645,
 // core/src/nn/sampling.cpp:157-203, 257-352):
@@ -31,11 +31,10 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr int THREADS = 512;
-constexpr int CLUSTER = 8;           // blocks that share a row
+constexpr int MOST = 8;              // blocks that share a row, at most
 constexpr int CANDIDATES = 256;      // core/include/sonicboom/nn/sampling.h:68
 constexpr float LOGIT_WINDOW = 30.0f;  // core/include/sonicboom/nn/sampling.h:61
 constexpr int MAX_HISTORY = 1024;    // the reference's device penalty window (capi.cpp:2711-2715)
-constexpr int RANK_SHARE = CANDIDATES / CLUSTER;
 constexpr int MAX_LIST = 2048;       // values collected for the sort
 
 __device__ __forceinline__ uint32_t order_key(float z) {
@@ -147,9 +146,12 @@ __device__ void select_by_radix(const float* lg, int vocab, float T, unsigned lo
   }
 }
 
+template <int CLUSTER>
 __global__ void __launch_bounds__(THREADS, 2)
 sample_kernel(float* logits, int vocab, const SbSampleParams* params, const int32_t* history,
               int history_stride, const int32_t* fed_pos, int32_t* out_tokens) {
+  constexpr int RANK_SHARE = CANDIDATES / CLUSTER;
+  static_assert(RANK_SHARE <= THREADS && CLUSTER <= MOST, "a block has a maximum a thread");
   __shared__ int32_t h_tok[MAX_HISTORY];
   __shared__ float h_old[MAX_HISTORY];
   __shared__ uint32_t hist[256];
@@ -208,10 +210,30 @@ sample_kernel(float* logits, int vocab, const SbSampleParams* params, const int3
 
   int result = -1;
   if (!(p.temperature > 0.0f)) {
-    // 2. greedy (the two zeros are equal; NaN loses against everything)
+    // 2. greedy (the two zeros are equal; NaN loses against everything): the group of eight values that holds the thread's
+    // largest first, then its first place in the group
+    constexpr int STEP = CLUSTER * THREADS, GROUP = 8;
+    float top = -INFINITY;
+    int group = -1;
+    int at = first;
+    for (; at + (GROUP - 1) * STEP < vocab; at += GROUP * STEP) {
+      float v[GROUP], largest;
+#pragma unroll
+      for (int j = 0; j < GROUP; ++j) v[j] = lg[at + j * STEP];
+      largest = v[0];
+#pragma unroll
+      for (int j = 1; j < GROUP; ++j) largest = fmaxf(largest, v[j]);        // passes over NaN
+      if (largest > top) { top = largest; group = at; }
+    }
+    for (; at < vocab; at += STEP)
+      if (lg[at] > top) { top = lg[at]; group = at; }
     unsigned long long best = 0ull;
-#pragma unroll 8
-    for (int i = first; i < vocab; i += CLUSTER * THREADS) best = max(best, key_and_id(order_key(lg[i] + 0.0f), i));
+    if (group >= 0) {
+      while (lg[group] != top) group += STEP;
+      best = key_and_id(order_key(top + 0.0f), group);
+    } else {                                          // nothing above minus infinity
+      for (int i = first; i < vocab; i += STEP) best = max(best, key_and_id(order_key(lg[i]), i));
+    }
     best = block_max(best, red);
     if (tid == 0) *cluster.map_shared_rank(&best_of[rank], 0) = best;
     cluster.sync();
@@ -376,20 +398,32 @@ extern "C" int sb_sample(float* logits, int n_rows, int vocab, const void* param
   if (history_stride < 0 || history_stride > MAX_HISTORY)
     SB_FAIL(SB_ERR_UNSUPPORTED, "sb_sample: a penalty window of %d tokens is above the cap of %d",
             history_stride, MAX_HISTORY);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)n_rows * CLUSTER);
-  cfg.blockDim = dim3(THREADS);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CLUSTER;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = (sb_pdl_enabled() & SB_K_OTHER) ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, sample_kernel, logits, vocab, (const SbSampleParams*)params, history, history_stride, fed_pos,
-                     out_tokens);
+  auto launch = [&](auto* kernel, unsigned cluster) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n_rows * cluster);
+    cfg.blockDim = dim3(THREADS);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = (sb_pdl_enabled() & SB_K_OTHER) ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, logits, vocab, (const SbSampleParams*)params, history, history_stride, fed_pos, out_tokens);
+  };
+  // Blocks a row: eight, while all rows' blocks run at once (two fit an SM) and have 4,096 values each.  A vocabulary of 152,064,
+  // greedy / sampled, us, with eight blocks and with the rule's: 64 rows 14.5 / 53.8 and 7.2 / 36.3, 128 rows 31.4 / 93.1 and 11.6 / 64.7, 256 rows
+  // 76.5 / 193 and 30.9 / 192; of 1,000, 32 rows 3.1 / 16.5 and 2.6 / 11.5.
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 0;
+  int cluster = MOST;
+  while (cluster > 1 && ((long)n_rows * cluster > 2 * sms || vocab < 4096 * cluster)) cluster /= 2;
+  if (cluster == 8) launch(sample_kernel<8>, 8);
+  else if (cluster == 4) launch(sample_kernel<4>, 4);
+  else if (cluster == 2) launch(sample_kernel<2>, 2);
+  else launch(sample_kernel<1>, 1);
   SB_CHECK_LAUNCH("sb_sample");
   return SB_OK;
 }

@@ -33,7 +33,7 @@ def rows(vocab):
     return x.to(DEV)
 
 
-# one value, less than a warp, one more than the candidates, more than the list but less than a pass of the cluster, more
+# one value, less than a warp, one more than the candidates, more than the list, up to here in one block; in two blocks; in eight
 @pytest.mark.parametrize("vocab", [1, 31, 257, 3000, 9001, 40000])
 def test_tokens_of_every_kind_of_row(vocab):
     sampler, x = Sampler(DEV), rows(vocab)
@@ -47,6 +47,17 @@ def test_tokens_of_every_kind_of_row(vocab):
         got = sampler.sample(x, [s] * len(x), [11 + i for i in range(len(x))], history)
         assert got == [plain(r, s, 11 + i, history[i]) for i, r in enumerate(x)], s
         assert torch.equal(x.view(torch.int32), kept.view(torch.int32))        # the row is as it was
+
+
+@pytest.mark.parametrize("n", [42, 90, 180])
+def test_tokens_of_many_rows(n):
+    """Rows whose blocks would not all run at once are shared by four, two or one: the tokens of the same rows with eight."""
+    sampler, x = Sampler(DEV), rows(33001)
+    x[4] = 0.0
+    many = x.repeat(n // 6, 1)
+    for s in (Sampling().checked(), Sampling(temperature=0.7, seed=3).checked(), Sampling(temperature=0.9, seed=5, top_p=0.8, repeat_penalty=1.2).checked()):
+        few = sampler.sample(x, [s] * 6, [11 + i for i in range(6)], [[7, 3]] * 6)
+        assert sampler.sample(many, [s] * n, [11 + i % 6 for i in range(n)], [[7, 3]] * n) == few * (n // 6), s
 
 
 def test_rows_that_are_not_finite():
