@@ -43,6 +43,7 @@ CORE = {
     "sb_gemm_tc5": ("i", _GEMM[:-1] + "pziis"),
     "sb_gemm_tc5_ex": ("i", _GEMM[:-1] + "pziips"),
     "sb_gemm_tc5_scratch_bytes": ("z", "iiii"),
+    "sb_gemm_tc5_swapped": ("i", "iiiii"),
     "sb_gemm_tc5_fuses_norm": ("i", "iiiiiii"),
     "sb_gemm_tc5_fuses_rope": ("i", "iiiiiiiii"),
     "sb_tc5_status": ("i", ""),

@@ -14,8 +14,8 @@
 //            rows it is a persistent kernel (further down), from 129 rows on one on pairs of SMs
 //            (gemm_tc5_pair.cuh); their epilogue keeps a thread's row and writes 16 bytes at a
 //            time along it (store_chunk_rowwise);
-//   swapped  A = weights (128 weight rows per tile), B = activations (up to 128 rows): the
-//            decode and short-prompt product, which is bound by reading the weights once.  K may be split over
+//   swapped  A = weights (128 weight rows per tile), B = activations (up to 64 rows, and where
+//            swapped_form says so up to 128): the decode and short-prompt product, which is bound by reading the weights once.  K may be split over
 //            several blocks; their partial tiles go to scratch memory and a second kernel adds
 //            them in split order and runs the epilogue, so the sum's order is fixed.  That
 //            second kernel can also apply the RMSNorm that follows the product
@@ -1128,6 +1128,15 @@ int pair_splits(int M, int N, int K, int clusters);
 // single SMs, and norm and rotation were kernels of their own: a prompt of 97 tokens 5.62 ms, now 4.07 (15, 15 and 27 us,
 // 63 us).
 constexpr int SWAPPED_ROWS = 128;
+int choose_splits(int M, int N, int K, int n_sms);
+// Whether a product takes the swapped form.  From 65 rows on: where K is split, and the gated activation where its tiles are one wave
+// (two blocks an SM), whose epilogue writes an eighth of what a float32 product's does.  Without a split, 97 rows, us, here / in the many-rows form:
+// gated 37888 x 3584 53.2 / 57.6, 17920 x 1536 18.5 / 21.1, 4096 x 520 11.5 / 15.1, but 55296 x 5120 110.8 / 100.4; float32 rows 152064 x 3584 228 / 190,
+// 32768 x 2048 32.8 / 29.5, 17920 x 1536 18.2 / 18.2, 4096 x 520 11.5 / 9.5.
+bool swapped_form(int M, int N, int K, int n_sms, int epilogue) {
+  if (M <= 64 || M > SWAPPED_ROWS) return M <= 64;
+  return choose_splits(M, N, K, n_sms) > 1 || (epilogue == SB_EPI_SWIGLU && (N + BM - 1) / BM <= 2 * n_sms);
+}
 // Whether the many-rows product runs on pairs of SMs.
 bool pair_form(int M, int N, int n_sms) { return M > BM && N >= 192 && n_sms > 1 && pair_enabled(); }
 // K splits of the pair kernel.  When even 256-column tiles leave at least half of the pairs of
@@ -1164,11 +1173,15 @@ extern "C" void sb_gemm_tc5_pairs(int mode) { g_pair_mode = mode; }
 // the width is chosen by the sizes again.
 extern "C" void sb_gemm_tc5_force_width(int bn) { g_forced_bn = valid_bn(bn); }
 
+extern "C" int sb_gemm_tc5_swapped(int M, int N, int K, int n_sms, int epilogue) {
+  return M > 0 && N > 0 && K > 0 && swapped_form(M, N, K, n_sms, epilogue) ? 1 : 0;
+}
+
 // The tile width the product of these sizes runs with in its many-rows form (for tests that
-// want every width covered); 0 when that form does not run.
+// want every width covered); 0 when that form does not run.  (At 65 to 128 rows it runs where swapped_form says no.)
 extern "C" int sb_gemm_tc5_tile_width(int M, int N, int n_sms) {
-  if (M <= SWAPPED_ROWS || N < 192 || n_sms <= 0) return 0;
-  if (n_sms > 1 && pair_enabled()) return pair_bn(M, N, n_sms / 2);
+  if (M <= 64 || N < 192 || n_sms <= 0) return 0;
+  if (pair_form(M, N, n_sms)) return pair_bn(M, N, n_sms / 2);
   return persistent_bn(M, N, n_sms);
 }
 
@@ -1367,7 +1380,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
   p.warm_bytes = extras ? sb_warm_bytes(extras->warm, extras->warm_bytes) : 0;
   CUtensorMap ma, mb;
   // form: 0 picks by the number of rows, 1 forces the normal form, 2 the swapped form
-  const bool normal = form == 1 || (form == 0 && M > SWAPPED_ROWS);
+  const bool normal = form == 1 || (form == 0 && !swapped_form(M, N, K, n_sms, epilogue));
   if (form == 2 && M > SWAPPED_ROWS)
     SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: the swapped form takes at most %d rows", SWAPPED_ROWS);
   if (normal && pair_form(M, N, n_sms)) {

@@ -164,6 +164,8 @@ int sb_gemm_tc5_ex(const void* A, int a_dtype, const void* W, int w_dtype, int M
                    void* out, int out_dtype, void* scratch, size_t scratch_bytes, int n_sms,
                    int form, const SbLinearExtras* extras, sb_stream_t stream);
 size_t sb_gemm_tc5_scratch_bytes(int M, int N, int K, int n_sms);
+/* Whether form 0 of sb_gemm_tc5_ex streams the weights past tiles of tokens (the swapped form) at these sizes. */
+int sb_gemm_tc5_swapped(int M, int N, int K, int n_sms, int epilogue);
 int sb_gemm_tc5_fuses_norm(int M, int N, int K, int n_sms, int epilogue, int out_dtype, int form);
 /* Whether sb_gemm_tc5_ex can finish a q|k|v product of these sizes with the rotation and the
  * cache write (the split-K decode form, bfloat16 queries and cache, head sizes in steps of 8). */
