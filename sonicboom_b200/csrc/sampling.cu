@@ -155,7 +155,7 @@ sample_kernel(float* logits, int vocab, const SbSampleParams* params, const int3
   __shared__ int32_t h_tok[MAX_HISTORY];
   __shared__ float h_old[MAX_HISTORY];
   __shared__ uint32_t hist[256];
-  __shared__ unsigned long long cand[MAX_LIST];     // key_and_id: sorts z desc, id asc
+  __shared__ __align__(16) unsigned long long cand[MAX_LIST];     // key_and_id: sorts z desc, id asc
   __shared__ unsigned long long red[32];
   __shared__ double score[CANDIDATES];
   __shared__ unsigned long long best_of[CLUSTER];
@@ -183,25 +183,34 @@ sample_kernel(float* logits, int vocab, const SbSampleParams* params, const int3
   const int win = penal ? min(p.history_len, MAX_HISTORY) : 0;
   if (penal) {
     const int32_t* hrow = history + (size_t)row * history_stride;
-    for (int i = tid; i < win && rank == 0; i += THREADS) {
-      const int32_t t = hrow[i];
-      int count = 0;
-      bool first_one = true;
-      for (int j = 0; j < win; ++j) {
-        if (hrow[j] == t) {
-          ++count;
-          if (j < i) first_one = false;
-        }
+    // The blocks share the window's places out; the first one keeps what they changed.  The window lies in every block's shared
+    // memory (over the candidates' list), filled up with ids that no token has.  (1,024 tokens and 152,064 greedy values, counted by one
+    // block of 512 threads from memory: 8 rows 51 us, 64 rows 98; shared out 15.6 and 33.)
+    int32_t* window = reinterpret_cast<int32_t*>(cand);
+    int32_t* kept_tok = cluster.map_shared_rank(h_tok, 0);
+    float* kept_old = cluster.map_shared_rank(h_old, 0);
+    const int fours = (win + 3) / 4;
+    for (int i = tid; i < 4 * fours; i += THREADS) window[i] = i < win ? hrow[i] : -1;
+    __syncthreads();
+    for (int i = tid * CLUSTER + rank; i < win; i += THREADS * CLUSTER) {
+      const int32_t t = window[i];
+      int count = 0, before = 0;                     // places of the token, those ahead of this one
+      for (int j = 0; j < fours; ++j) {
+        const int4 w = reinterpret_cast<const int4*>(window)[j];
+        const int at = 4 * j;
+        count += (w.x == t) + (w.y == t) + (w.z == t) + (w.w == t);
+        before += (w.x == t && at < i) + (w.y == t && at + 1 < i) + (w.z == t && at + 2 < i) + (w.w == t && at + 3 < i);
       }
-      h_tok[i] = -1;
+      const bool first_one = before == 0;
+      kept_tok[i] = -1;
       if (first_one && t >= 0 && t < vocab) {
         const float old = lg[t];
         float v = old;
         if (p.repeat_penalty != 1.0f)
           v = v > 0.0f ? __fdiv_rn(v, p.repeat_penalty) : __fmul_rn(v, p.repeat_penalty);
         const float adjust = __fmaf_rn(p.frequency_penalty, (float)count, p.presence_penalty);
-        h_tok[i] = t;
-        h_old[i] = old;
+        kept_tok[i] = t;
+        kept_old[i] = old;
         lg[t] = __fsub_rn(v, adjust);
       }
     }

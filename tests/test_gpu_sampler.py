@@ -60,6 +60,21 @@ def test_tokens_of_many_rows(n):
         assert sampler.sample(many, [s] * n, [11 + i % 6 for i in range(n)], [[7, 3]] * n) == few * (n // 6), s
 
 
+@pytest.mark.parametrize("vocab", [9, 900, 40000])
+@pytest.mark.parametrize("win", [1, 3, 130, 1023, 1024])
+def test_penalties_over_windows_of_any_length(vocab, win):
+    """Windows that end inside a group of four, with a token in many places, ids outside the vocabulary, up to the longest."""
+    sampler, x = Sampler(DEV), rows(vocab)[:2]
+    g = torch.Generator().manual_seed(win)
+    history = torch.randint(-2, min(vocab, 700) + 2, (2, win), generator=g).tolist()
+    for s in (Sampling(repeat_penalty=1.3, presence_penalty=0.5, frequency_penalty=0.2, repeat_last_n=1024).checked(),
+              Sampling(temperature=0.8, seed=6, repeat_penalty=1.3, frequency_penalty=0.1, repeat_last_n=1024).checked()):
+        kept = x.clone()
+        got = sampler.sample(x, [s] * 2, [5, 6], history)
+        assert got == [plain(r, s, 5 + i, [t for t in history[i] if 0 <= t < vocab]) for i, r in enumerate(x)], s
+        assert torch.equal(x.view(torch.int32), kept.view(torch.int32))
+
+
 def test_rows_that_are_not_finite():
     x = torch.randn(3, 5000, generator=torch.Generator().manual_seed(1)).to(DEV)
     x[0, 100], x[1, 17], x[2, 4999] = float("nan"), float("inf"), float("nan")
