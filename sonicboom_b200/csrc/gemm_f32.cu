@@ -14,7 +14,12 @@
 //
 // Measured on one B200 inside a step of the 1.5B layers (28 layers: 2048, 1536 and 17920 x 1536, 1536 x 8960): three rows
 // 15.5 us a product on average where the plain kernel took 636 (one row of 151936 x 1536: 140 us, 6.6 TB/s).
-// Error against float64 at K = 8960: 1.2e-7 (the plain kernel's terms one after the other 9e-7).
+// The tile form and the plain kernel, us a product: 64 rows of 512 x 128 10.5 and 20.8, 201 of 4096 x 128 19.0 and 43.0,
+// 1,000 of 1000 x 252 34.8 and 81.7, 2,048 of 4096 x 64 36.6 and 59.9.
+// Error of the rows form against float64 at K = 8960: 1.2e-7, of terms one after the other 9e-7.
+//
+// A row's rounding depends on the number of rows in the launch: its form changes at 17 and 33 rows, and on the tensor cores
+// the blocks that share K with the number of tiles.  Up to 16 rows it does not.
 // Epilogues as in gemm_plain.cu, which computes the same sums in another order and takes the sizes and
 // alignments that these forms do not (K a multiple of 4, rows on 16 bytes).
 #include "common.cuh"
@@ -334,9 +339,12 @@ int run_f32(const F32Args& p, TO* out, int n_sms, cudaStream_t stream) {
 
 }  // namespace
 
-// The tensor-core form (gemm_f32_tc5.cu).  Below this K its splitting of the operands (22 to 23 bits) would be its whole error,
-// 1.4e-7, where 256 float32 terms added one after the other have as much of their own.  From 17 rows on it takes the wide products,
-// whose tiles give every SM work (17 rows of 17920 x 1536: 51 us, streaming the weights 77; of 1536 x 1536 13 and 9).
+// The tensor-core form (gemm_f32_tc5.cu).  Its splitting of the operands (22 to 23 bits) makes an error of 1.4e-7 whatever K is; terms
+// added one after the other have 2.0e-7 at K = 128, 2.9e-7 at 256, and a short K leaves its stages no time to overlap.
+// Streaming the weights / the tensor cores, us at 17 and 28 rows: 2048 x 1536 11.0, 13.9 / 12.2, 12.7; 1536 x 8960 32.9, 47.9 / 36.3, 36.8;
+// 3584 x 3584 32.9, 44.5 / 30.7, 31.4; 6144 x 1536 27.0, 35.2 / 26.9, 27.6; 8192 x 1536 35.5, 45.9 / 27.9, 28.6; 17920 x 1536 73.9, 96.9 /
+// 50.5, 51.2; 37888 x 3584 299, 405 / 209, 211.  8,192 columns is where the tensor cores gain a fifth and more at every count from 17 on
+// (64 tiles of 128 columns); below it the two lie within a tenth of each other at 17 rows, and the line stays at 33.
 constexpr int SPLIT_MIN_K = 256, SPLIT_WIDE_ROWS = 16, SPLIT_WIDE_N = 8192;
 int sb_gemm_f32_tc5(const float* A, const float* W, int M, int N, int K, int epilogue, const void* bias, int bias_dtype,
                     const float* residual, void* out, int out_dtype, int n_sms, cudaStream_t stream);

@@ -6,10 +6,12 @@
 // (`tcgen05.mma kind::tf32`) on one float32 accumulator in tensor memory.  The accumulator covers 32 values of K only;
 // its sums are then added up in registers with float32's own rounding, so that the tensor cores' accumulation, which may
 // not round to nearest, stays a chain of twelve.
-// Error against 64 bits, 2-norm, K = 1,536 and 8,960: 1.0e-7 and 1.6e-7, with the gated activation 3.1e-7; packed FMA in the order of K had 1.6e-7,
-// 5.3e-7 and 7.4e-7, one term after the other 9e-7 at 8,960.
+// Error against 64 bits, 2-norm, here / one term after the other: K = 256 1.4e-7 / 2.9e-7, 1,536 1.5e-7 / 7.0e-7, 8,960 1.8e-7 / 1.7e-6; with positive,
+// long-tailed and gated operands at most a tenth more.  Splitting an operand into two values of a shorter type and leaving
+// out the product of the small halves is a published method (Ootomo and Yokota, "Recovering single precision accuracy from
+// Tensor Cores while surpassing the FP32 theoretical peak performance", 2022).
 //
-// A block computes 128 weight rows (the MMA's rows) x up to 256 tokens.  Warp 0 loads float32 tiles by TMA (128-byte
+// A block computes 128 weight rows (the MMA's rows) x up to 224 tokens.  Warp 0 loads float32 tiles by TMA (128-byte
 // swizzle, 32 values of K), warp 1 issues the MMAs, and eight warps do the arithmetic: they split a stage's
 // values (hi over the loaded value, lo into a buffer of its own; the order of the values does not matter, so the swizzle is left as it is), and while its
 // MMAs run drain the stage before it from the other of two accumulators.  Where the tiles leave SMs idle a cluster of blocks
@@ -17,7 +19,7 @@
 //
 // Bound by the tensor cores (three TF32 products) and, close to it, by shared memory, which the MMAs and the splitting share.
 // 201 rows, us, packed FMA tiles / here: 17920 x 1536 with the gate 327 / 100, 1536 x 8960 278 / 74, 2048 x 1536 48 / 26, 1536 x 1536 55 / 25;
-// a prompt of 201 tokens of the 1.5B model 22.6 to 8.5 ms (the plain kernel: 110).  What is left is a stage's chain of
+// a prompt of 201 tokens of the 1.5B model 22.6 to 8.5 ms, now 7.2 (the plain kernel: 110).  What is left is a stage's chain of
 // loading, splitting, MMAs and draining: 2 us for 32 values of K at 224 tokens, of which the MMAs take 0.7.
 //
 // A value that is not finite, or that rounds to infinity as TF32, makes its sums NaN here (infinity times a lo of 0): a result that is not
@@ -37,6 +39,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
+// 224 tokens: three stages beside the two of lo, and 112 sums a thread; with 256 two stages would be left.
 constexpr int TC_ROWS = 128, TC_K = 32, TC_MAX_TOKENS = 224, TC_ACC = 256;        // weight rows, values of K of a stage, tokens, columns between accumulators
 constexpr int TC_ROW_BYTES = TC_K * 4;                              // a swizzled row
 constexpr int TC_W_BYTES = TC_ROWS * TC_ROW_BYTES;

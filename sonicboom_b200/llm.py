@@ -38,7 +38,9 @@ class Model:
 
 def model_load(path, dtype: str = "bfloat16", device: str = "cuda:0") -> Model:
     """`boom_llm_model_load`: a model folder (config.json + safetensors) to a model on the
-    device.  `dtype` "bfloat16" serves; "float32" runs everything in true 32-bit."""
+    device.  `dtype` "bfloat16" serves; "float32" keeps weights, cache and activations in 32 bits; products
+    of more than a few rows run on the tensor cores with every operand as two TF32 values (22 to 23 bits; below the error of
+    a chain of float32 additions), all else in float32 arithmetic."""
     return Model(load_model(path, dtype=dtype, device=device))
 
 
