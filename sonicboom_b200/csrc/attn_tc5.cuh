@@ -15,14 +15,22 @@
 //               for both tiles left the tensor pipe idle half of the time;
 //   warps 2-9   softmax, four warps per query tile: a thread owns one row.  It reads its 64
 //               scores with tcgen05.ld, keeps a reference maximum and the row sum in float32
-//               registers and writes the probabilities exp2(s - reference) as bfloat16 into
-//               the swizzled P tile (two buffers).  The reference follows the running maximum
+//               registers and writes the probabilities exp2(s - reference) as bfloat16 with
+//               tcgen05.st over the first half of the scores they were made of, where P.V reads
+//               them as its A operand.  The reference follows the running maximum
 //               lazily: only when a row's maximum has grown by more than 2^8 over its
 //               reference does the warp rescale its rows of O in tensor memory (and the sums)
 //               to the new maximum, so probabilities stay below 2^8 and most pages need no
 //               pass over O at all.
 // Scores, maxima, sums and the output are float32; probabilities are rounded to bfloat16 only
 // as the P.V operand, and the row sum uses them before rounding.
+//
+// Bound by the softmax threads: 64 exponentials a row and page are 1,024 cycles of a page's four quarters of an SM, the MMAs 1,400.
+// Measured page by page before P went through tensor memory (cycles): 4,700, of them waits for the MMAs 1,400, tcgen05.ld 500,
+// arrivals of every thread on one barrier 450, the maximum 700, exponentials 1,190, P to shared memory and the fence
+// for the tensor cores 430; and 13,000 ahead of the first page, for query rows loaded one 16 bytes after another.
+// The kernel alone, us, that form / this one: 2,048 tokens of 28/4 heads of 128 53.5 / 43.0 (700 TFLOP/s), 8,192 580 / 456
+// (1,055), 97 14.7 / 11.2; turns of 500, 2,200 and 3,500 tokens 529 / 421; 64 prompts of 16 to 1,024 with 12/2 heads 268 / 181.
 //
 // Every mbarrier wait is bounded (tc5.cuh); a wait that gives up makes its role stop, the
 // others then give up as well, and the block frees its tensor memory and leaves.
@@ -34,26 +42,24 @@ namespace {
 
 constexpr int T5_ROWS = 128;                                // rows of a query tile = UMMA M
 constexpr int T5_QT = 2;                                    // query tiles per block
-constexpr int T5_ST = 3;                                    // depth of the K ring and of the V ring
+constexpr int T5_ST = 4;                                    // depth of the K ring and of the V ring
 constexpr int T5_THREADS = 64 + 128 * T5_QT + 32 * (T5_QT - 1);   // + the other tiles' MMA warps
 constexpr int T5_SUB = HD / 64 > 0 ? HD / 64 : 1;            // 64-wide pieces of a head
 constexpr uint32_t T5_Q_BYTES = T5_SUB * T5_ROWS * 128;     // one query tile
 constexpr uint32_t T5_KV_BYTES = T5_SUB * KT * 128;         // one K or one V page
-constexpr uint32_t T5_P_BYTES = T5_ROWS * 128;
-constexpr uint32_t T5_SMEM =
-    T5_QT * T5_Q_BYTES + 2 * T5_ST * T5_KV_BYTES + 2 * T5_QT * T5_P_BYTES + 512;
-constexpr uint32_t T5_TILE_COLS = 2 * KT + HD;              // tensor memory of a query tile: S0 S1 O
+constexpr uint32_t T5_SMEM = T5_QT * T5_Q_BYTES + 2 * T5_ST * T5_KV_BYTES + 512;
+constexpr uint32_t T5_TILE_COLS = 2 * KT + HD;              // tensor memory of a query tile: S0 S1 O (P over each S)
 constexpr uint32_t T5_TMEM_COLS = T5_QT * T5_TILE_COLS <= 256 ? 256 : 512;
 constexpr float T5_LAZY = 8.0f;                             // log2 of how far a maximum may run ahead
 static_assert(T5_QT * T5_TILE_COLS <= 512, "tensor memory has 512 columns");
 
 // barriers: the rings first (a stage is free when every query tile's product that read it has
-// been committed: T5_QT arrivals), then one set per query tile.  PFREE of a page also says "O
-// holds every page up to this one".
+// been committed: T5_QT arrivals), then one set per query tile.  PFREE of a page says that P.V has
+// read its probabilities and O holds every page up to this one.
 enum { T5_KFULL = 0, T5_KFREE = T5_ST, T5_VFULL = 2 * T5_ST, T5_VFREE = 3 * T5_ST,
        T5_PER_TILE = 4 * T5_ST,
-       T5_SFULL = 0, T5_SFREE = 2, T5_PFULL = 4, T5_PFREE = 6, T5_QFULL = 8,
-       T5_TILE_BARS = 9, T5_NBARS = 4 * T5_ST + T5_QT * T5_TILE_BARS };
+       T5_SFULL = 0, T5_PFULL = 2, T5_PFREE = 4, T5_QFULL = 6,
+       T5_TILE_BARS = 7, T5_NBARS = 4 * T5_ST + T5_QT * T5_TILE_BARS };
 static_assert(T5_NBARS * 8 + 8 <= 512, "barrier space");
 
 // K-major tile with the 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
@@ -96,6 +102,42 @@ __device__ __forceinline__ void t5_tmem_st32(uint32_t taddr, const uint32_t (&r)
       : "memory");
 }
 
+// D += A.B with A (bfloat16, two values a column) in tensor memory.
+__device__ __forceinline__ void t5_umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ float t5_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;\n" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// Two float32 values as one operand: each lane of the pair is rounded as an instruction of its own.
+__device__ __forceinline__ unsigned long long t5_two(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 t5_parts(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long t5_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long t5_add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // Multiplies the thread's row of O in tensor memory by `factor` (a whole warp calls this).
 __device__ __forceinline__ void t5_rescale(uint32_t taddr, float factor) {
   tc_fence_after();
@@ -118,13 +160,10 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(t5_smem);
   const uint32_t q_s = raw;                                  // checked below: 1024-byte aligned
   const uint32_t k_s = q_s + T5_QT * T5_Q_BYTES, v_s = k_s + T5_ST * T5_KV_BYTES;
-  const uint32_t p_s = v_s + T5_ST * T5_KV_BYTES;            // [query tile][2] P buffers
-  const uint32_t bars = p_s + 2 * T5_QT * T5_P_BYTES, tmem_slot = bars + 8 * T5_NBARS;
+  const uint32_t bars = v_s + T5_ST * T5_KV_BYTES, tmem_slot = bars + 8 * T5_NBARS;
   volatile uint32_t* tmem_slot_ptr = (volatile uint32_t*)(t5_smem + (tmem_slot - raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  sb_pdl_launch();
-  sb_pdl_wait();
-
+  // the step's plan was written before the step's first kernel, which triggers after its own wait
   // blockIdx.x = (block of query rows, key/value head), heads fastest and the last rows first:
   // blocks are handed out in this order, so the longest ones of every head start first
   const int b = blockIdx.z, kvh = blockIdx.x % p.n_kv_heads;
@@ -132,15 +171,19 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
   const int row0 = p.seq_row0[b], n_new = p.seq_row0[b + 1] - row0, pos0 = p.seq_pos0[b];
   const int R = n_new * G;
   const int r_base = (int)(gridDim.x / p.n_kv_heads - 1 - blockIdx.x / p.n_kv_heads) * (T5_QT * T5_ROWS);
-  if (r_base >= R) return;
-  // positions without pages in the sequence's own list: nothing is read
-  if (pos0 < 0 || (pos0 + n_new - 1) / KT >= p.page_off[b + 1] - p.page_off[b]) return;
+  // no rows, or positions without pages in the sequence's own list: nothing is read (the wait all the same: a launch
+  // whose blocks all left early would be over before the kernel before it)
+  if (r_base >= R || pos0 < 0 || (pos0 + n_new - 1) / KT >= p.page_off[b + 1] - p.page_off[b]) {
+    sb_pdl_wait();
+    return;
+  }
   const int r_last = min(R, r_base + T5_QT * T5_ROWS) - 1;
   const int tile_lo = low_key(p, pos0 + r_base / G) / KT;
   const int tile_hi = (pos0 + r_last / G) / KT;
   const int n_tiles = tile_hi - tile_lo + 1;
   if (raw & 1023u) {                       // the swizzled tiles need this alignment
     if (threadIdx.x == 0) atomicCAS(&g_status, 0, 10);
+    sb_pdl_wait();
     return;
   }
 
@@ -151,8 +194,8 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
     }
     for (int q = 0; q < T5_QT; ++q)
       for (int i = 0; i < T5_TILE_BARS; ++i) {
-        const bool by_threads = (i >= T5_SFREE && i < T5_PFREE) || i == T5_QFULL;   // else: one commit
-        mbar_init(bars + 8 * (T5_PER_TILE + q * T5_TILE_BARS + i), by_threads ? 128 : 1);
+        const bool by_warps = (i >= T5_PFULL && i < T5_PFREE) || i == T5_QFULL;   // else: one commit
+        mbar_init(bars + 8 * (T5_PER_TILE + q * T5_TILE_BARS + i), by_warps ? 4 : 1);
       }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     fence_async_smem();
@@ -162,6 +205,10 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot_ptr;
+  // Only now may the next kernel's blocks start: a product that took tensor memory on this SM ahead of this block, and then
+  // waited for it, would leave both waiting for good.
+  sb_pdl_launch();
+  sb_pdl_wait();                           // queries, keys and values come from the kernels before this one
 
   if (warp == 0) {
     // ---- producer.  The K ring and the V ring advance independently: whichever has a free
@@ -236,13 +283,13 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
     const bool leader = elect_one();
     const uint32_t tb = bars + 8 * (T5_PER_TILE + q * T5_TILE_BARS);
     const uint32_t t_tile = tmem + q * T5_TILE_COLS;
-    const uint64_t q_desc = t5_desc_k(q_s + q * T5_Q_BYTES), k_desc = t5_desc_k(k_s),
-                   p_desc = t5_desc_k(p_s + q * 2 * T5_P_BYTES), v_desc = t5_desc_mn(v_s);
+    const uint64_t q_desc = t5_desc_k(q_s + q * T5_Q_BYTES), k_desc = t5_desc_k(k_s), v_desc = t5_desc_mn(v_s);
     int ks = 0, kphase = 0;                       // K ring position of the next S product
     auto issue_s = [&](int i) -> bool {           // S of page i
       const int sb = i & 1;
       if (!mbar_wait(bars + 8 * (T5_KFULL + ks), kphase, 22)) return false;
-      if (i >= 2 && !mbar_wait(tb + 8 * (T5_SFREE + sb), ((i >> 1) - 1) & 1, 23)) return false;
+      // the scores go where the probabilities of two pages ago were: the product that read them has finished
+      if (i >= 2 && !mbar_wait(tb + 8 * (T5_PFREE + sb), ((i >> 1) - 1) & 1, 23)) return false;
       tc_fence_after();
       const uint64_t kd = k_desc + (uint64_t)(ks * (int)(T5_KV_BYTES >> 4));
       if (leader) {
@@ -267,19 +314,17 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
            mbar_wait(tb + 8 * (T5_PFULL + (j & 1)), (j >> 1) & 1, 24);
       if (!ok) break;
       tc_fence_after();
-      const uint64_t pd = p_desc + (uint64_t)((j & 1) * (int)(T5_P_BYTES >> 4));
       const uint64_t vd = v_desc + (uint64_t)(vs * (int)(T5_KV_BYTES >> 4));
       if (leader) {
 #pragma unroll
         for (int kk = 0; kk < KT / 16; ++kk)
-          umma_bf16(t_tile + 2 * KT, pd + (uint64_t)((kk * 32) >> 4),
-                    vd + (uint64_t)((kk * 16 * 128) >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          t5_umma_ts(t_tile + 2 * KT, t_tile + (j & 1) * KT + kk * 8, vd + (uint64_t)((kk * 16 * 128) >> 4), idesc_o,
+                     (j > 0 || kk > 0) ? 1u : 0u);
         umma_commit(tb + 8 * (T5_PFREE + (j & 1)));
         umma_commit(bars + 8 * (T5_VFREE + vs));
       }
       __syncwarp();
       if (++vs == T5_ST) { vs = 0; vphase ^= 1; }
-      // the softmax has read S of this page (it wrote P from it): S two pages on
       if (j + 2 < n_tiles) ok = issue_s(j + 2);
     }
   } else {
@@ -290,20 +335,31 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
     const int row = (warp & 3) * 32 + lane;
     const uint32_t tb = bars + 8 * (T5_PER_TILE + qt * T5_TILE_BARS);
     const uint32_t t_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + qt * T5_TILE_COLS;
-    const uint32_t q_tile = q_s + qt * T5_Q_BYTES, p_tile = p_s + qt * 2 * T5_P_BYTES;
+    const uint32_t q_tile = q_s + qt * T5_Q_BYTES;
     const int rq_base = r_base + qt * T5_ROWS;
-    for (int idx = tid_s; idx < T5_ROWS * (HD / 8); idx += 128) {
-      const int rr = idx / (HD / 8), ch = idx % (HD / 8);
-      const int r = rq_base + rr;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (r < R)
-        v = *reinterpret_cast<const uint4*>(
-            p.q + ((size_t)(row0 + r / G) * p.n_q_heads + kvh * G + r % G) * HD + ch * 8);
-      t5_st_shared16(q_tile + (ch >> 3) * (T5_ROWS * 128) + rr * 128 + (((ch & 7) ^ (rr & 7)) << 4),
-                     v.x, v.y, v.z, v.w);
+    // eight 16-byte pieces of the query rows a thread at once
+    constexpr int Q_PIECES = T5_ROWS * (HD / 8) / 128, Q_AT_ONCE = 8;
+#pragma unroll
+    for (int i0 = 0; i0 < Q_PIECES; i0 += Q_AT_ONCE) {
+      uint4 v[Q_AT_ONCE];
+#pragma unroll
+      for (int i = 0; i < Q_AT_ONCE; ++i) {
+        const int idx = tid_s + (i0 + i) * 128, r = rq_base + idx / (HD / 8), ch = idx % (HD / 8);
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (r < R)
+          v[i] = *reinterpret_cast<const uint4*>(
+              p.q + ((size_t)(row0 + r / G) * p.n_q_heads + kvh * G + r % G) * HD + ch * 8);
+      }
+#pragma unroll
+      for (int i = 0; i < Q_AT_ONCE; ++i) {
+        const int idx = tid_s + (i0 + i) * 128, rr = idx / (HD / 8), ch = idx % (HD / 8);
+        t5_st_shared16(q_tile + (ch >> 3) * (T5_ROWS * 128) + rr * 128 + (((ch & 7) ^ (rr & 7)) << 4),
+                       v[i].x, v[i].y, v[i].z, v[i].w);
+      }
     }
     fence_async_smem();
-    mbar_arrive(tb + 8 * T5_QFULL);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(tb + 8 * T5_QFULL);
 
     const int r = rq_base + row;
     const RowView rv = row_view<BIAS>(p, r < R ? pos0 + r / G : -1, kvh * G + r % G);
@@ -319,17 +375,13 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
     bool ok = true;
     for (int j = 0; j < n_tiles; ++j) {
       const int s = j & 1, use = j >> 1, key0 = (tile_lo + j) * KT;
-      // this page's P buffer is free when the product that read it two pages ago has finished
-      if (j >= 2) ok = mbar_wait(tb + 8 * (T5_PFREE + s), (use - 1) & 1, 33);
-      if (ok) ok = mbar_wait(tb + 8 * (T5_SFULL + s), use & 1, 31);
+      ok = mbar_wait(tb + 8 * (T5_SFULL + s), use & 1, 31);
       if (!ok) break;
       tc_fence_after();
       uint32_t sv[KT];
       tmem_ld32_nowait(t_base + s * KT, sv);
       tmem_ld32_nowait(t_base + s * KT + 32, sv + 32);
       tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(tb + 8 * (T5_SFREE + s));
 
       // every key of the page visible to every row of the tile: no mask to apply
       const bool open = key0 + KT - 1 <= p_lo && key0 >= lo_hi;
@@ -367,7 +419,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < KT; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(sv[i]));
+      for (int i = 0; i < KT; i += 2) mx[(i >> 1) & 3] = t5_max3(mx[(i >> 1) & 3], __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
       // scale > 0 and the cap is monotone: the largest dot product gives the largest exponent
       const float mx_all = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       const float m_tile = BIAS ? mx_all : capped ? (mx_all == -INFINITY ? -INFINITY : mapped_score(mx_all, sm)) : mx_all * p.scale_log2;
@@ -384,25 +436,34 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
         m_ref = m_new;
       }
       const float base = m_ref == -INFINITY ? 0.0f : m_ref;       // nothing seen yet: exp2(-inf) = 0
-      float sum0 = 0.0f, sum1 = 0.0f;
+      unsigned long long sums = t5_two(0.0f, 0.0f);             // of even and of odd keys
+      const unsigned long long scale2 = t5_two(p.scale_log2, p.scale_log2), base2 = t5_two(-base, -base);
+      uint32_t pv[KT / 2];
 #pragma unroll
       for (int i = 0; i < KT; i += 2) {
         const float d0 = __uint_as_float(sv[i]), d1 = __uint_as_float(sv[i + 1]);
-        const float p0 = BIAS ? t5_ex2(d0 - base) : capped ? (d0 == -INFINITY ? 0.0f : t5_ex2(mapped_score(d0, sm) - base))
-                                : t5_ex2(fmaf(d0, p.scale_log2, -base));
-        const float p1 = BIAS ? t5_ex2(d1 - base) : capped ? (d1 == -INFINITY ? 0.0f : t5_ex2(mapped_score(d1, sm) - base))
-                                : t5_ex2(fmaf(d1, p.scale_log2, -base));
-        sum0 += p0;
-        sum1 += p1;
-        sv[i >> 1] = pack_bf16(p0, p1);
+        float p0, p1;
+        if (BIAS) {
+          p0 = t5_ex2(d0 - base);
+          p1 = t5_ex2(d1 - base);
+        } else if (capped) {
+          p0 = d0 == -INFINITY ? 0.0f : t5_ex2(mapped_score(d0, sm) - base);
+          p1 = d1 == -INFINITY ? 0.0f : t5_ex2(mapped_score(d1, sm) - base);
+        } else {
+          const float2 e = t5_parts(t5_fma2(t5_two(d0, d1), scale2, base2));
+          p0 = t5_ex2(e.x);
+          p1 = t5_ex2(e.y);
+        }
+        sums = t5_add2(sums, t5_two(p0, p1));
+        pv[i >> 1] = pack_bf16(p0, p1);
       }
-      l += sum0 + sum1;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        t5_st_shared16(p_tile + s * T5_P_BYTES + row * 128 + ((c ^ (row & 7)) << 4), sv[4 * c],
-                       sv[4 * c + 1], sv[4 * c + 2], sv[4 * c + 3]);
-      fence_async_smem();
-      mbar_arrive(tb + 8 * (T5_PFULL + s));
+      const float2 sum = t5_parts(sums);
+      l += sum.x + sum.y;
+      t5_tmem_st32(t_base + s * KT, pv);
+      asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tb + 8 * (T5_PFULL + s));
     }
     if (ok) ok = mbar_wait(tb + 8 * (T5_PFREE + ((n_tiles - 1) & 1)), ((n_tiles - 1) >> 1) & 1, 34);
     if (ok) {
