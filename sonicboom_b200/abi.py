@@ -98,6 +98,8 @@ CORE = {
     "sb_moe_down": ("i", "pipippiiiiiips"),
     "sb_moe_combine": ("i", "pppiiis"),
     "sb_moe_join": ("i", "ppppfipippipiiiipis"),
+    "sb_gemm_tc5_takes_angles": ("i", "iiiiiiiii"),
+    "sb_rotation_table": ("i", "piipps"),
     "sb_sample_params_size": ("i", ""),
     "sb_sample": ("i", "piippipps"),
     "sb_add_i32": ("i", "piis"),

@@ -537,6 +537,28 @@ __global__ void rope_store_vec_kernel(const float* qkv, int n_q_heads, int n_kv_
   }
 }
 
+// The rotation's angles of every row of a step, for the product that rotates as it ends: made once for all its layers.
+__global__ void rotation_table_kernel(const int32_t* row_pos, int n_rows, int half, const float* __restrict__ inv_freq, float* out) {
+  sb_pdl_launch();
+  sb_pdl_wait();
+  const size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (at >= (size_t)n_rows * half) return;
+  const int t = (int)(at / half), i = (int)(at % half);
+  const float theta = (float)row_pos[t] * inv_freq[i];
+  out[(size_t)t * 2 * half + i] = cosf(theta);
+  out[(size_t)t * 2 * half + half + i] = sinf(theta);
+}
+
+extern "C" int sb_rotation_table(const int32_t* row_pos, int n_rows, int rot, const float* inv_freq, float* out, cudaStream_t stream) {
+  if (!row_pos || !inv_freq || !out || n_rows <= 0 || rot <= 0 || (rot & 1))
+    SB_FAIL(SB_ERR_ARG, "sb_rotation_table: %d rows, %d rotated values", n_rows, rot);
+  const size_t n = (size_t)n_rows * (rot / 2);
+  sb_launch<SB_K_ELEMENTWISE>(rotation_table_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, row_pos, n_rows, rot / 2,
+                              inv_freq, out);
+  SB_CHECK_LAUNCH("sb_rotation_table");
+  return SB_OK;
+}
+
 extern "C" int sb_rope_store(const float* qkv, int n_rows, int n_q_heads, int n_kv_heads, int hd,
                              int rot, const float* inv_freq, const int32_t* row_seq,
                              const int32_t* row_pos, const int32_t* page_off,

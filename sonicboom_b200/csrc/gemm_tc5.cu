@@ -1033,13 +1033,13 @@ int persistent_bn(int M, int N, int n_sms) {
 }
 
 // The pair kernel: clusters of two blocks, as many as the device runs at once (cached per kernel).
-template <int BN, typename TO>
+template <int BN, typename TO, bool ROPE = false>
 int pair_clusters() {
   static int clusters = -1;
   if (clusters >= 0) return clusters;
   constexpr int smem = pair_smem_bytes(BN, PAIR_STAGES);
   clusters = 0;
-  if (cudaFuncSetAttribute(gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem) != cudaSuccess) {
     cudaGetLastError();
     return clusters;
@@ -1049,18 +1049,18 @@ int pair_clusters() {
   cfg.blockDim = dim3(PAIR_THREADS);
   cfg.dynamicSmemBytes = smem;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO>, &cfg) == cudaSuccess && n > 0)
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO, ROPE>, &cfg) == cudaSuccess && n > 0)
     clusters = n;
   else
     cudaGetLastError();
   return clusters;
 }
 
-template <int BN, typename TO>
+template <int BN, typename TO, bool ROPE = false>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const Tc5Params& p, int clusters,
-                cudaStream_t stream) {
-  sb_launch<SB_K_TC5>(gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO>, dim3(2 * clusters), dim3(PAIR_THREADS),
-                      pair_smem_bytes(BN, PAIR_STAGES), stream, ma, mb, p);
+                cudaStream_t stream, const PairRope& rope = PairRope{}) {
+  sb_launch<SB_K_TC5>(gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO, ROPE>, dim3(2 * clusters), dim3(PAIR_THREADS),
+                      pair_smem_bytes(BN, PAIR_STAGES), stream, ma, mb, p, rope);
   SB_CHECK_LAUNCH("sb_gemm_tc5 (pairs)");
   return SB_OK;
 }
@@ -1248,6 +1248,18 @@ static bool rope_fuses(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_h
   return splits_k(M, N, K, n_sms) > 1;
 }
 
+// Whether the pair kernel finishes these rows with the rotation from a table of angles (PairRope): no K split, tiles of whole heads.
+static bool table_rotates(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_heads, int hd, int rot, int has_kv) {
+  if (M <= 0 || K <= 0 || n_q_heads <= 0 || (hd != 64 && hd != 128) || rot != hd || (has_kv && n_kv_heads <= 0)) return false;
+  if (N != (n_q_heads + (has_kv ? 2 * n_kv_heads : 0)) * hd || M <= SWAPPED_ROWS || !pair_form(M, N, n_sms)) return false;
+  return pair_splits(M, N, K, n_sms / 2) == 1 && pair_bn(M, N, n_sms / 2) == 256 && pair_clusters<256, float, true>() > 0;
+}
+
+extern "C" int sb_gemm_tc5_takes_angles(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_heads,
+                                        int hd, int rot, int has_kv) {
+  return table_rotates(M, N, K, n_sms, n_q_heads, n_kv_heads, hd, rot, has_kv) ? 1 : 0;
+}
+
 extern "C" int sb_gemm_tc5_fuses_rope(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_heads,
                                       int hd, int rot, int has_kv) {
   return rope_fuses(M, N, K, n_sms, n_q_heads, n_kv_heads, hd, rot, has_kv) ? 1 : 0;
@@ -1323,13 +1335,15 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
   if (rope) {
     // the product's rows go through the rotation into q_out and the cache; `out` is not written
     if (norm || (epilogue != SB_EPI_BIAS && epilogue != SB_EPI_NONE) || form == 1 ||
-        !rope_fuses(M, N, K, n_sms, rope->n_q_heads, rope->n_kv_heads, rope->hd, rope->rot, rope->cache != nullptr))
+        !(rope->angles ? table_rotates : rope_fuses)(M, N, K, n_sms, rope->n_q_heads, rope->n_kv_heads, rope->hd, rope->rot,
+                                                     rope->cache != nullptr))
       SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: these sizes do not take the fused rotation "
               "(see sb_gemm_tc5_fuses_rope)");
     if (!rope->q_out || !rope->inv_freq || !rope->row_pos || (rope->cache && (!rope->row_seq || !rope->page_off ||
         !rope->page_ids || rope->page_size <= 0)))
       SB_FAIL(SB_ERR_ARG, "sb_gemm_tc5: rotation arguments missing");
-    if ((((uintptr_t)rope->q_out | (uintptr_t)rope->cache) & 7) || ((uintptr_t)rope->inv_freq & 15))
+    if ((((uintptr_t)rope->q_out | (uintptr_t)rope->cache) & (rope->angles ? 15 : 7)) || ((uintptr_t)rope->inv_freq & 15) ||
+        ((uintptr_t)rope->angles & 15) || (rope->angles && ((uintptr_t)bias & 15)))
       SB_FAIL(SB_ERR_ARG, "sb_gemm_tc5: unaligned rotation operands");
     if (epilogue == SB_EPI_BIAS && !bias) SB_FAIL(SB_ERR_ARG, "sb_gemm_tc5: bias epilogue without a bias");
   } else if (int rc = sb_check_linear_args("sb_gemm_tc5", M, N, K, epilogue, bias, residual, out_dtype))
@@ -1405,6 +1419,7 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
     SB_TC5_PAIR_CLUSTERS(192)
 #undef SB_TC5_PAIR_CLUSTERS
     if (splits > 1) clusters = pair_clusters<256, float>();   // the kernel that writes the partial sums
+    if (rope && rope->angles) clusters = pair_clusters<256, float, true>();
     if (rope && clusters <= 0) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tc5: no pairs of SMs for the fused rotation");
     if (clusters > 0) {                               // else: the one-block kernel below
       if (!make_map(&ma, A, M, K, BM) || !make_map(&mb, W, N, K, bn / 2))
@@ -1421,6 +1436,11 @@ static int tc5_run(const void* A, int a_dtype, const void* W, int w_dtype, int M
         else sb_launch<SB_K_REDUCE>(tc5_splitk_reduce_kernel<bf16>, rgrid, dim3(256), 0, stream, p);
         SB_CHECK_LAUNCH("sb_gemm_tc5 (pairs, sum of the K splits)");
         return SB_OK;
+      }
+      if (rope) {
+        const PairRope r{rope->n_q_heads, rope->n_kv_heads, rope->hd, rope->angles, rope->row_seq, rope->row_pos,
+                         rope->page_off, rope->page_ids, rope->page_size, (bf16*)rope->cache, (bf16*)rope->q_out};
+        return launch_pair<256, float, true>(ma, mb, p, clusters, stream, r);
       }
 #define SB_TC5_PAIR_LAUNCH(BN_)                                                                    \
       if (bn == BN_)                                                                               \

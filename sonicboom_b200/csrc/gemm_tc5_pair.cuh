@@ -55,10 +55,98 @@ __device__ __forceinline__ void pair_tile(const Tc5Params& p, int tile, int& til
   tile_b = in_group / rows;
 }
 
-template <int BN, int STAGES, typename TO>
+// What finishes a q|k|v product of many rows (ROPE, 256-column tiles, heads of 64 or 128 that are rotated as a whole): the
+// thread keeps its row, takes 32 columns of a head and the 32 half a head further on, turns them by the row's
+// angles (a table, made once a step: worked out here they would take longer than the MMAs of a short inner dimension)
+// and writes queries and the cache's keys and values.
+struct PairRope {
+  int n_q, n_kv, hd;
+  const float* angles;                                 // [row][cos of hd / 2, sin of hd / 2]
+  const int32_t *row_seq, *row_pos, *page_off, *page_ids;
+  int page_size;
+  bf16 *cache, *q_out;
+};
+// Eight values of a bias vector.
+__device__ __forceinline__ void pair_bias8(const Tc5Params& p, int n, float (&v)[8]) {
+  if (p.bias_dtype == SB_F32) {
+    const float4* b = reinterpret_cast<const float4*>((const float*)p.bias + n);
+    const float4 x = b[0], y = b[1];
+    v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w; v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+  } else {
+    const uint4 x = *reinterpret_cast<const uint4*>((const bf16*)p.bias + n);
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+      v[2 * j] += f.x;
+      v[2 * j + 1] += f.y;
+    }
+  }
+}
+// Row m's place in the cache: its page (-1: none of its own there) and the row within.
+__device__ __forceinline__ int pair_page(const PairRope& r, int m, int& at) {
+  const int pos = r.row_pos[m], seq = r.row_seq[m], first = r.page_off[seq], pi = pos / r.page_size;
+  at = pos % r.page_size;
+  return pos >= 0 && pi < r.page_off[seq + 1] - first ? r.page_ids[first + pi] : -1;
+}
+// A warp's share of a finished tile: pairs of 32-column chunks `group`, `group` + 2, ... of its 32 rows.
+__device__ __forceinline__ void pair_rotate_tile(const Tc5Params& p, const PairRope& r, uint32_t t_row, int n_tile, int m, int group,
+                                                 int page, int at) {
+  const int half = r.hd / 2, per_head = r.hd / 32;     // chunks of a head
+#pragma unroll 1
+  for (int pi = group; pi < 4; pi += PAIR_EPI_GROUPS) {
+    const int c_lo = per_head == 4 ? (pi >> 1) * 4 + (pi & 1) : 2 * pi, n_lo = n_tile + c_lo * 32;
+    if (n_lo >= p.N) break;
+    uint32_t a[32], b[32];
+    tmem_ld32_nowait(t_row + c_lo * 32, a);
+    tmem_ld32_nowait(t_row + c_lo * 32 + half, b);
+    tmem_wait_ld();
+    const int head = n_lo / r.hd, i0 = n_lo - head * r.hd;
+    if (m >= p.M || (head >= r.n_q && page < 0)) continue;
+    bf16* dst = r.q_out + ((size_t)m * r.n_q + head) * r.hd + i0;
+    if (head >= r.n_q) {
+      const int kv = head - r.n_q, is_v = kv >= r.n_kv;
+      dst = r.cache + ((((size_t)page * 2 + is_v) * r.n_kv + kv - is_v * r.n_kv) * r.page_size + at) * r.hd + i0;
+    }
+    const bool rotates = head < r.n_q + r.n_kv;
+    const float* cs = r.angles + (size_t)m * r.hd + i0;
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      float lo[8], hi[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        lo[e] = __uint_as_float(a[j + e]);
+        hi[e] = __uint_as_float(b[j + e]);
+      }
+      if (p.epilogue == SB_EPI_BIAS) {
+        pair_bias8(p, n_lo + j, lo);
+        pair_bias8(p, n_lo + half + j, hi);
+      }
+      if (rotates) {
+        float c[8], s[8];
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+          *reinterpret_cast<float4*>(c + e) = *reinterpret_cast<const float4*>(cs + j + e);
+          *reinterpret_cast<float4*>(s + e) = *reinterpret_cast<const float4*>(cs + half + j + e);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float x = lo[e];
+          lo[e] = sb_rot_lo(x, hi[e], c[e], s[e]);
+          hi[e] = sb_rot_hi(x, hi[e], c[e], s[e]);
+        }
+      }
+      store_row(dst + j, lo, 8);
+      store_row(dst + half + j, hi, 8);
+    }
+  }
+}
+
+template <int BN, int STAGES, typename TO, bool ROPE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS)
 gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
-                     const __grid_constant__ CUtensorMap map_b, const Tc5Params p) {
+                     const __grid_constant__ CUtensorMap map_b, const Tc5Params p, const PairRope rope) {
+  static_assert(!ROPE || BN == 256, "whole heads of 64 or 128 in a tile");
   static_assert(BN % 16 == 0 && BN <= 256, "the MMA's width");
   static_assert(pair_stage_bytes(BN) % 1024 == 0, "stages keep the swizzle's 1024-byte alignment");
   extern __shared__ unsigned char smem_raw[];
@@ -182,11 +270,16 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const uint32_t acc = lt & 1;
       const int m_base = tile_a * PAIR_M + (int)rank * BM + q * 32;
       uint4 add[8];
-      if (S == 1 && chunk_rowwise(p, tile_b * BN + group * 32)) chunk_ahead(p, add, m_base + lane, tile_b * BN + group * 32);
+      int page = -1, at = 0;
+      if constexpr (ROPE) {
+        if ((tile_b + 1) * BN > rope.n_q * rope.hd && m_base + lane < p.M && rope.cache) page = pair_page(rope, m_base + lane, at);
+      } else if (S == 1 && chunk_rowwise(p, tile_b * BN + group * 32)) chunk_ahead(p, add, m_base + lane, tile_b * BN + group * 32);
       if (!mbar_wait(acc_full0 + 8 * acc, (lt >> 1) & 1, 4)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * ACC_COLS;
-      if (S > 1) {
+      if constexpr (ROPE) {
+        pair_rotate_tile(p, rope, t_row, tile_b * BN, m_base + lane, group, page, at);
+      } else if (S > 1) {
         // the split's part of the sum as it is: the thread's row, 16 bytes at a time
         const int m = m_base + lane;
         float* dst = p.scratch + ((size_t)split * p.M + (m < p.M ? m : 0)) * p.N;

@@ -67,6 +67,7 @@ typedef struct SbRopeStore {
   int page_size;
   void* cache;                 /* bfloat16 pages of the schedule entry; null: queries only */
   void* q_out;                 /* bfloat16 [rows, n_q_heads, hd] */
+  const float* angles;         /* null, or sb_rotation_table's of these rows: only where sb_gemm_tc5_takes_angles says so */
 } SbRopeStore;
 
 /* What may accompany a product (all optional): the RMSNorm of its finished rows, memory to ask
@@ -470,6 +471,11 @@ int sb_moe_join(float* x, const float* pair_out, const int32_t* ids, const float
                 const void* h, int h_dtype, const float* shared, const float* gate, int gate_ld,
                 const void* scale, int scale_dtype, int n_rows, int top, int width, void* copy,
                 int copy_dtype, sb_stream_t stream);
+
+/* Whether a q|k|v product that no K split finishes takes the rotation with it, from a table of the rows' angles. */
+int sb_gemm_tc5_takes_angles(int M, int N, int K, int n_sms, int n_q_heads, int n_kv_heads, int hd, int rot, int has_kv);
+/* out [n_rows, rot] float32: the cosines of position * inv_freq[i] for i < rot / 2, then the sines. */
+int sb_rotation_table(const int32_t* row_pos, int n_rows, int rot, const float* inv_freq, float* out, sb_stream_t stream);
 
 int sb_sample_params_size(void);
 int sb_sample(float* logits, int n_rows, int vocab, const void* params, const int32_t* history,

@@ -327,7 +327,8 @@ class RopeStore(ctypes.Structure):
     _fields_ = [("n_q_heads", ctypes.c_int), ("n_kv_heads", ctypes.c_int), ("hd", ctypes.c_int),
                 ("rot", ctypes.c_int), ("inv_freq", ctypes.c_void_p), ("row_seq", ctypes.c_void_p),
                 ("row_pos", ctypes.c_void_p), ("page_off", ctypes.c_void_p), ("page_ids", ctypes.c_void_p),
-                ("page_size", ctypes.c_int), ("cache", ctypes.c_void_p), ("q_out", ctypes.c_void_p)]
+                ("page_size", ctypes.c_int), ("cache", ctypes.c_void_p), ("q_out", ctypes.c_void_p),
+                ("angles", ctypes.c_void_p)]
 
 
 class LinearExtras(ctypes.Structure):
@@ -343,12 +344,13 @@ class LinearExtras(ctypes.Structure):
 def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, n_q_heads: int,
                    n_kv_heads: int, head_dim: int, rotary_dim: int, inv_freq: torch.Tensor, row_seq,
                    row_pos, page_off, page_ids, page_size: int, cache: torch.Tensor | None,
-                   q_out: torch.Tensor) -> torch.Tensor:
+                   q_out: torch.Tensor, angles: torch.Tensor | None = None) -> torch.Tensor:
     """The fused [q | k | v] projection of the rows `h` (+ bias), the rotation of q and k, q into
     `q_out` [rows, heads, hd] and k, v into the cache pages (`cache=None`: the weight holds the
     query rows only).  Where the weight-streaming kernel runs (up to 8 rows of bfloat16) or the tcgen05 product
     splits K (9 to several hundred rows), the kernel that finishes the sums does the rotation and the cache write too
-    and the float32 row is never written; else the product and `rope_store` run one after the other."""
+    and the float32 row is never written.  `angles`: the `rotation_table` of `row_pos` and `inv_freq`; with it the
+    product of many rows does the same where `takes_rotation_table` says so.  Else the product and `rope_store` run one after the other."""
     M, K = h.shape
     N = w.shape[0]
     assert w.shape[1] == K, f"qkv_rope_store: h is [{M},{K}], w is {tuple(w.shape)}"
@@ -364,6 +366,11 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
         if kernel == "tc5" and aligned and l.sb_gemm_tc5_fuses_rope(M, N, K, _sm_count(h.device), n_q_heads, n_kv_heads,
                                                                     head_dim, rotary_dim, 1 if has_kv else 0):
             fused = kernel
+        elif kernel == "tc5" and angles is not None and takes_rotation_table(M, w, n_q_heads, n_kv_heads, head_dim, rotary_dim, has_kv) \
+                and (inv_freq.data_ptr() | q_out.data_ptr() | (cache.data_ptr() if has_kv else 0)
+                     | (bias.data_ptr() if bias is not None else 0)) % 16 == 0:
+            fused = "table"
+            assert angles.dtype == torch.float32 and tuple(angles.shape) == (M, rotary_dim) and angles.device == h.device
         elif kernel == "skinny" and l.sb_gemm_skinny_takes_rope(M, N, n_q_heads, n_kv_heads, head_dim, rotary_dim,
                                                                 1 if has_kv else 0):
             fused = kernel
@@ -384,14 +391,34 @@ def qkv_rope_store(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, 
                "q|k|v product with rotation (weight-streaming kernel)")
         return q_out
     extras = LinearExtras()
+    if fused == "table":
+        rope.angles = _ptr(angles)
     extras.rope = ctypes.pointer(rope)
     ws = _tc5_workspace(M, N, K, h.device)
     _check(l.sb_gemm_tc5_ex(_ptr(h), BF16, _ptr(w), BF16, M, N, K, EPI_BIAS if bias is not None else EPI_NONE,
                             _ptr(bias), _code(bias.dtype) if bias is not None else 0, _ptr(None), _ptr(None), F32,
-                            _ptr(ws), ctypes.c_size_t(ws.numel()), _sm_count(h.device), 0,
+                            _ptr(ws), ctypes.c_size_t(ws.numel() if ws is not None else 0), _sm_count(h.device), 0,
                             ctypes.byref(extras), _stream()),
-           "q|k|v product with rotation (tcgen05 kernel)", launches=2)
+           "q|k|v product with rotation (tcgen05 kernel)", launches=1 if fused == "table" else 2)
     return q_out
+
+
+def takes_rotation_table(n_rows: int, w: torch.Tensor, n_q_heads: int, n_kv_heads: int, head_dim: int, rotary_dim: int,
+                         has_kv: bool = True) -> bool:
+    """Whether `qkv_rope_store` of `n_rows` bfloat16 rows through `w` rotates inside the product when it is given the
+    rows' `rotation_table`."""
+    N, K = w.shape
+    return n_rows > 128 and w.dtype == torch.bfloat16 and K % 8 == 0 and bool(lib().sb_gemm_tc5_takes_angles(
+        n_rows, N, K, _sm_count(w.device), n_q_heads, n_kv_heads, head_dim, rotary_dim, 1 if has_kv else 0))
+
+
+def rotation_table(row_pos: torch.Tensor, inv_freq: torch.Tensor, rotary_dim: int) -> torch.Tensor:
+    """[rows, rotary_dim] float32: cosines, then sines, of every row's position times `inv_freq`."""
+    assert inv_freq.dtype == torch.float32 and inv_freq.numel() >= rotary_dim // 2
+    out = torch.empty((row_pos.numel(), rotary_dim), dtype=torch.float32, device=row_pos.device)
+    _check(lib().sb_rotation_table(_i32(row_pos, "row_pos"), row_pos.numel(), rotary_dim, _ptr(inv_freq), _ptr(out), _stream()),
+           "rotation table")
+    return out
 
 
 def _warm_args(warm):

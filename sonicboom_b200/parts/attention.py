@@ -68,11 +68,15 @@ class Attention(Mixer):
         storage = ctx.kv_storage()
         g = plan.groups[ctx.kv_group()]
         q = torch.empty((rows, self.hq, self.hd), dtype=self.dtype, device=h.device)
-        ops.qkv_rope_store(h, self.w_qkv[:width_in],
+        w_in, rot = self.w_qkv[:width_in], self.position.rotary_dim
+        angles = None
+        if h.dtype == torch.bfloat16 and ops.takes_rotation_table(rows, w_in, self.hq, self.hkv, self.hd, rot, ctx.owns_cache):
+            angles = ctx.rotation_table(self.position, self.spec.position)
+        ops.qkv_rope_store(h, w_in,
                            self.b_qkv[:width_in] if self.b_qkv is not None else None, self.hq, self.hkv,
-                           self.hd, self.position.rotary_dim, self.position.inv_freq, plan.row_seq,
+                           self.hd, rot, self.position.inv_freq, plan.row_seq,
                            plan.row_pos, g.page_off, g.page_ids, g.page_size,
-                           storage if ctx.owns_cache else None, q)
+                           storage if ctx.owns_cache else None, q, angles)
         mixed = torch.empty((rows, self.qw), dtype=self.dtype, device=h.device)
         ops.attention(q, mixed, plan, ctx.kv_group(), storage, self.hq, self.hkv, self.hd,
                       self.spec.window, self.spec.scale, warm=self.w_o)

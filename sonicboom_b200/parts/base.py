@@ -87,6 +87,13 @@ class StepContext:
         kept, self._normed, self.next_norm = self._normed, None, None
         return kept[2] if kept is not None and kept[0] is norm and kept[1] is x else None
 
+    def rotation_table(self, position, spec) -> torch.Tensor:
+        """`ops.rotation_table` of the step's rows, made by the first layer that asks: layers of one position spec share it."""
+        key = ("rotation table", type(position), spec)
+        if key not in self.kept:
+            self.kept[key] = ops.rotation_table(self.plan.row_pos, position.inv_freq, position.rotary_dim)
+        return self.kept[key]
+
     def kv_storage(self) -> torch.Tensor:
         """[page, k|v, kv head, position in page, hd] of the cache this entry reads."""
         g = self.cache.groups[self.cache.group_of_entry[self.kv_entry]]
