@@ -245,13 +245,16 @@ __device__ __forceinline__ void conv_walk(const float* x, int ld, int row0, int 
       hist[d] = 0.0f;
       if (d >= 1 && d < taps) hist[d] = t0 - d >= 0 ? x[(size_t)(row0 + t0 - d) * ld + c] : before(t0 - d);
     }
-#pragma unroll 4
-    for (int i = 0; i < cnt; ++i) {
-      hist[0] = x[(size_t)(row0 + t0 + i) * ld + c];
+    float in[TB];                       // the chunk's inputs at once: four at a time they were most of the kernel
+#pragma unroll
+    for (int i = 0; i < TB; ++i) in[i] = i < cnt ? x[(size_t)(row0 + t0 + i) * ld + c] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < TB; ++i) {
+      hist[0] = in[i];
       float acc = 0.0f;
 #pragma unroll
       for (int d = MAXT - 1; d >= 0; --d) acc = fmaf(wd[d], hist[d], acc);
-      put(i, sb_silu(acc));
+      if (i < cnt) put(i, sb_silu(acc));
 #pragma unroll
       for (int d = MAXT - 1; d >= 1; --d) hist[d] = hist[d - 1];
     }
