@@ -29,8 +29,10 @@
 // Measured page by page before P went through tensor memory (cycles): 4,700, of them waits for the MMAs 1,400, tcgen05.ld 500,
 // arrivals of every thread on one barrier 450, the maximum 700, exponentials 1,190, P to shared memory and the fence
 // for the tensor cores 430; and 13,000 ahead of the first page, for query rows loaded one 16 bytes after another.
-// The kernel alone, us, that form / this one: 2,048 tokens of 28/4 heads of 128 53.5 / 43.0 (700 TFLOP/s), 8,192 580 / 456
-// (1,055), 97 14.7 / 11.2; turns of 500, 2,200 and 3,500 tokens 529 / 421; 64 prompts of 16 to 1,024 with 12/2 heads 268 / 181.
+// The kernel alone, us, that form / this one: 2,048 tokens of 28/4 heads of 128 53.7 / 39.9 (750 TFLOP/s), 97 14.6 / 9.9, 300
+// 18.1 / 12.7; turns of 500, 2,200 and 3,500 tokens 529 / 412 (1,010); 64 prompts of 16 to 1,024 with 12/2 heads 265 / 167.
+// A block runs its prologue once, from a cold instruction cache: query addresses with a division each, unrolled, were 3 us of it (97
+// tokens 11.2 us alone, and no gain at all inside a prompt).
 //
 // Every mbarrier wait is bounded (tc5.cuh); a wait that gives up makes its role stop, the
 // others then give up as well, and the block frees its tensor memory and leaves.
@@ -337,22 +339,25 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
     const uint32_t t_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + qt * T5_TILE_COLS;
     const uint32_t q_tile = q_s + qt * T5_Q_BYTES;
     const int rq_base = r_base + qt * T5_ROWS;
-    // eight 16-byte pieces of the query rows a thread at once
-    constexpr int Q_PIECES = T5_ROWS * (HD / 8) / 128, Q_AT_ONCE = 8;
-#pragma unroll
+    // Eight 16-byte pieces of the query rows a thread at once.  Row r's query is (r / G) (n_q_heads - G) + r rows after the
+    // first one's; r / G by a multiplication, exact for r below 2^32 / G.
+    constexpr int Q_PIECES = T5_ROWS * (HD / 8) / 128, Q_AT_ONCE = 8, Q_STEP = 128 / (HD / 8);
+    const uint32_t by_group = 0xffffffffu / (uint32_t)G + 1u;            // (0 for G = 1)
+    const int rr0 = tid_s / (HD / 8), ch = tid_s % (HD / 8);
+    const bf16* q0 = p.q + ((size_t)row0 * p.n_q_heads + kvh * G) * HD + ch * 8;
+#pragma unroll 1
     for (int i0 = 0; i0 < Q_PIECES; i0 += Q_AT_ONCE) {
       uint4 v[Q_AT_ONCE];
 #pragma unroll
       for (int i = 0; i < Q_AT_ONCE; ++i) {
-        const int idx = tid_s + (i0 + i) * 128, r = rq_base + idx / (HD / 8), ch = idx % (HD / 8);
+        const int r = rq_base + rr0 + (i0 + i) * Q_STEP;
+        const int t = G == 1 ? r : (int)__umulhi((uint32_t)r, by_group);
         v[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < R)
-          v[i] = *reinterpret_cast<const uint4*>(
-              p.q + ((size_t)(row0 + r / G) * p.n_q_heads + kvh * G + r % G) * HD + ch * 8);
+        if (r < R) v[i] = *reinterpret_cast<const uint4*>(q0 + ((size_t)t * (p.n_q_heads - G) + r) * HD);
       }
 #pragma unroll
       for (int i = 0; i < Q_AT_ONCE; ++i) {
-        const int idx = tid_s + (i0 + i) * 128, rr = idx / (HD / 8), ch = idx % (HD / 8);
+        const int rr = rr0 + (i0 + i) * Q_STEP;
         t5_st_shared16(q_tile + (ch >> 3) * (T5_ROWS * 128) + rr * 128 + (((ch & 7) ^ (rr & 7)) << 4),
                        v[i].x, v[i].y, v[i].z, v[i].w);
       }
