@@ -11,6 +11,7 @@
 //
 // Both need K to be a multiple of 8 (16-byte rows) and refuse other K with a clear error.
 #include "common.cuh"
+#include "device_cache.h"
 
 int sb_check_linear_args(const char* who, int M, int N, int K, int epilogue, const void* bias,
                          const float* residual, int out_dtype);
@@ -56,6 +57,43 @@ constexpr int SK_WARPS = 8;      // warps of a block; they split K
 // projection at up to 8 rows): batch 1 2.896 ms with two, 2.850 with four, 2.830 with eight,
 // 2.847 with twelve, 2.905 with sixteen; batch 8 3.115 / 3.073 / 3.064 / 3.072 / 3.130.
 constexpr int SK_UNROLL = 8;
+
+// Epilogue of 16 W rows from m0 on: thread e takes W row r = e % 16 of batch row b = e / 16, sums the warps'
+// partial results in warp order, and applies the epilogue.
+template <int NT, typename TO>
+__device__ __forceinline__ void skinny_epilogue(const float (*partial)[NT][32][4], int m0, int M, int N, int epilogue,
+                                                const void* bias, int bias_dtype, const float* residual, TO* out,
+                                                float gate_limit, float gate_slope) {
+  for (int e = threadIdx.x; e < 16 * 8 * NT; e += SK_WARPS * 32) {
+    const int r = e & 15, b = e >> 4;
+    if (b >= M) continue;
+    const int nt = b >> 3, src_lane = (r & 7) * 4 + ((b & 7) >> 1), reg = (r >> 3) * 2 + (b & 1);
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < SK_WARPS; ++w) v += partial[w][nt][src_lane][reg];
+    const int n = m0 + r;
+    if (epilogue == SB_EPI_SWIGLU) {
+      if (r >= 8 || n >= N) continue;           // rows 0..7 are gates, 8..15 their up rows
+      float up = 0.0f;
+#pragma unroll
+      for (int w = 0; w < SK_WARPS; ++w) up += partial[w][nt][src_lane][reg + 2];
+      // gate_limit > 0: the clamped form a sigmoid(slope a) (b + 1) instead of silu(gate) * up;
+      // gate_limit < 0: gelu(gate) * up in gelu's tanh form
+      out[(size_t)b * (N / 2) + (m0 / 2 + r)] = sb_from_f32<TO>(
+          gate_limit > 0.0f ? sb_glu_clamped(v, up, gate_limit, gate_slope)
+                            : gate_limit < 0.0f ? sb_gelu_tanh(v) * up : sb_silu(v) * up);
+      continue;
+    }
+    if (n >= N) continue;
+    if (epilogue == SB_EPI_BIAS)
+      v += bias_dtype == SB_F32 ? load_bias<float>(bias, n) : load_bias<bf16>(bias, n);
+    else if (epilogue == SB_EPI_RESIDUAL)
+      v += residual[(size_t)b * N + n];
+    else if (epilogue == SB_EPI_RELU2)
+      v = sb_relu2(v);
+    out[(size_t)b * N + n] = sb_from_f32<TO>(v);
+  }
+}
 
 // W is the MMA's A operand (16 rows of W), the activations its B operand (8 rows each).
 // Within a 32-wide K block, thread t of a quad loads the 8 consecutive values k0+8t..k0+8t+7
@@ -171,37 +209,108 @@ gemm_skinny_kernel(const bf16* X, const bf16* __restrict__ W, int M, int N, int 
     dst[e_hi] = __float2bfloat16_rn(hi);
     return;
   }
-  // Epilogue: thread e takes W row r = e % 16 of batch row b = e / 16, sums the warps'
-  // partial results in warp order, and applies the epilogue.
-  for (int e = threadIdx.x; e < 16 * 8 * NT; e += SK_WARPS * 32) {
-    const int r = e & 15, b = e >> 4;
-    if (b >= M) continue;
-    const int nt = b >> 3, src_lane = (r & 7) * 4 + ((b & 7) >> 1), reg = (r >> 3) * 2 + (b & 1);
-    float v = 0.0f;
+  skinny_epilogue<NT, TO>(partial, m0, M, N, epilogue, bias, bias_dtype, residual, out, gate_limit, gate_slope);
+}
+
+// The same sums for up to 8 rows of a W with more groups of 16 rows than run at once: a block stays for every gridDim.x-th
+// group and keeps U K blocks of its warps' share in flight.  A K block's registers are asked for again, for the share's
+// next part or the next group's first, as soon as its MMAs have read them, so that loads go on through the sums, the
+// epilogue and what would be the start of another block.  Norm and gate/up product of one row of 17,920 x 1,536 14.4 to
+// 12.6 us (8.4 at the memory's pace); a grid of two waves or less gains nothing (a decode step of the recurrent design).
+template <int U, typename TO>
+__global__ void __launch_bounds__(SK_WARPS * 32, 2)
+gemm_skinny_stream_kernel(const bf16* X, const bf16* __restrict__ W, int M, int N, int K,
+                          int epilogue, const void* __restrict__ bias, int bias_dtype,
+                          const float* residual, TO* out, float gate_limit, float gate_slope) {
+  __shared__ __align__(16) float partials[2][SK_WARPS][1][32][4];  // sums of one group are written while the last one's are read
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int groups = (N + 15) / 16;
+  const uint4 *w0, *w1;
+  auto point_at = [&](int group) {
+    w0 = (const uint4*)(W + (size_t)min(group * 16 + g, N - 1) * K) + t;
+    w1 = (const uint4*)(W + (size_t)min(group * 16 + 8 + g, N - 1) * K) + t;
+  };
+  const bool xok = g < M;
+  const uint4* xp = (const uint4*)(X + (size_t)min(g, M - 1) * K) + t;
+  const int n_blocks = (K + 31) >> 5, steps = (n_blocks + SK_WARPS * U - 1) / (SK_WARPS * U);
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  auto inside = [&](int k) { return k < n_blocks && (k * 32 + 8 * t + 8 <= K); };
+  uint4 wa[U], wb[U];
+  point_at(blockIdx.x);
 #pragma unroll
-    for (int w = 0; w < SK_WARPS; ++w) v += partial[w][nt][src_lane][reg];
-    const int n = m0 + r;
-    if (epilogue == SB_EPI_SWIGLU) {
-      if (r >= 8 || n >= N) continue;           // rows 0..7 are gates, 8..15 their up rows
-      float up = 0.0f;
-#pragma unroll
-      for (int w = 0; w < SK_WARPS; ++w) up += partial[w][nt][src_lane][reg + 2];
-      // gate_limit > 0: the clamped form a sigmoid(slope a) (b + 1) instead of silu(gate) * up;
-      // gate_limit < 0: gelu(gate) * up in gelu's tanh form
-      out[(size_t)b * (N / 2) + (m0 / 2 + r)] = sb_from_f32<TO>(
-          gate_limit > 0.0f ? sb_glu_clamped(v, up, gate_limit, gate_slope)
-                            : gate_limit < 0.0f ? sb_gelu_tanh(v) * up : sb_silu(v) * up);
-      continue;
-    }
-    if (n >= N) continue;
-    if (epilogue == SB_EPI_BIAS)
-      v += bias_dtype == SB_F32 ? load_bias<float>(bias, n) : load_bias<bf16>(bias, n);
-    else if (epilogue == SB_EPI_RESIDUAL)
-      v += residual[(size_t)b * N + n];
-    else if (epilogue == SB_EPI_RELU2)
-      v = sb_relu2(v);
-    out[(size_t)b * N + n] = sb_from_f32<TO>(v);
+  for (int u = 0; u < U; ++u) {
+    const int k = warp + u * SK_WARPS;
+    const bool ok = inside(k);
+    wa[u] = ok ? ldg_stream(w0 + k * 4) : zero;
+    wb[u] = ok ? ldg_stream(w1 + k * 4) : zero;
   }
+  sb_pdl_wait();                     // the weights above do not depend on the kernel before this one; all that follows does
+  int buffer = 0;
+  for (int group = blockIdx.x; group < groups; group += gridDim.x) {
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int step = 0; step < steps; ++step) {
+      const bool last = step + 1 == steps, more = !last || group + (int)gridDim.x < groups;
+      const int first = warp + step * U * SK_WARPS, next = last ? warp : first + U * SK_WARPS;
+      if (last && more) point_at(group + gridDim.x);
+      uint4 xs[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = first + u * SK_WARPS;
+        xs[u] = inside(k) && xok ? ldg_cached(xp + k * 4) : zero;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        mma_bf16(acc, wa[u].x, wb[u].x, wa[u].y, wb[u].y, xs[u].x, xs[u].y);
+        mma_bf16(acc, wa[u].z, wb[u].z, wa[u].w, wb[u].w, xs[u].z, xs[u].w);
+        const int k = next + u * SK_WARPS;
+        const bool ok = more && inside(k);
+        wa[u] = ok ? ldg_stream(w0 + k * 4) : zero;
+        wb[u] = ok ? ldg_stream(w1 + k * 4) : zero;
+      }
+      if (!more) sb_pdl_launch();    // the weights have been read
+    }
+    *reinterpret_cast<float4*>(partials[buffer][warp][0][lane]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    __syncthreads();
+    skinny_epilogue<1, TO>(partials[buffer], group * 16, M, N, epilogue, bias, bias_dtype, residual, out, gate_limit, gate_slope);
+    buffer ^= 1;
+  }
+}
+
+// How many of a kernel's blocks run at once on the current device (0: not known).
+template <auto kernel>
+int skinny_resident() {
+  static SbDeviceCache most;
+  int device = -1;
+  cudaGetDevice(&device);
+  const int n = most.get(device, [&] {
+    int per_sm = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SK_WARPS * 32, 0) != cudaSuccess) return -1;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return -1;
+    return per_sm * sms;
+  });
+  return n > 0 ? n : 0;
+}
+
+// Launches the streaming form if the product has more than two waves of groups; U leaves the fewest places of a warp's
+// share empty, the more in flight the better.
+template <int U, typename TO, typename... Args>
+bool stream_with(int N, cudaStream_t stream, Args... args) {
+  const int groups = (N + 15) / 16, most = skinny_resident<gemm_skinny_stream_kernel<U, TO>>();
+  if (most == 0 || groups <= 2 * most) return false;
+  sb_launch<SB_K_SKINNY>(gemm_skinny_stream_kernel<U, TO>, dim3(most), dim3(SK_WARPS * 32), 0, stream, args...);
+  return true;
+}
+template <typename TO, typename... Args>
+bool launch_stream(int N, int K, cudaStream_t stream, Args... args) {
+  const int mine = ((K + 31) / 32 + SK_WARPS - 1) / SK_WARPS;     // a warp's K blocks
+  auto places = [&](int u) { return (mine + u - 1) / u * u; };
+  int best = 8;
+  for (int u = 7; u >= 5; --u)
+    if (places(u) < places(best)) best = u;
+  if (best == 8) return stream_with<8, TO>(N, stream, args...);
+  if (best == 7) return stream_with<7, TO>(N, stream, args...);
+  if (best == 6) return stream_with<6, TO>(N, stream, args...);
+  return stream_with<5, TO>(N, stream, args...);
 }
 
 template <int NT>
@@ -210,7 +319,10 @@ int launch_skinny(const bf16* X, const bf16* W, int M, int N, int K, int epilogu
                   int out_dtype, float gate_limit, float gate_slope, cudaStream_t stream) {
   const int blocks = (N + 15) / 16;
   SB_DISPATCH_DTYPE(out_dtype, TO, {
-    sb_launch<SB_K_SKINNY>(gemm_skinny_kernel<NT, TO, false>, dim3(blocks), dim3(SK_WARPS * 32), 0, stream,
+    bool streams = false;
+    if constexpr (NT == 1)
+      streams = launch_stream<TO>(N, K, stream, X, W, M, N, K, epilogue, bias, bias_dtype, residual, (TO*)out, gate_limit, gate_slope);
+    if (!streams) sb_launch<SB_K_SKINNY>(gemm_skinny_kernel<NT, TO, false>, dim3(blocks), dim3(SK_WARPS * 32), 0, stream,
         X, W, M, N, K, epilogue, bias, bias_dtype, residual, (TO*)out, gate_limit, gate_slope, SbRopeStore{});
   });
   SB_CHECK_LAUNCH("sb_gemm_skinny");
