@@ -58,7 +58,9 @@ __device__ __forceinline__ void pair_tile(const Tc5Params& p, int tile, int& til
 // What finishes a q|k|v product of many rows (ROPE, 256-column tiles, heads of 64 or 128 that are rotated as a whole): the
 // thread keeps its row, takes 32 columns of a head and the 32 half a head further on, turns them by the row's
 // angles (a table, made once a step: worked out here they would take longer than the MMAs of a short inner dimension)
-// and writes queries and the cache's keys and values.
+// and writes queries and the cache's keys and values.  33,000 rows of 12/2 heads of 128 at K = 1,536: product and rotation kernel
+// about 200 and 188 us, this 262; three 7B turns of 6,000 rows with it and the attention 85.0 to 81.2 ms, 64 prompts 103.2 to 98.4
+// (attention alone: 83.2 and 101.1).
 struct PairRope {
   int n_q, n_kv, hd;
   const float* angles;                                 // [row][cos of hd / 2, sin of hd / 2]
