@@ -24,6 +24,9 @@ def test_pieces_give_the_same_bits(M, N, K):
         if gated and N % 16:
             continue
         for dt in (torch.float32, torch.bfloat16):
+            if epi == ops.EPI_RESIDUAL and dt != torch.float32:      # refused: the residual sum is kept in float32
+                continue
+
             def product(s):
                 out = torch.empty(M, (s.stop - s.start) // (2 if gated else 1), device=DEV, dtype=dt)
                 return ops.linear(a, w[s], out, epi, bias=bias[s].contiguous() if epi == ops.EPI_BIAS else None,
