@@ -949,7 +949,7 @@ cudaError_t launch_scan(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
     return launch_scan_columns<NPL, 2, VEC>(a, n_seqs, stream);
   } else {
     const long blocks4 = (long)((a.vdim + 4 * SCAN_GROUPS - 1) / (4 * SCAN_GROUPS)) * a.n_heads * n_seqs;
-    if (g_force_cpt > 1 ? g_force_cpt == 4 : blocks4 >= sm_count()) return launch_scan_columns<NPL, 4, VEC>(a, n_seqs, stream);
+    if (g_force_cpt ? g_force_cpt == 4 : blocks4 >= sm_count()) return launch_scan_columns<NPL, 4, VEC>(a, n_seqs, stream);
     return launch_scan_columns<NPL, 2, VEC>(a, n_seqs, stream);
   }
 }
@@ -1065,14 +1065,8 @@ extern "C" int sb_gdelta_scan(const float* act, const float* mats, const float* 
   const int need = (dim + SCAN_LANES - 1) / SCAN_LANES;
   cudaError_t e;
 #define SB_GD_SCAN(N) e = vec ? launch_scan<N, true>(a, n_seqs, stream) : launch_scan<N, false>(a, n_seqs, stream)
-  // Whole quarters of 16 or 32 channels, whole groups of columns, 16-byte rows: the tensor cores, where their blocks are more
-  // than the SMs.  A block alone on its SM takes a chunk in 3.1 us (its MMAs and four barriers one after the other), the FFMA
-  // form in 2.4 with two blocks and 1.6 with one, but the MMAs of several blocks overlap.  Prep, scan and gate together, us, FFMA / MMA:
-  // 32 heads of 128 x 128, eight sequences of 300 tokens (1,024 blocks) 417 / 336; 56 heads, one of 2,048 (224) 721 / 570;
-  // 32 heads, one of 2,048 (128) 415 / 503; 16 heads (64) 373 / 461; 32 heads of 64 x 64 (64) 420 / 412.
-  const long mma_blocks = (long)(vdim / GM_COLS) * n_heads * n_seqs;
-  const bool mma = vec && vdim % GM_COLS == 0 && (dim == 64 || dim == 128) && !((uintptr_t)memory & 7) &&
-                   (g_force_cpt == 1 || (g_force_cpt == 0 && mma_blocks > sm_count()));
+  // whole quarters of 16 or 32 channels, whole groups of columns, 16-byte rows: the tensor cores
+  const bool mma = vec && vdim % GM_COLS == 0 && (dim == 64 || dim == 128) && g_force_cpt == 0 && !((uintptr_t)memory & 7);
   if (mma) e = dim == 64 ? launch_scan_mma<64>(a, n_seqs, stream) : launch_scan_mma<128>(a, n_seqs, stream);
   else if (need <= 2) SB_GD_SCAN(2);
   else if (need <= 4) SB_GD_SCAN(4);
@@ -1084,6 +1078,6 @@ extern "C" int sb_gdelta_scan(const float* act, const float* mats, const float* 
   return SB_OK;
 }
 
-// For measurements and tests: the FFMA scan with 2 or 4 columns per thread for every call (where the sizes allow four), 1 the
-// tensor-core scan wherever the sizes allow it, 0 by the sizes again.
-extern "C" void sb_gdelta_force_columns(int cpt) { g_force_cpt = cpt == 1 || cpt == 2 || cpt == 4 ? cpt : 0; }
+// For measurements and tests: the FFMA scan with 2 or 4 columns per thread for every call (where the sizes allow four), 0 by the
+// sizes again.
+extern "C" void sb_gdelta_force_columns(int cpt) { g_force_cpt = cpt == 2 || cpt == 4 ? cpt : 0; }
