@@ -439,20 +439,6 @@ __device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
   return r;
 }
 
-// The convolution's last inputs (the kernel before the scan has read the old ones): a head keeps its own values' channels, a
-// group's first head those of q and k too.
-template <int N_THREADS>
-__device__ __forceinline__ void keep_inputs(const ScanArgs& p, int b, int h, int row0, int n, int slot) {
-  const int dim = p.dim, vdim = p.vdim, taps = p.taps, per = p.n_heads / p.n_kv_heads, kv = h / per;
-  const int kw = p.n_kv_heads * dim, C = 2 * kw + p.n_heads * vdim;
-  float* ring = p.ring + (size_t)slot * taps * C;
-  const int pos0 = p.seq_pos0[b], keep = min(n, taps), n_ch = vdim + (h == kv * per ? 2 * dim : 0);
-  for (int i = threadIdx.x; i < n_ch; i += N_THREADS) {
-    const int c = i < vdim ? 2 * kw + h * vdim + i : (i < vdim + dim ? kv * dim + i - vdim : kw + kv * dim + i - vdim - dim);
-    for (int t = n - keep; t < n; ++t) ring[(size_t)((pos0 + t) % taps) * C + c] = p.proj[(size_t)(row0 + t) * p.ld + p.q_off + c];
-  }
-}
-
 // The lanes of a column add their parts of eight tokens' sums, halving what a lane keeps each time: lane `sub` ends with the
 // sum of token sub % 8, by the same tree of additions for every token.
 __device__ __forceinline__ float share_sums(float (&a)[HALF], int sub) {
@@ -694,222 +680,16 @@ __global__ void __launch_bounds__(SCAN_THREADS) gdelta_scan_kernel(const ScanArg
       if (col + x < vdim && c < dim) memory[(size_t)(col + x) * dim + c] = f.x;
       if (col + x < vdim && c + 1 < dim) memory[(size_t)(col + x) * dim + c + 1] = f.y;
     }
-  if (taps > 1 && blockIdx.x == 0) keep_inputs<SCAN_THREADS>(p, b, h, row0, n, slot);
-}
-
-// ------------------------------------------------------------------------------------------- the scan on the tensor cores
-// The same chunk for heads of DK = 64 or 128 key channels and whole groups of 32 columns.  The passes over the state are
-// products of 16 tokens with it, and the FFMA kernel above is bound by what it reads of shared memory for them (and by
-// the chain of a chunk's phases with two blocks an SM).  Here the state's transpose lies in the accumulator fragments of
-// mma.sync m16n8k8 (16 columns x 8 channels a tile): as they are, channel 2t in slot t and 2t + 1 in slot t + 4, they are
-// also the A operand of S^T [k; q], so the state never leaves its registers, and the keys and queries are read once a
-// warp for 16 columns.  Warp (mt, dq) holds 16 columns and a quarter of the channels; the quarters' sums are added in
-// order through shared memory, the 16 x 16 matrices T and P are applied in float32.
-// Operands are split into two TF32 values (see gemm_f32_tc5.cu; three MMAs a product, the small ones first, chains of at
-// most twelve, what is added to the state rounded once by a float32 fma).
-constexpr int GM_COLS = 32, GM_THREADS = 256, GM_XP = 33, GM_UP = 40;
-
-template <int DK>
-struct MmaShape {
-  static constexpr int DW = DK / 4, NT = DW / 8;                        // channels of a warp, their tiles
-  static constexpr int KP = DK + 8, VP = GM_COLS + 4;                   // pitches: fragments without bank conflicts
-  static constexpr int STAGE = 2 * TB * KP + TB * VP + MAT_SM;
-  static constexpr int EXTRA = 4 * GM_COLS * GM_XP + 2 * TB * GM_UP;
-  static constexpr int STAGES = 3;
-  static constexpr size_t BYTES = ((size_t)STAGES * STAGE + EXTRA) * sizeof(float);
-};
-
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi)) & 0xffffe000u;
-}
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-template <int DK>
-__global__ void __launch_bounds__(GM_THREADS, 2) gdelta_scan_mma_kernel(const ScanArgs p) {
-  using Sh = MmaShape<DK>;
-  constexpr int NT = Sh::NT, KP = Sh::KP, VP = Sh::VP, STAGES = Sh::STAGES;
-  extern __shared__ __align__(16) float sm[];
-  float* xs = sm + STAGES * Sh::STAGE;                 // [quarter][column][token of k, then of q]
-  float* ws = xs + 4 * GM_COLS * GM_XP;                // [token][column]: w = v - G S^T k
-  float* us = ws + TB * GM_UP;                         // [token][column]: u = T w
-  sb_pdl_launch();
-  const int b = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3, mt = warp >> 2, dq = warp & 3;
-  const int vdim = p.vdim, taps = p.taps, per = p.n_heads / p.n_kv_heads, kv = h / per;
-  const int kw = p.n_kv_heads * DK, C = 2 * kw + p.n_heads * vdim, col0 = blockIdx.x * GM_COLS;
-  const int row0 = p.seq_row0[b], n = p.seq_row0[b + 1] - row0, slot = p.seq_slot[b];
-  sb_pdl_wait();
-  const float* act = p.act + (size_t)row0 * C;
-  const float* mats = p.mats + ((size_t)chunk_base(row0, b) * p.n_heads + h) * MATS;
-  const float* q_src = act + kv * DK;
-  const float* v_src = act + 2 * kw + h * vdim + col0;
-  auto stage = [&](int st, int ch) {
-    float* dst = sm + (size_t)st * Sh::STAGE;
-    constexpr int PIECES = DK / 4;
-#pragma unroll
-    for (int i = tid; i < 2 * TB * PIECES; i += GM_THREADS) {          // queries, then keys
-      const int is_k = i / (TB * PIECES), tok = i / PIECES % TB, c = i % PIECES * 4;
-      const bool ok = ch * TB + tok < n;
-      cp_async16(dst + (is_k * TB + tok) * KP + c, q_src + is_k * kw + (size_t)(ok ? ch * TB + tok : 0) * C + c, ok);
-    }
-    float* vs = dst + 2 * TB * KP;
-    if (tid < TB * GM_COLS / 4) {
-      const int tok = tid / (GM_COLS / 4), c = tid % (GM_COLS / 4) * 4;
-      const bool ok = ch * TB + tok < n;
-      cp_async16(vs + tok * VP + c, v_src + (size_t)(ok ? ch * TB + tok : 0) * C + c, ok);
-    }
-    float* m = vs + TB * VP;
-    const float* src = mats + (size_t)ch * p.n_heads * MATS;
-    if (tid < MATS / 4) {
-      const int e = tid * 4;
-      cp_async16(m + (e < 2 * TB * TB ? (e / TB) * TP + e % TB : 2 * TB * TP + e - 2 * TB * TB), src + e, true);
-    }
-  };
-  const int n_chunks = (n + TB - 1) / TB;
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < n_chunks) stage(s, s);
-    cp_commit();
-  }
-  // the warp's part of the state: columns mt * 16 + g (+ 8), channels dq * DW + 8 j + 2t (+ 1)
-  float* memory = p.memory + (((size_t)slot * p.n_heads + h) * vdim + col0 + mt * 16 + g) * DK + dq * Sh::DW + 2 * t;
-  float S[NT][4];
-#pragma unroll
-  for (int j = 0; j < NT; ++j) {
-    const float2 x = *reinterpret_cast<const float2*>(memory + 8 * j), y = *reinterpret_cast<const float2*>(memory + 8 * DK + 8 * j);
-    S[j][0] = x.x; S[j][1] = x.y; S[j][2] = y.x; S[j][3] = y.y;
-  }
-  const int cc = tid & 31, i0 = (tid >> 5) * 2;        // what the thread has of the column work: a column, two tokens
-
-  for (int ch = 0; ch < n_chunks; ++ch) {
-    cp_wait<STAGES - 2>();
-    __syncthreads();                    // the chunk has landed, and every thread is done with the buffer staged next
-    if (ch + STAGES - 1 < n_chunks) stage((ch + STAGES - 1) % STAGES, ch + STAGES - 1);
-    cp_commit();
-    const float* q = sm + (size_t)(ch % STAGES) * Sh::STAGE;
-    const float* k = q + TB * KP;
-    const float* v = k + TB * KP;
-    const float* T = v + TB * VP;
-    const float* P = T + TB * TP;
-    const float* G = P + TB * TP;
-    const float* D = G + TB;
-    {  // S^T [k; q] over the warp's channels: tokens 8 nt ... of k (nt 0, 1) and of q (2, 3)
-      float x[4][4] = {};
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        uint32_t ah[4], al[4];          // slot t: channel 2t, slot t + 4: channel 2t + 1
-        split_tf32(S[j][0], ah[0], al[0]);
-        split_tf32(S[j][2], ah[1], al[1]);
-        split_tf32(S[j][1], ah[2], al[2]);
-        split_tf32(S[j][3], ah[3], al[3]);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const float2 f = *reinterpret_cast<const float2*>((nt < 2 ? k : q) + ((nt & 1) * 8 + g) * KP + dq * Sh::DW + 8 * j + 2 * t);
-          uint32_t bh[2], bl[2];
-          split_tf32(f.x, bh[0], bl[0]);
-          split_tf32(f.y, bh[1], bl[1]);
-          mma_tf32(x[nt], al, bh);
-          mma_tf32(x[nt], ah, bl);
-          mma_tf32(x[nt], ah, bh);
-        }
-      }
-      float* to = xs + (dq * GM_COLS + mt * 16 + g) * GM_XP + 2 * t;
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        to[8 * nt] = x[nt][0];
-        to[8 * nt + 1] = x[nt][1];
-        to[8 * GM_XP + 8 * nt] = x[nt][2];
-        to[8 * GM_XP + 8 * nt + 1] = x[nt][3];
-      }
-    }
-    __syncthreads();
-    float o[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float d = 0.0f, e = 0.0f;
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        d += xs[(s * GM_COLS + cc) * GM_XP + i0 + i];
-        e += xs[(s * GM_COLS + cc) * GM_XP + TB + i0 + i];
-      }
-      const float gi = G[i0 + i];
-      ws[(i0 + i) * GM_UP + cc] = v[(i0 + i) * VP + cc] - gi * d;
-      o[i] = gi * e;
-    }
-    __syncthreads();
-    float u[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int j = 0; j < TB; j += 4) {
-      const float4 m0 = *reinterpret_cast<const float4*>(T + i0 * TP + j), m1 = *reinterpret_cast<const float4*>(T + (i0 + 1) * TP + j);
-      const float w0 = ws[j * GM_UP + cc], w1 = ws[(j + 1) * GM_UP + cc], w2 = ws[(j + 2) * GM_UP + cc], w3 = ws[(j + 3) * GM_UP + cc];
-      u[0] = fmaf(m0.x, w0, u[0]); u[0] = fmaf(m0.y, w1, u[0]); u[0] = fmaf(m0.z, w2, u[0]); u[0] = fmaf(m0.w, w3, u[0]);
-      u[1] = fmaf(m1.x, w0, u[1]); u[1] = fmaf(m1.y, w1, u[1]); u[1] = fmaf(m1.z, w2, u[1]); u[1] = fmaf(m1.w, w3, u[1]);
-    }
-    us[i0 * GM_UP + cc] = u[0];
-    us[(i0 + 1) * GM_UP + cc] = u[1];
-    __syncthreads();
-    {  // S^T <- G_15 S^T + (D u)^T k
-      const float g_all = G[TB - 1];
-      float add[NT][4] = {};
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const float* at = us + (8 * s + t) * GM_UP + mt * 16 + g;
-        const float d0 = D[8 * s + t], d1 = D[8 * s + t + 4];
-        uint32_t ah[4], al[4];
-        split_tf32(d0 * at[0], ah[0], al[0]);
-        split_tf32(d0 * at[8], ah[1], al[1]);
-        split_tf32(d1 * at[4 * GM_UP], ah[2], al[2]);
-        split_tf32(d1 * at[4 * GM_UP + 8], ah[3], al[3]);
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          const float* kb = k + (8 * s + t) * KP + dq * Sh::DW + 8 * j + g;
-          uint32_t bh[2], bl[2];
-          split_tf32(kb[0], bh[0], bl[0]);
-          split_tf32(kb[4 * KP], bh[1], bl[1]);
-          mma_tf32(add[j], al, bh);
-          mma_tf32(add[j], ah, bl);
-          mma_tf32(add[j], ah, bh);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) S[j][i] = fmaf(S[j][i], g_all, add[j][i]);
-    }
-    // o += P u
-#pragma unroll
-    for (int j = 0; j < TB; j += 4) {
-      const float4 m0 = *reinterpret_cast<const float4*>(P + i0 * TP + j), m1 = *reinterpret_cast<const float4*>(P + (i0 + 1) * TP + j);
-      const float w0 = us[j * GM_UP + cc], w1 = us[(j + 1) * GM_UP + cc], w2 = us[(j + 2) * GM_UP + cc], w3 = us[(j + 3) * GM_UP + cc];
-      o[0] = fmaf(m0.x, w0, o[0]); o[0] = fmaf(m0.y, w1, o[0]); o[0] = fmaf(m0.z, w2, o[0]); o[0] = fmaf(m0.w, w3, o[0]);
-      o[1] = fmaf(m1.x, w0, o[1]); o[1] = fmaf(m1.y, w1, o[1]); o[1] = fmaf(m1.z, w2, o[1]); o[1] = fmaf(m1.w, w3, o[1]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int at = ch * TB + i0 + i;
-      if (at < n) p.out[((size_t)(row0 + at) * p.n_heads + h) * vdim + col0 + cc] = o[i];
+  // the convolution's last inputs (the kernel before this one has read the old ones): a head keeps its own values'
+  // channels, a group's first head those of q and k too
+  if (taps > 1 && blockIdx.x == 0) {
+    float* ring = p.ring + (size_t)slot * taps * C;
+    const int pos0 = p.seq_pos0[b], keep = min(n, taps), n_ch = vdim + (h == kv * per ? 2 * dim : 0);
+    for (int i = tid; i < n_ch; i += SCAN_THREADS) {
+      const int c = i < vdim ? 2 * kw + h * vdim + i : (i < vdim + dim ? kv * dim + i - vdim : kw + kv * dim + i - vdim - dim);
+      for (int t = n - keep; t < n; ++t) ring[(size_t)((pos0 + t) % taps) * C + c] = p.proj[(size_t)(row0 + t) * p.ld + p.q_off + c];
     }
   }
-  cp_wait<0>();
-#pragma unroll
-  for (int j = 0; j < NT; ++j) {
-    *reinterpret_cast<float2*>(memory + 8 * j) = make_float2(S[j][0], S[j][1]);
-    *reinterpret_cast<float2*>(memory + 8 * DK + 8 * j) = make_float2(S[j][2], S[j][3]);
-  }
-  if (taps > 1 && blockIdx.x == 0) keep_inputs<GM_THREADS>(p, b, h, row0, n, slot);
-}
-
-template <int DK>
-cudaError_t launch_scan_mma(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
-  constexpr size_t smem = MmaShape<DK>::BYTES;
-  if (cudaError_t e = cudaFuncSetAttribute(gdelta_scan_mma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
-  return sb_launch<SB_K_OTHER>(gdelta_scan_mma_kernel<DK>, dim3(a.vdim / GM_COLS, a.n_heads, n_seqs), dim3(GM_THREADS), smem, stream, a);
 }
 
 int sm_count() {
@@ -1065,10 +845,7 @@ extern "C" int sb_gdelta_scan(const float* act, const float* mats, const float* 
   const int need = (dim + SCAN_LANES - 1) / SCAN_LANES;
   cudaError_t e;
 #define SB_GD_SCAN(N) e = vec ? launch_scan<N, true>(a, n_seqs, stream) : launch_scan<N, false>(a, n_seqs, stream)
-  // whole quarters of 16 or 32 channels, whole groups of columns, 16-byte rows: the tensor cores
-  const bool mma = vec && vdim % GM_COLS == 0 && (dim == 64 || dim == 128) && g_force_cpt == 0 && !((uintptr_t)memory & 7);
-  if (mma) e = dim == 64 ? launch_scan_mma<64>(a, n_seqs, stream) : launch_scan_mma<128>(a, n_seqs, stream);
-  else if (need <= 2) SB_GD_SCAN(2);
+  if (need <= 2) SB_GD_SCAN(2);
   else if (need <= 4) SB_GD_SCAN(4);
   else if (need <= 8) SB_GD_SCAN(8);
   else if (need <= 16) SB_GD_SCAN(16);
@@ -1078,6 +855,5 @@ extern "C" int sb_gdelta_scan(const float* act, const float* mats, const float* 
   return SB_OK;
 }
 
-// For measurements and tests: the FFMA scan with 2 or 4 columns per thread for every call (where the sizes allow four), 0 by the
-// sizes again.
+// For measurements and tests: 2 or 4 columns per thread for every call (where the sizes allow four), 0 by the sizes again.
 extern "C" void sb_gdelta_force_columns(int cpt) { g_force_cpt = cpt == 2 || cpt == 4 ? cpt : 0; }
