@@ -165,27 +165,9 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
   const uint32_t bars = v_s + T5_ST * T5_KV_BYTES, tmem_slot = bars + 8 * T5_NBARS;
   volatile uint32_t* tmem_slot_ptr = (volatile uint32_t*)(t5_smem + (tmem_slot - raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the step's plan was written before the step's first kernel, which triggers after its own wait
-  // blockIdx.x = (block of query rows, key/value head), heads fastest and the last rows first:
-  // blocks are handed out in this order, so the longest ones of every head start first
-  const int b = blockIdx.z, kvh = blockIdx.x % p.n_kv_heads;
-  const int G = p.n_q_heads / p.n_kv_heads;
-  const int row0 = p.seq_row0[b], n_new = p.seq_row0[b + 1] - row0, pos0 = p.seq_pos0[b];
-  const int R = n_new * G;
-  const int r_base = (int)(gridDim.x / p.n_kv_heads - 1 - blockIdx.x / p.n_kv_heads) * (T5_QT * T5_ROWS);
-  // no rows, or positions without pages in the sequence's own list: nothing is read (the wait all the same: a launch
-  // whose blocks all left early would be over before the kernel before it)
-  if (r_base >= R || pos0 < 0 || (pos0 + n_new - 1) / KT >= p.page_off[b + 1] - p.page_off[b]) {
-    sb_pdl_wait();
-    return;
-  }
-  const int r_last = min(R, r_base + T5_QT * T5_ROWS) - 1;
-  const int tile_lo = low_key(p, pos0 + r_base / G) / KT;
-  const int tile_hi = (pos0 + r_last / G) / KT;
-  const int n_tiles = tile_hi - tile_lo + 1;
   if (raw & 1023u) {                       // the swizzled tiles need this alignment
     if (threadIdx.x == 0) atomicCAS(&g_status, 0, 10);
-    sb_pdl_wait();
+    sb_pdl_wait();                         // a launch that left early would be over before the kernel before it
     return;
   }
 
@@ -210,7 +192,27 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
   // Only now may the next kernel's blocks start: a product that took tensor memory on this SM ahead of this block, and then
   // waited for it, would leave both waiting for good.
   sb_pdl_launch();
-  sb_pdl_wait();                           // queries, keys and values come from the kernels before this one
+  // The plan, queries, keys and values come from the kernels before this one, the plan maybe from the very last (sb_advance_rows
+  // triggers at its first instruction).  Reading the plan ahead of this wait saved 0.7 us a launch: 97 tokens of the 7B
+  // sizes 3.99 ms instead of 4.01, nothing measurable from 2,048 tokens on.
+  sb_pdl_wait();
+
+  // blockIdx.x = (block of query rows, key/value head), heads fastest and the last rows first:
+  // blocks are handed out in this order, so the longest ones of every head start first
+  const int b = blockIdx.z, kvh = blockIdx.x % p.n_kv_heads;
+  const int G = p.n_q_heads / p.n_kv_heads;
+  const int row0 = p.seq_row0[b], n_new = p.seq_row0[b + 1] - row0, pos0 = p.seq_pos0[b];
+  const int R = n_new * G;
+  const int r_base = (int)(gridDim.x / p.n_kv_heads - 1 - blockIdx.x / p.n_kv_heads) * (T5_QT * T5_ROWS);
+  // no rows, or positions without pages in the sequence's own list: nothing is read
+  if (r_base >= R || pos0 < 0 || (pos0 + n_new - 1) / KT >= p.page_off[b + 1] - p.page_off[b]) {
+    if (warp == 1) tmem_dealloc(tmem, T5_TMEM_COLS);
+    return;
+  }
+  const int r_last = min(R, r_base + T5_QT * T5_ROWS) - 1;
+  const int tile_lo = low_key(p, pos0 + r_base / G) / KT;
+  const int tile_hi = (pos0 + r_last / G) / KT;
+  const int n_tiles = tile_hi - tile_lo + 1;
 
   if (warp == 0) {
     // ---- producer.  The K ring and the V ring advance independently: whichever has a free

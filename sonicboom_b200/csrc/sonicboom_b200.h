@@ -264,7 +264,7 @@ int sb_attention_plain(const void* q, void* out, int act_dtype, int n_rows, cons
 
 /* The same attention for float32 rows over a float32 cache of n_pages pages, by tiles of query rows: the step's
  * sequences own the rows seq_row0[s] ... seq_row0[s + 1] - 1 at positions from seq_pos0[s] on, at most max_new each, below
- * max_len; head sizes that are multiples of 4 up to 256. */
+ * max_len; head sizes that are multiples of 4 up to 256.  The step's arrays are read ahead, as sb_attention's of few rows. */
 int sb_attention_f32(const float* q, float* out, int n_rows, int n_seqs, int max_new, int max_len, const int32_t* seq_row0,
                      const int32_t* seq_pos0, const int32_t* page_off, const int32_t* page_ids, int page_size,
                      const float* cache, int n_pages, int n_q_heads, int n_kv_heads, int hd, int window, float scale,
@@ -496,7 +496,10 @@ size_t sb_attention_scratch_bytes(int n_rows, int n_q_heads, int n_kv_heads, int
                                   int max_len);
 /* Causal grouped-query attention of a step's rows over one cache entry's pages (bfloat16).
  * sink, chunk: as in sb_attention_plain.  bias: null, or float32 [n_q_heads][64 + bias_len + 64], the biases of
- * sb_attention_plain times log2(e) with 64 zeros before them and the last one 64 times more after them. */
+ * sb_attention_plain times log2(e) with 64 zeros before them and the last one 64 times more after them.
+ * Steps of few rows a sequence read seq_row0, seq_pos0 and page_off before the kernel ahead of them in the stream has
+ * ended: that kernel must not be the one that writes them, unless it lets its successors start only after its own wait or the
+ * attention is launched without programmatic dependent launch (sb_set_pdl).  Steps of more rows read them after it. */
 int sb_attention(const void* q, void* out, int n_rows, int n_seqs, int max_new,
                  const int32_t* seq_row0, const int32_t* seq_pos0, const int32_t* page_off,
                  const int32_t* page_ids, int page_size, const void* cache, int n_q_heads,

@@ -610,7 +610,9 @@ def attention(q: torch.Tensor, out: torch.Tensor, plan, group_index: int, cache:
     kernel would run (head sizes 64, 128); `"tma"` runs that decode kernel whatever the number of
     key splits (by itself it runs from about a wave of splits on).
     `warm`: a tensor the kernel after this one will stream (weights); the decode kernel asks for
-    it into L2 while it merges its partial results.  A hint: it changes no result."""
+    it into L2 while it merges its partial results.  A hint: it changes no result.
+    With few rows a sequence the plan's arrays are read while the kernel ahead may still run: that kernel must not be
+    the one that writes them (`advance_rows`, say)."""
     n = q.shape[0]
     g = plan.groups[group_index]
     if sink is not None:
