@@ -95,9 +95,10 @@ __device__ __forceinline__ float sb_warp_max(float v) {
 // start while its predecessor in the stream is still running.  A kernel calls sb_pdl_wait()
 // before it first touches anything a predecessor wrote; what it does before the wait (barrier
 // set-up, requesting weights) overlaps the predecessor's tail.  It calls sb_pdl_launch() where
-// its successor may be scheduled: small kernels at their start, the products and the attention
-// once their own operands have been requested, so that a successor does not take resources the
-// kernel still wants.  Without the launch attribute both are no-ops.
+// its successor may be scheduled: small kernels at their start, others once their own operands have been requested, so that
+// a successor does not take resources the kernel still wants.  Without the launch attribute both are no-ops.
+// A kernel that uses tensor memory triggers only when that memory is its own: its successor may take tensor memory ahead of
+// the wait for it, and on the same SM the two would wait for each other for good.
 // Starting is transitive: behind kernels that trigger at their first instruction a kernel can start while one several
 // places before it still runs.  A step's plan (positions, page lists) may be read ahead of the wait all the same, because
 // the step's first kernel, the embedding, triggers after its own wait.

@@ -502,7 +502,6 @@ gemm_tc5_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
   constexpr uint32_t ACC_COLS = 256;                   // column offset of the second accumulator
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  sb_pdl_launch();
   const int n_tiles = p.tiles_a * p.tiles_b;
   const int n_k = (p.K + BK - 1) / BK;
 
@@ -522,6 +521,7 @@ gemm_tc5_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  sb_pdl_launch();                         // the tensor memory is this block's: see sb_pdl_launch
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0 && lane == 0) {

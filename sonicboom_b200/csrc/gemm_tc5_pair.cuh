@@ -164,7 +164,6 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
-  sb_pdl_launch();
   const int S = p.k_splits;                            // K splits of a tile (1: none)
   const int n_tiles = p.tiles_a * p.tiles_b * S;       // units of work: (tile of 256 x BN, split), splits first
   const int n_k_all = (p.K + BK - 1) / BK, k_per = (n_k_all + S - 1) / S;
@@ -188,6 +187,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   cluster_arrive();                                    // the other block's barriers exist from here on
   cluster_wait();
   tc_fence_after();
+  sb_pdl_launch();                                     // the tensor memory is the pair's: see sb_pdl_launch
   const uint32_t tmem_base = *tmem_slot_ptr;
 
   if (warp == 0 && lane == 0) {
