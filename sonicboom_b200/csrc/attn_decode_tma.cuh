@@ -587,15 +587,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPar
 
 template <bool BIAS>
 int configure_decode_tma() {
-  static bool configured = false;
-  if (configured) return SB_OK;
-  cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_SMEM);
-  if (e == cudaSuccess)                          // all of the SM's memory as shared memory: three blocks fit
-    e = cudaFuncSetAttribute(attn_decode_tma_kernel<BIAS>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
+  const cudaError_t e = sb_set_once<attn_decode_tma_kernel<BIAS>>([] {
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_tma_kernel<BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_SMEM);
+    if (e == cudaSuccess)                        // all of the SM's memory as shared memory: three blocks fit
+      e = cudaFuncSetAttribute(attn_decode_tma_kernel<BIAS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               cudaSharedmemCarveoutMaxShared);
+    return e;
+  });
   if (e != cudaSuccess)
     SB_FAIL(SB_ERR_CUDA, "sb_attention: shared memory opt-in failed: %s", cudaGetErrorString(e));
-  configured = true;
   return SB_OK;
 }
 

@@ -673,25 +673,25 @@ int n_splits_for(int max_len) {
   return longs > most_short ? longs : most_short;
 }
 
-// Shared memory opt-ins of the mma.sync kernels, once per instantiation.
+// Shared memory opt-ins of the mma.sync kernels, once per instantiation and device.
 template <bool BIAS>
 int configure_mma() {
-  static bool configured = false;
-  if (configured) return SB_OK;
-  cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       PREFILL_SMEM);
-  if (e == cudaSuccess && DECODE_FITS)
-    e = cudaFuncSetAttribute(attn_decode_kernel<DEC_STAGES, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             DECODE_SMEM);
-  if (e == cudaSuccess && DECODE_FEW_FITS)
-    e = cudaFuncSetAttribute(attn_decode_kernel<DEC_STAGES_FEW, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             decode_smem(DEC_STAGES_FEW));
-  if (e == cudaSuccess && DECODE_SOME_FITS)
-    e = cudaFuncSetAttribute(attn_decode_kernel<DEC_STAGES_SOME, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             decode_smem(DEC_STAGES_SOME));
+  const cudaError_t e = sb_set_once<attn_prefill_kernel<BIAS>>([] {
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         PREFILL_SMEM);
+    if (e == cudaSuccess && DECODE_FITS)
+      e = cudaFuncSetAttribute(attn_decode_kernel<DEC_STAGES, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               DECODE_SMEM);
+    if (e == cudaSuccess && DECODE_FEW_FITS)
+      e = cudaFuncSetAttribute(attn_decode_kernel<DEC_STAGES_FEW, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               decode_smem(DEC_STAGES_FEW));
+    if (e == cudaSuccess && DECODE_SOME_FITS)
+      e = cudaFuncSetAttribute(attn_decode_kernel<DEC_STAGES_SOME, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               decode_smem(DEC_STAGES_SOME));
+    return e;
+  });
   if (e != cudaSuccess)
     SB_FAIL(SB_ERR_CUDA, "sb_attention: shared memory opt-in failed: %s", cudaGetErrorString(e));
-  configured = true;
   return SB_OK;
 }
 

@@ -451,22 +451,12 @@ __global__ void __launch_bounds__(TC_THREADS) attn_sigmoid_mma_decode_kernel(con
 
 template <int HD>
 int launch_sigmoid_mma(const SigmoidParams& p, int n_seqs, int max_new, cudaStream_t stream) {
-  static bool opted = false;
-  if (!opted) {
-    cudaError_t e = cudaFuncSetAttribute(attn_sigmoid_mma_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tc_smem<HD>());
-    if (e != cudaSuccess) SB_FAIL(SB_ERR_CUDA, "sb_attention_sigmoid: shared memory opt-in failed: %s", cudaGetErrorString(e));
-    opted = true;
-  }
+  if (cudaError_t e = sb_allow_shared<attn_sigmoid_mma_kernel<HD>>(tc_smem<HD>()))
+    SB_FAIL(SB_ERR_CUDA, "sb_attention_sigmoid: shared memory opt-in failed: %s", cudaGetErrorString(e));
   const int G = p.n_q_heads / p.n_kv_heads;
   if (max_new * G <= DEC_ROWS) {
-    static bool dec_opted = false;
-    if (!dec_opted) {
-      cudaError_t e = cudaFuncSetAttribute(attn_sigmoid_mma_decode_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           dec_smem<HD>());
-      if (e != cudaSuccess) SB_FAIL(SB_ERR_CUDA, "sb_attention_sigmoid: shared memory opt-in failed: %s", cudaGetErrorString(e));
-      dec_opted = true;
-    }
+    if (cudaError_t e = sb_allow_shared<attn_sigmoid_mma_decode_kernel<HD>>(dec_smem<HD>()))
+      SB_FAIL(SB_ERR_CUDA, "sb_attention_sigmoid: shared memory opt-in failed: %s", cudaGetErrorString(e));
     sb_launch(attn_sigmoid_mma_decode_kernel<HD>, dim3(p.n_kv_heads, 1, n_seqs), dim3(TC_THREADS), (size_t)dec_smem<HD>(),
               stream, p);
     return SB_OK;

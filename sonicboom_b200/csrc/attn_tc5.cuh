@@ -517,12 +517,8 @@ inline bool t5_make_map(CUtensorMap* map, const void* cache, long rows) {
 
 template <bool BIAS>
 int configure_tc5() {
-  static bool configured = false;
-  if (configured) return SB_OK;
-  cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5_SMEM);
-  if (e != cudaSuccess)
+  if (cudaError_t e = sb_allow_shared<attn_prefill_tc5_kernel<BIAS>>(T5_SMEM))
     SB_FAIL(SB_ERR_CUDA, "sb_attention: shared memory opt-in failed: %s", cudaGetErrorString(e));
-  configured = true;
   return SB_OK;
 }
 

@@ -9,6 +9,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include "device_cache.h"
 #include "sonicboom_b200.h"      // the public types and every entry point's declaration
 
 // Rows of a fused gate/up matrix alternate in blocks of this many: 8 gate rows, then the 8 up
@@ -105,6 +106,27 @@ __device__ __forceinline__ float sb_warp_max(float v) {
 __device__ __forceinline__ void sb_pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void sb_pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// Runs set(), which gives `kernel` its attributes, once per device: attributes belong to the device they were set on.  Safe with
+// several threads; a failure is returned, left in no one's way (the runtime's last error is cleared) and tried again next time.
+template <auto kernel, typename Set>
+cudaError_t sb_set_once(Set set) {
+  static SbDeviceCache done;
+  int device = -1;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    done.get(device, [&] {
+      e = set();
+      return e == cudaSuccess ? 0 : -1;
+    });
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+// Raises a kernel's limit of dynamic shared memory to `bytes` (always the same for one kernel).
+template <auto kernel>
+cudaError_t sb_allow_shared(int bytes) {
+  return sb_set_once<kernel>([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
 }
 
 // Asks for memory that a later kernel will stream (weights) to be brought into L2: a kernel

@@ -263,13 +263,8 @@ cudaError_t launch_delta_staged(dim3 grid, cudaStream_t stream, const float* pro
                                 int v_off, const float* aux, const int32_t* seq_row0, const int32_t* seq_slot,
                                 int n_heads, int dim, float* state, float* out) {
   constexpr size_t smem = (size_t)STAGES * TB * (5 * NPL * LPC + COLS) * sizeof(float);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<NPL, VEC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  configured = true;
+  if (smem > 48 * 1024)
+    if (cudaError_t e = sb_allow_shared<delta_scan_kernel<NPL, VEC, STAGES>>((int)smem)) return e;
   return sb_launch<SB_K_OTHER>(delta_scan_kernel<NPL, VEC, STAGES>, grid, dim3(THREADS), smem, stream, proj, ld, r_off,
                                k_off, v_off, aux, seq_row0, seq_slot, n_heads, dim, state, out);
 }

@@ -706,12 +706,8 @@ template <int NPL, int CPT, bool VEC>
 cudaError_t launch_scan_columns(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
   constexpr int STAGES = ScanShape<NPL, CPT>::bytes(3) <= 112 * 1024 ? 3 : 2;
   constexpr size_t smem = ScanShape<NPL, CPT>::bytes(STAGES);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(gdelta_scan_kernel<NPL, CPT, VEC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  configured = true;
+  if (smem > 48 * 1024)
+    if (cudaError_t e = sb_allow_shared<gdelta_scan_kernel<NPL, CPT, VEC, STAGES>>((int)smem)) return e;
   const dim3 grid((a.vdim + ScanShape<NPL, CPT>::COLS - 1) / ScanShape<NPL, CPT>::COLS, a.n_heads, n_seqs);
   return sb_launch<SB_K_OTHER>(gdelta_scan_kernel<NPL, CPT, VEC, STAGES>, grid, dim3(SCAN_THREADS), smem, stream, a);
 }

@@ -11,7 +11,6 @@
 //
 // Both need K to be a multiple of 8 (16-byte rows) and refuse other K with a clear error.
 #include "common.cuh"
-#include "device_cache.h"
 
 int sb_check_linear_args(const char* who, int M, int N, int K, int epilogue, const void* bias,
                          const float* residual, int out_dtype);
@@ -557,15 +556,9 @@ extern "C" int sb_gemm_tiled(const void* A, int a_dtype, const void* W, int w_dt
   if (!sb_valid_dtype(out_dtype)) SB_FAIL(SB_ERR_ARG, "sb_gemm_tiled: out dtype %d", out_dtype);
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) SB_FAIL(SB_ERR_UNSUPPORTED, "sb_gemm_tiled: M=%d is too many rows", M);
-  static bool configured[2] = {false, false};
   SB_DISPATCH_DTYPE(out_dtype, TO, {
-    if (!configured[out_dtype]) {
-      cudaError_t e = cudaFuncSetAttribute(gemm_tiled_kernel<TO>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, TILED_SMEM);
-      if (e != cudaSuccess)
-        SB_FAIL(SB_ERR_CUDA, "sb_gemm_tiled: shared memory opt-in failed: %s", cudaGetErrorString(e));
-      configured[out_dtype] = true;
-    }
+    if (cudaError_t e = sb_allow_shared<gemm_tiled_kernel<TO>>(TILED_SMEM))
+      SB_FAIL(SB_ERR_CUDA, "sb_gemm_tiled: shared memory opt-in failed: %s", cudaGetErrorString(e));
     sb_launch<SB_K_SKINNY>(gemm_tiled_kernel<TO>, grid, dim3(TILED_THREADS), TILED_SMEM, stream,
         (const bf16*)A, (const bf16*)W, M, N, K, epilogue, bias, bias_dtype, residual, (TO*)out);
   });

@@ -965,15 +965,9 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows)
 template <int BN, int STAGES, bool SWAPPED, typename TO>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Tc5Params& p, int blocks,
            cudaStream_t stream) {
-  static bool configured = false;
   constexpr int smem = smem_bytes(BN, STAGES);
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc5_kernel<BN, STAGES, SWAPPED, TO>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess)
-      SB_FAIL(SB_ERR_CUDA, "sb_gemm_tc5: shared memory opt-in failed: %s", cudaGetErrorString(e));
-    configured = true;
-  }
+  if (cudaError_t e = sb_allow_shared<gemm_tc5_kernel<BN, STAGES, SWAPPED, TO>>(smem))
+    SB_FAIL(SB_ERR_CUDA, "sb_gemm_tc5: shared memory opt-in failed: %s", cudaGetErrorString(e));
   sb_launch<SB_K_TC5>(gemm_tc5_kernel<BN, STAGES, SWAPPED, TO>, dim3(blocks), dim3(kernel_threads(BN, SWAPPED)), smem, stream,
                   ma, mb, p);
   SB_CHECK_LAUNCH("sb_gemm_tc5");
@@ -983,15 +977,9 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Tc5Params& p, int
 template <int BN, int STAGES, typename TO>
 int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const Tc5Params& p, int blocks,
                       cudaStream_t stream) {
-  static bool configured = false;
   constexpr int smem = persist_smem_bytes(BN, STAGES);
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc5_persistent_kernel<BN, STAGES, TO>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess)
-      SB_FAIL(SB_ERR_CUDA, "sb_gemm_tc5: shared memory opt-in failed: %s", cudaGetErrorString(e));
-    configured = true;
-  }
+  if (cudaError_t e = sb_allow_shared<gemm_tc5_persistent_kernel<BN, STAGES, TO>>(smem))
+    SB_FAIL(SB_ERR_CUDA, "sb_gemm_tc5: shared memory opt-in failed: %s", cudaGetErrorString(e));
   sb_launch<SB_K_TC5>(gemm_tc5_persistent_kernel<BN, STAGES, TO>, dim3(blocks), dim3(THREADS), smem, stream, ma,
             mb, p);
   SB_CHECK_LAUNCH("sb_gemm_tc5 (persistent)");
@@ -1032,28 +1020,26 @@ int persistent_bn(int M, int N, int n_sms) {
   return best;
 }
 
-// The pair kernel: clusters of two blocks, as many as the device runs at once (cached per kernel).
+// The pair kernel: clusters of two blocks, as many as the current device runs at once (0: none, or not known).
 template <int BN, typename TO, bool ROPE = false>
 int pair_clusters() {
-  static int clusters = -1;
-  if (clusters >= 0) return clusters;
+  static SbDeviceCache clusters;
+  constexpr auto kernel = gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO, ROPE>;
   constexpr int smem = pair_smem_bytes(BN, PAIR_STAGES);
-  clusters = 0;
-  if (cudaFuncSetAttribute(gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           smem) != cudaSuccess) {
+  int device = -1;
+  if (cudaGetDevice(&device) != cudaSuccess) cudaGetLastError();
+  const int n = clusters.get(device, [&] {
+    if (sb_allow_shared<kernel>(smem) != cudaSuccess) return -1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    int most = 0;
+    if (cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) == cudaSuccess) return most;
     cudaGetLastError();
-    return clusters;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2);
-  cfg.blockDim = dim3(PAIR_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_tc5_pair_kernel<BN, PAIR_STAGES, TO, ROPE>, &cfg) == cudaSuccess && n > 0)
-    clusters = n;
-  else
-    cudaGetLastError();
-  return clusters;
+    return -1;
+  });
+  return n > 0 ? n : 0;
 }
 
 template <int BN, typename TO, bool ROPE = false>

@@ -251,13 +251,8 @@ cudaError_t launch_scan(dim3 grid, cudaStream_t stream, const float* proj, int l
                         const float* decay, const float* head_decay, const float* token_decay, int heads_per_qk, const int32_t* seq_row0,
                         const int32_t* seq_slot, int n_heads, int dim, int vdim, float* state, float* out) {
   constexpr size_t smem = scan_smem<NPL>(PC, STAGES, CPT);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(linrec_scan_kernel<NPL, PC, VEC, STAGES, CPT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  configured = true;
+  if (smem > 48 * 1024)
+    if (cudaError_t e = sb_allow_shared<linrec_scan_kernel<NPL, PC, VEC, STAGES, CPT>>((int)smem)) return e;
   return sb_launch<SB_K_OTHER>(linrec_scan_kernel<NPL, PC, VEC, STAGES, CPT>, grid, dim3(THREADS), smem, stream, proj, ld,
                                q_off, k_off, v_off, decay, head_decay, token_decay, heads_per_qk, seq_row0, seq_slot, n_heads, dim, vdim, state, out);
 }

@@ -527,13 +527,8 @@ moe_gemm_mma_kernel(const bf16* a, const bf16* __restrict__ w, const int32_t* or
 template <int MI, int UP>
 int launch_mma(const void* a, const void* w, const int32_t* order, const int32_t* meta, int tiles, int top, int n_out,
                int n_in, float limit, float slope, void* out, cudaStream_t stream) {
-  static bool opted = false;
-  if (!opted) {
-    cudaError_t e = cudaFuncSetAttribute(moe_gemm_mma_kernel<MI, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         mma_smem(MI));
-    if (e != cudaSuccess) SB_FAIL(SB_ERR_CUDA, "mixture of experts: shared memory opt-in failed: %s", cudaGetErrorString(e));
-    opted = true;
-  }
+  if (cudaError_t e = sb_allow_shared<moe_gemm_mma_kernel<MI, UP>>(mma_smem(MI)))
+    SB_FAIL(SB_ERR_CUDA, "mixture of experts: shared memory opt-in failed: %s", cudaGetErrorString(e));
   constexpr int per = UP == GATED ? TN / 2 : TN;
   const dim3 grid(tiles, (n_out + per - 1) / per);
   sb_launch<SB_K_OTHER>(moe_gemm_mma_kernel<MI, UP>, grid, dim3(MMA_THREADS), (size_t)mma_smem(MI), stream,

@@ -1,10 +1,11 @@
 """The host code's memory of what a device answered, compiled and run here."""
+import re
 import shutil
 import subprocess
 
 import pytest
 
-from sonicboom_b200.csrc.build import SRC_DIR
+from sonicboom_b200.csrc.build import ARCH_FLAGS, SRC_DIR, BuildError, _nvcc
 
 PROGRAM = r"""
 #include <cstdio>
@@ -38,3 +39,49 @@ def test_device_cache(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(SRC_DIR), str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t"),
                     "-pthread"], check=True)
     assert subprocess.run([str(tmp_path / "t")]).returncode == 0
+
+ONCE = r"""
+#include <cuda_runtime.h>
+static int g_device = 0, g_fails = 0, g_set[2] = {0, 0}, g_cleared = 0;
+static cudaError_t fake_device(int* d) { *d = g_device; return cudaSuccess; }
+static cudaError_t fake_attribute(const void*, cudaFuncAttribute, int) {
+  if (g_fails > 0) { --g_fails; return cudaErrorInvalidValue; }
+  ++g_set[g_device];
+  return cudaSuccess;
+}
+static cudaError_t fake_last() { ++g_cleared; return cudaSuccess; }
+#define cudaGetDevice fake_device
+#define cudaFuncSetAttribute(k, a, v) fake_attribute((const void*)(k), a, v)
+#define cudaGetLastError fake_last
+#include "common.cuh"
+template <int N> __global__ void some_kernel() {}
+int main() {
+  g_fails = 1;
+  if (sb_allow_shared<some_kernel<1>>(1024) == cudaSuccess || g_cleared != 1) return 1;       // reported, and cleared
+  for (int i = 0; i < 3; ++i)
+    if (sb_allow_shared<some_kernel<1>>(1024) != cudaSuccess) return 2;                       // tried again, then kept
+  if (g_set[0] != 1) return 3;
+  g_device = 1;
+  if (sb_allow_shared<some_kernel<1>>(1024) != cudaSuccess || g_set[1] != 1) return 4;        // another device
+  g_device = 0;
+  if (sb_allow_shared<some_kernel<2>>(1024) != cudaSuccess || g_set[0] != 2) return 5;        // another kernel
+  return g_cleared == 1 ? 0 : 6;
+}
+"""
+
+
+def test_a_kernels_attributes_are_set_once_per_device(tmp_path):
+    try:
+        nvcc = _nvcc()
+    except BuildError:
+        pytest.skip("no nvcc")
+    (tmp_path / "t.cu").write_text(ONCE)
+    subprocess.run([nvcc, *ARCH_FLAGS, "-std=c++17", "-I", str(SRC_DIR), str(tmp_path / "t.cu"), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
+
+
+@pytest.mark.parametrize("path", sorted(SRC_DIR.glob("*.cu*")), ids=lambda p: p.name)
+def test_no_attribute_or_cluster_count_is_kept_for_all_devices(path):
+    """A flag or number of the whole process beside a query or attribute of one device."""
+    kept = re.compile(r"^ +static (?:bool|int) \w+(?:\[\d+\])? = [^;]*;\n(?:.*\n){0,4}?.*(?:cudaFuncSetAttribute|cudaOccupancy)", re.M)
+    assert not kept.findall(path.read_text())
