@@ -275,17 +275,20 @@ gemm_skinny_stream_kernel(const bf16* X, const bf16* __restrict__ W, int M, int 
   }
 }
 
-// How many of a kernel's blocks run at once on the current device (0: not known).
+// How many of a kernel's blocks run at once on the current device (0: not known, and no error left behind for the launch that
+// then takes place).
 template <auto kernel>
 int skinny_resident() {
   static SbDeviceCache most;
   int device = -1;
-  cudaGetDevice(&device);
+  if (cudaGetDevice(&device) != cudaSuccess) cudaGetLastError();
   const int n = most.get(device, [&] {
     int per_sm = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SK_WARPS * 32, 0) != cudaSuccess) return -1;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return -1;
-    return per_sm * sms;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SK_WARPS * 32, 0) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess)
+      return per_sm * sms;
+    cudaGetLastError();
+    return -1;
   });
   return n > 0 ? n : 0;
 }

@@ -80,6 +80,41 @@ def test_a_kernels_attributes_are_set_once_per_device(tmp_path):
     assert subprocess.run([str(tmp_path / "t")]).returncode == 0
 
 
+RESIDENT = r"""
+#include <cuda_runtime.h>
+static int g_bad = 0, g_last = 0;                  // which query fails; the runtime's last error
+static cudaError_t answer(int query) { return g_bad == query ? (cudaError_t)(g_last = cudaErrorInvalidValue) : cudaSuccess; }
+static cudaError_t fake_device(int* device) { *device = 0; return answer(1); }
+static cudaError_t fake_blocks(int* n, const void*, int, size_t) { *n = 2; return answer(2); }
+static cudaError_t fake_attribute(int* n, cudaDeviceAttr, int) { *n = 148; return answer(3); }
+static cudaError_t fake_last() { const int e = g_last; g_last = 0; return (cudaError_t)e; }
+#define cudaGetDevice fake_device
+#define cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, k, t, s) fake_blocks(n, (const void*)(k), t, s)
+#define cudaDeviceGetAttribute fake_attribute
+#define cudaGetLastError fake_last
+#include "gemm_mma.cu"
+int sb_check_linear_args(const char*, int, int, int, int, const void*, const float*, int) { return 0; }
+int main() {
+  for (g_bad = 2; g_bad <= 3; ++g_bad)
+    if (skinny_resident<gemm_skinny_stream_kernel<5, float>>() != 0 || g_last) return g_bad;
+  g_bad = 0;
+  return skinny_resident<gemm_skinny_stream_kernel<5, float>>() == 296 ? 0 : 4;
+}
+"""
+
+
+def test_a_failed_occupancy_query_leaves_no_error_for_the_launch_that_follows(tmp_path):
+    """The weight-streaming product then runs a block per group, and that launch is checked with the runtime's last error."""
+    try:
+        nvcc = _nvcc()
+    except BuildError:
+        pytest.skip("no nvcc")
+    (tmp_path / "t.cu").write_text(RESIDENT)
+    subprocess.run([nvcc, *ARCH_FLAGS, "-std=c++17", "--expt-relaxed-constexpr", "-O0", "-Xptxas", "-O0", "-I", str(SRC_DIR),
+                    str(tmp_path / "t.cu"), str(SRC_DIR / "error.cu"), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
+
+
 @pytest.mark.parametrize("path", sorted(SRC_DIR.glob("*.cu*")), ids=lambda p: p.name)
 def test_no_attribute_or_cluster_count_is_kept_for_all_devices(path):
     """A flag or number of the whole process beside a query or attribute of one device."""
