@@ -215,7 +215,7 @@ gemm_skinny_kernel(const bf16* X, const bf16* __restrict__ W, int M, int N, int 
 // group and keeps U K blocks of its warps' share in flight.  A K block's registers are asked for again, for the share's
 // next part or the next group's first, as soon as its MMAs have read them, so that loads go on through the sums, the
 // epilogue and what would be the start of another block.  Norm and gate/up product of one row of 17,920 x 1,536 14.4 to
-// 12.6 us (8.4 at the memory's pace); a grid of two waves or less gains nothing (a decode step of the recurrent design).
+// 12.6 us (8.4 at the memory's pace); a grid of two waves or less gains nothing.
 template <int U, typename TO>
 __global__ void __launch_bounds__(SK_WARPS * 32, 2)
 gemm_skinny_stream_kernel(const bf16* X, const bf16* __restrict__ W, int M, int N, int K,
@@ -293,8 +293,7 @@ int skinny_resident() {
   return n > 0 ? n : 0;
 }
 
-// Launches the streaming form if the product has more than two waves of groups; U leaves the fewest places of a warp's
-// share empty, the more in flight the better.
+// Launches the streaming form if the product has more than two waves of groups.
 template <int U, typename TO, typename... Args>
 bool stream_with(int N, cudaStream_t stream, Args... args) {
   const int groups = (N + 15) / 16, most = skinny_resident<gemm_skinny_stream_kernel<U, TO>>();
@@ -302,6 +301,12 @@ bool stream_with(int N, cudaStream_t stream, Args... args) {
   sb_launch<SB_K_SKINNY>(gemm_skinny_stream_kernel<U, TO>, dim3(most), dim3(SK_WARPS * 32), 0, stream, args...);
   return true;
 }
+// The streaming form with the U that leaves the fewest places of a warp's share empty, the more in flight the better; not where
+// eight, which the block-per-group kernel has, fit as well as any.  Time of that kernel over this one's, 9,488 to 18,928 rows of
+// W, 1 to 8 rows of activations, alone and behind a norm kernel:
+//   U = 5 to 7: K = 256 1.30 to 1.60, 512 1.26 to 1.48, 768 1.17 to 1.38, 1,024 1.10 to 1.28, 1,280 1.08 to 1.22, 1,536 1.07 to 1.15,
+//     2,560 1.15 to 1.27, 3,584 0.996 to 1.06, 4,608 1.06 to 1.17, 5,120 1.01 to 1.09, 6,656 to 7,680 1.01 to 1.12;
+//   U = 8: K = 1,800 to 2,048 0.95 to 1.06 on three GPUs, another sign from one to the next; 4,096, 6,144 and 8,184 0.965 to 1.03.
 template <typename TO, typename... Args>
 bool launch_stream(int N, int K, cudaStream_t stream, Args... args) {
   const int mine = ((K + 31) / 32 + SK_WARPS - 1) / SK_WARPS;     // a warp's K blocks
@@ -309,10 +314,10 @@ bool launch_stream(int N, int K, cudaStream_t stream, Args... args) {
   int best = 8;
   for (int u = 7; u >= 5; --u)
     if (places(u) < places(best)) best = u;
-  if (best == 8) return stream_with<8, TO>(N, stream, args...);
   if (best == 7) return stream_with<7, TO>(N, stream, args...);
   if (best == 6) return stream_with<6, TO>(N, stream, args...);
-  return stream_with<5, TO>(N, stream, args...);
+  if (best == 5) return stream_with<5, TO>(N, stream, args...);
+  return false;
 }
 
 template <int NT>

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-# a warp's share of K of less than one K block, of five to eight in flight, and of several parts; N with a ragged last group
+# a warp's share of K of less than one K block, of five to seven in flight, of eight (a block a group), and of several parts; N with a ragged last group
 @pytest.mark.parametrize("K", [8, 72, 200, 1280, 1536, 1800, 2048, 3584])
 @pytest.mark.parametrize("N", [9488, 12008, 17920])
 @pytest.mark.parametrize("M", [1, 5, 8])
