@@ -12,19 +12,25 @@ def i32(x):
     return torch.tensor(x, dtype=torch.int32, device=DEV)
 
 
-# rows that end inside a tile and inside a warp, and last column tiles that are not full
-@pytest.mark.parametrize("rows", [1025, 2048, 3007])
-@pytest.mark.parametrize("hq,hkv,hd,K", [(28, 4, 128, 512), (12, 2, 128, 1536), (16, 4, 64, 200), (5, 5, 128, 72), (40, 8, 64, 264)])
+@pytest.fixture
+def widest_tiles():
+    """256 columns for every product of many rows, as most sizes of a prompt have them: no K split, no narrower tile."""
+    ops.force_tc5_tile_width(256)
+    yield
+    ops.force_tc5_tile_width(0)
+
+
+# rows that end inside a tile and inside a warp; column tiles that are full, and last ones with 64, 128 and 192 columns
+@pytest.mark.parametrize("rows", [129, 1025, 2048, 3007])
+@pytest.mark.parametrize("hq,hkv,hd,K", [(28, 4, 128, 512), (12, 2, 128, 1536), (16, 4, 64, 200), (5, 5, 128, 72), (40, 8, 64, 264),
+                                         (9, 2, 64, 136), (11, 2, 64, 200)])
 @pytest.mark.parametrize("bias", [None, torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("has_kv", [True, False])
-def test_table_gives_the_rotation_kernels_bits(rows, hq, hkv, hd, K, bias, has_kv):
+def test_table_gives_the_rotation_kernels_bits(widest_tiles, rows, hq, hkv, hd, K, bias, has_kv):
     torch.manual_seed(rows + K)
     N = (hq + (2 * hkv if has_kv else 0)) * hd
     w = torch.randn(N, K, device=DEV, dtype=torch.bfloat16) * K ** -0.5
-    if not ops.takes_rotation_table(rows, w, hq, hkv, hd, hd, has_kv):
-        # K is split, one wave of narrower tiles, or a narrower tile leaves fewer columns outside
-        assert (rows + 255) // 256 * ((N + 255) // 256) <= 74 or ops.tc5_tile_width(rows, N) != 256
-        return
+    assert ops.takes_rotation_table(rows, w, hq, hkv, hd, hd, has_kv)
     h = torch.randn(rows, K, device=DEV, dtype=torch.bfloat16)
     b = torch.randn(N, device=DEV).to(bias) if bias is not None else None
     inv = torch.rand(hd // 2, device=DEV)
@@ -34,7 +40,7 @@ def test_table_gives_the_rotation_kernels_bits(rows, hq, hkv, hd, K, bias, has_k
     pos = [r - cut[s] + (100 if s == 1 else 0) for r, s in enumerate(seq)]
     pos[5] = -1
     need = [(cut[s + 1] - cut[s] + 100 + 63) // 64 for s in range(3)]
-    need[2] -= 3
+    need[2] = max(1, need[2] - 3)
     off = [0, need[0], need[0] + need[1], sum(need)]
     pages = torch.randperm(sum(need)).tolist()
     where = (inv, i32(seq), i32(pos), i32(off), i32(pages), 64)
@@ -70,3 +76,16 @@ def test_a_table_is_left_alone_where_the_product_does_not_take_it():
             ops.qkv_rope_store(h, w, None, hq, hkv, hd, hd, *where, cache, q, table)
             outs.append((q.clone(), cache))
         assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("rows,hq,hkv,hd,K,takes", [
+    (128, 28, 4, 128, 3584, False), (512, 28, 4, 128, 3584, False),                                   # few rows, K split
+    (768, 28, 4, 128, 3584, False), (769, 28, 4, 128, 3584, True), (2048, 28, 4, 128, 3584, True),    # one wave of narrower tiles; more
+    (1024, 12, 2, 128, 1536, False), (2048, 12, 2, 128, 1536, False), (2049, 12, 2, 128, 1536, True),
+    (3007, 5, 5, 128, 72, False)])                                                                     # a narrower tile wastes less
+def test_which_products_take_a_table(rows, hq, hkv, hd, K, takes):
+    if torch.cuda.get_device_properties(DEV).multi_processor_count != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    w = torch.empty((hq + 2 * hkv) * hd, K, device=DEV, dtype=torch.bfloat16)
+    assert ops.takes_rotation_table(rows, w, hq, hkv, hd, hd) == takes
+    assert not ops.takes_rotation_table(rows, w, hq, hkv, hd, hd // 2)
