@@ -25,12 +25,15 @@
 // Scores, maxima, sums and the output are float32; probabilities are rounded to bfloat16 only
 // as the P.V operand, and the row sum uses them before rounding.
 //
-// Bound by the softmax threads: 64 exponentials a row and page are 1,024 cycles of a page's four quarters of an SM, the MMAs 1,400.
-// Measured page by page before P went through tensor memory (cycles): 4,700, of them waits for the MMAs 1,400, tcgen05.ld 500,
-// arrivals of every thread on one barrier 450, the maximum 700, exponentials 1,190, P to shared memory and the fence
-// for the tensor cores 430; and 13,000 ahead of the first page, for query rows loaded one 16 bytes after another.
-// The kernel alone, us, that form / this one: 2,048 tokens of 28/4 heads of 128 53.7 / 39.9 (750 TFLOP/s), 97 14.6 / 9.9, 300
-// 18.1 / 12.7; turns of 500, 2,200 and 3,500 tokens 529 / 412 (1,010); 64 prompts of 16 to 1,024 with 12/2 heads 265 / 167.
+// Bound by a page's chain S, scores out, maximum, exponentials, P in, P.V, of which a block's two tiles overlap a part: long turns take
+// 2,350 cycles a page (452 us at 1.77 GHz for 341 pages an SM), one prompt of 2,048 tokens 2,860 with the blocks' starts and
+// ends (25 pages an SM).  No unit is full: of the latter the tensor pipe is active for 36 % (1,020 cycles a page), the
+// unit of the exponentials for 37 % (64 a row are 1,024 cycles of a page's four quarters of an SM).  With P through shared memory a
+// page took 4,700: waits for the MMAs 1,400, tcgen05.ld 500, arrivals of every thread on one barrier 450, the maximum
+// 700, exponentials 1,190, P and the fence for the tensor cores 430; and 13,000 ahead of the first page, for query rows
+// loaded one 16 bytes after another.
+// The kernel alone, us, that form / this one: 2,048 tokens of 28/4 heads of 128 53.7 / 41.0 (730 TFLOP/s), 97 14.6 / 10.3, 300
+// 18.1 / 13.2; turns of 500, 2,200 and 3,500 tokens 529 / 414 (1,005); 64 prompts of 16 to 1,024 with 12/2 heads 265 / 171.
 // A block runs its prologue once, from a cold instruction cache: query addresses with a division each, unrolled, were 3 us of it (97
 // tokens 11.2 us alone, and no gain at all inside a prompt).
 //
@@ -193,19 +196,20 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
   // waited for it, would leave both waiting for good.
   sb_pdl_launch();
   // The plan, queries, keys and values come from the kernels before this one, the plan maybe from the very last (sb_advance_rows
-  // triggers at its first instruction).  Reading the plan ahead of this wait saved 0.7 us a launch: 97 tokens of the 7B
-  // sizes 3.99 ms instead of 4.01, nothing measurable from 2,048 tokens on.
+  // triggers at its first instruction).  With the plan read ahead of this wait, and blocks without rows gone by then, the kernel
+  // alone took 0.5 us less (97 tokens 9.9 for 10.3, 64 prompts 166 for 171), a prompt's step the same.
   sb_pdl_wait();
 
   // blockIdx.x = (block of query rows, key/value head), heads fastest and the last rows first:
   // blocks are handed out in this order, so the longest ones of every head start first
   const int b = blockIdx.z, kvh = blockIdx.x % p.n_kv_heads;
   const int G = p.n_q_heads / p.n_kv_heads;
-  const int row0 = p.seq_row0[b], n_new = p.seq_row0[b + 1] - row0, pos0 = p.seq_pos0[b];
-  const int R = n_new * G;
+  const int row0 = p.seq_row0[b], row1 = p.seq_row0[b + 1], pos0 = p.seq_pos0[b];      // asked for together, ahead of any branch
+  const int page0 = p.page_off[b], n_own_pages = p.page_off[b + 1] - page0;
+  const int n_new = row1 - row0, R = n_new * G;
   const int r_base = (int)(gridDim.x / p.n_kv_heads - 1 - blockIdx.x / p.n_kv_heads) * (T5_QT * T5_ROWS);
   // no rows, or positions without pages in the sequence's own list: nothing is read
-  if (r_base >= R || pos0 < 0 || (pos0 + n_new - 1) / KT >= p.page_off[b + 1] - p.page_off[b]) {
+  if (r_base >= R || pos0 < 0 || (pos0 + n_new - 1) / KT >= n_own_pages) {
     if (warp == 1) tmem_dealloc(tmem, T5_TMEM_COLS);
     return;
   }
@@ -218,7 +222,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPa
     // ---- producer.  The K ring and the V ring advance independently: whichever has a free
     // stage gets its next page requested, so a wait for one never holds up the other.  The
     // whole warp walks the loop; lanes fetch 32 page ids at a time, one elected lane issues.
-    const int32_t* pages = p.page_ids + p.page_off[b] + tile_lo;
+    const int32_t* pages = p.page_ids + page0 + tile_lo;
     const bool leader = elect_one();
     int ik = 0, iv = 0;                       // next K page and next V page to request
     int ids_k = 0, ids_v = 0;                 // page ids of the 32-page block ik / iv lies in
